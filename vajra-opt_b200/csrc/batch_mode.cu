@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "halpern_state.cuh"
 #include "solver.cuh"
 
 namespace vajra {
@@ -115,10 +116,10 @@ struct EpiBPrimal {
     template <typename Acc>
     __device__ void operator()(int j, Acc v, const Pre& p) const {
         if (p.done) return;
-        T xp = p.xo - p.tau * (p.c + static_cast<T>(v));
-        xp = xp < p.cl ? p.cl : (xp > p.cu ? p.cu : xp);
-        xb[j] = xp + xp - p.xo;
-        x[j] = p.w1 * ((T(1) + p.g) * xp - p.g * p.xo) + p.w0 * p.x0;
+        T xp, xbn, xn;
+        halpern_primal(p.xo, static_cast<T>(v), p.c, p.cl, p.cu, p.x0, p.tau, p.w1, p.w0, p.g, &xp, &xbn, &xn);
+        xb[j] = xbn;
+        x[j] = xn;
         if (write_cand) xc[j] = xp;
     }
     template <typename Acc>
@@ -154,12 +155,9 @@ struct EpiBDual {
     template <typename Acc>
     __device__ void operator()(int r, Acc w, const Pre& p) const {
         if (p.done) return;
-        const T sg = p.sigma;
-        const T yh = p.yo + sg * static_cast<T>(w);
-        T q = yh * p.inv_sigma;
-        q = q < p.rl ? p.rl : (q > p.ru ? p.ru : q);
-        const T yp = yh - sg * q;
-        y[r] = p.w1 * ((T(1) + p.g) * yp - p.g * p.yo) + p.w0 * p.y0;
+        T yp, yn;
+        halpern_dual(p.yo, static_cast<T>(w), p.rl, p.ru, p.y0, p.sigma, p.inv_sigma, p.w1, p.w0, p.g, &yp, &yn);
+        y[r] = yn;
         if (write_cand) yc[r] = yp;
     }
     template <typename Acc>

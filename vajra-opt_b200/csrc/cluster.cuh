@@ -1,0 +1,553 @@
+// Cluster-resident PDHG iterations: one thread-block cluster (1..16 CTAs) keeps an LP in its
+// shared memory and runs whole chunks of iterations in one launch.
+//
+// Why: on an LP of a few 10^4 entries an iteration kernel moves a few hundred KB, a
+// microsecond of work, and two launches an iteration cost 5.5 to 6.8 us whatever they do.  Here the
+// iterates never leave shared memory, and the only thing an iteration waits for is the
+// exchange of x_bar and of y between the CTAs.
+//
+// Layout.  CTA r of the cluster owns a slice of the columns and a slice of the rows (contiguous,
+// cut at equal shares of entries + 16 per row, at multiples of four so that slices are 16-byte
+// aligned): a thread owns at most one of each and keeps its vectors in registers.  Shared memory
+// holds both matrices' entries of the slices and full copies of x_bar and y, from which the row
+// sums gather.
+// Exchange.  After each half-iteration a CTA sends its slice of the new vector to every other
+// CTA with one bulk copy each (cp.async.bulk, shared memory to shared memory), which signals the
+// receiver's mbarrier; a CTA goes on when all slices have arrived.  That is the only barrier of
+// a half-iteration.  Measured for 8 CTAs of 512 threads (B200): 0.62 us for 2 KB, 0.64 us for
+// 8 KB, 0.95 us for 20 KB; plain remote stores and a cluster barrier took 0.88 to 1.33 us, a copy
+// through L2 1.3 to 1.5 us.
+// Why no buffer is written early: x_bar and y alternate.  A CTA overwrites a peer's copy of x_bar
+// only after it has received that peer's y of the iteration before, which the peer sends after
+// its last read of x_bar; the same with the names exchanged.
+// Why each vector has its own mbarrier: a CTA that runs ahead sends at most one exchange ahead,
+// and that one goes to the other mbarrier, so bytes are never counted in the wrong phase.
+// Row sums are formed exactly as the grouped-lane kernel forms them (G lanes a row, strided,
+// butterfly; rows longer than long_len by 256 threads), so results have the same bits.
+#pragma once
+
+#include "common.cuh"
+#include "spmv.cuh"
+
+namespace vajra {
+
+constexpr int kClThreads = 512;                // most threads of a CTA
+constexpr int kClMaxChains = 8;                // chains of a row that one thread may form
+constexpr int kClMaxLong = 16;                 // rows summed by 256 threads that a CTA may have
+constexpr int kClMaxCtas = 16;
+constexpr int kClRowWeight = 16;               // a row's share of the work beside its entries
+constexpr size_t kClSmemCap = 216 * 1024;      // dynamic shared memory a CTA may ask for
+constexpr int kClWaitTries = 1 << 20;          // bound of every mbarrier wait
+
+// One matrix of the LP: rows `rows`, indices minus idx_base are local.
+template <typename V>
+struct ClMat {
+    int rows;
+    const int64_t* ptr;
+    const int32_t* idx;
+    const V* val;
+    int idx_base;
+    int group;          // lanes per row: 1, 2, 4, .. 32
+    int64_t long_len;   // rows longer than this are summed by 256 threads
+};
+
+__device__ __forceinline__ uint32_t cl_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cl_size() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+// All threads of the cluster; global and shared writes before it are visible after it.
+__device__ __forceinline__ void cl_barrier() {
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cl_map(uint32_t addr, uint32_t rank) {
+    uint32_t o;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(addr), "r"(rank));
+    return o;
+}
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// First row of slice `r` of `parts`: the smallest multiple of four whose rows before it carry
+// at least r / parts of the weight (entries + kClRowWeight a row).
+__host__ __device__ inline int cl_bound(int rows, const int64_t* ptr, int r, int parts) {
+    if (r <= 0) return 0;
+    if (r >= parts) return rows;
+    const int64_t p0 = ptr[0];
+    const int64_t total = ptr[rows] - p0 + static_cast<int64_t>(kClRowWeight) * rows;
+    const int64_t target = total * r / parts;
+    int lo = 0, hi = (rows + 3) / 4;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        const int j = 4 * mid < rows ? 4 * mid : rows;
+        if (ptr[j] - p0 + static_cast<int64_t>(kClRowWeight) * j < target) lo = mid + 1; else hi = mid;
+    }
+    return 4 * lo < rows ? 4 * lo : rows;
+}
+// No slice has more rows than this (its weight is at most a part plus the last four rows').
+inline int64_t cl_slice_rows(int64_t rows, int64_t nnz, int parts) {
+    if (parts == 1) return rows;
+    const int64_t b = (nnz + kClRowWeight * rows) / (static_cast<int64_t>(kClRowWeight) * parts) + 8;
+    return b < rows ? b : rows;
+}
+
+inline int64_t pad4(int64_t v) { return (v + 3) / 4 * 4; }
+
+// Shared memory of a CTA: the two full vectors, the larger scratch of dealing a slice, and both
+// slices' entries (an equal share of `value` bytes and a 4-byte place each, a half more for
+// padding, at least a pair a thread).
+inline size_t cl_smem_bytes(size_t t, size_t value, int64_t m, int64_t n, int64_t nnz, int parts, int threads) {
+    const size_t share = static_cast<size_t>(nnz + nnz / 2) / parts + 2 * threads;
+    return t * (pad4(n + 1) + pad4(m + 1)) + 2 * share * (value + 4) + 8 * threads + 24 * kClMaxLong + 1024;
+}
+
+// The dynamic shared memory of a cluster kernel and an array in it.  Arrays are kept as offsets,
+// not as pointers, so that every access compiles to a shared-memory instruction.
+extern __shared__ __align__(16) unsigned char cl_smem[];
+template <typename U>
+struct ClArray {
+    uint32_t off = 0;
+    __device__ __forceinline__ U* ptr() const { return reinterpret_cast<U*>(cl_smem + off); }
+    __device__ __forceinline__ U& operator[](int i) const { return ptr()[i]; }
+};
+
+// One matrix slice as the iterations read it: every row of the slice has its own threads, so a
+// CTA has at most blockDim.x rows and columns, and everything an iteration needs of a row is in
+// its owner's registers.
+// The grouped-lane kernel gives a row G chains of products (entry k to chain k mod G) and adds
+// the chains in a butterfly.  Here tpr (<= G) threads share a row: thread l forms the chains l,
+// l + tpr, l + 2 tpr, .. in order, adds them up the butterfly as far as they go, and shuffles do
+// the rest.  The rows are sorted by length and dealt to the threads in that order; the entries
+// of a warp's 32 tasks lie side by side, two of a task in one load, padded with zero values that
+// point at the zero behind the vector.
+// (Reading the slice as CSR, with the vectors in shared memory and rounds over the rows, took
+// 370 instructions a thread and iteration: with 8 to 16 warps on an SM those instructions, one
+// after another, were what an iteration waited for -- 1.9 us on a 60 x 150 LP.)
+struct ClSlice {                // uniform over the CTA, in shared memory
+    int b0, rows;               // first row, number of rows
+    int tpr_shift;              // threads per row, log2
+    int n_long;                 // rows longer than long_len (summed by 256 threads), and of
+    uint32_t longs;             // each its number, first entry and length
+    long long e0;               // first entry
+};
+struct ClInfo {                 // uniform over the CTA, in shared memory
+    unsigned long long bar_x, bar_y;     // mbarriers of the two exchanges
+    ClSlice cols, rows;
+    int m, n;
+    uint32_t rank, size;
+    uint32_t bytes_x, bytes_y;           // my slices of x_bar and y
+    uint32_t expect_x, expect_y;         // what the peers send
+    uint32_t top, end;                   // free dynamic shared memory
+    int count;
+};
+// Two entries of a task: the vector entries' places in shared memory (bytes) and the values.
+template <typename T> struct ClPair;
+template <> struct alignas(16) ClPair<float> { uint32_t off0; float val0; uint32_t off1; float val1; };
+template <> struct alignas(8) ClPair<double> { uint32_t off0, off1; double val0, val1; };
+struct ClTask {                 // a thread's task of one slice
+    int row;                    // its row of the slice, -1: none
+    int pairs, turn;            // pairs of entries and pairs a chain (the same for all of a warp)
+    uint32_t pair;              // its first pair; the next ones follow 32 pairs apart
+};
+
+// Bytes of `rows` entries of a vector, rounded up to whole groups of four (the full vectors are
+// padded to multiples of four).
+template <typename T>
+__host__ __device__ inline uint32_t cl_bytes(int rows) { return static_cast<uint32_t>((rows + 3) / 4 * 4 * sizeof(T)); }
+// Offset of the full y behind the full x_bar (which starts the dynamic shared memory); each has
+// at least one zero after its end.
+template <typename T>
+__device__ __forceinline__ uint32_t cl_y_offset(int n) { return static_cast<uint32_t>((n / 4 * 4 + 4) * sizeof(T)); }
+
+// Cuts the slices and sets the mbarriers up.  A cluster barrier has to follow before the first
+// exchange.
+template <typename T, typename V>
+__device__ __noinline__ void cl_begin(const ClMat<V>& a, const ClMat<V>& at, uint32_t bytes, ClInfo& I) {
+    if (threadIdx.x == 0) {
+        const uint32_t rank = cl_rank(), size = cl_size();
+        I.rank = rank;
+        I.size = size;
+        I.m = a.rows;
+        I.n = at.rows;
+        // arrivals of a phase: my own and one from every peer that has nothing to send
+        uint32_t ax = 1, ay = 1;
+        int c = 0, r = 0;
+#pragma unroll 1
+        for (uint32_t q = 0; q < size; ++q) {
+            const int c1 = cl_bound(at.rows, at.ptr, q + 1, size), r1 = cl_bound(a.rows, a.ptr, q + 1, size);
+            if (q == rank) {
+                I.cols.b0 = c; I.cols.rows = c1 - c; I.cols.e0 = at.ptr[c];
+                I.rows.b0 = r; I.rows.rows = r1 - r; I.rows.e0 = a.ptr[r];
+            } else {
+                ax += c1 == c ? 1 : 0;
+                ay += r1 == r ? 1 : 0;
+            }
+            c = c1;
+            r = r1;
+        }
+        I.bytes_x = cl_bytes<T>(I.cols.rows);
+        I.bytes_y = cl_bytes<T>(I.rows.rows);
+        I.expect_x = cl_bytes<T>(at.rows) - I.bytes_x;
+        I.expect_y = cl_bytes<T>(a.rows) - I.bytes_y;
+        I.top = cl_y_offset<T>(at.rows) + cl_y_offset<T>(a.rows);
+        I.end = bytes;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&I.bar_x)), "r"(ax) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&I.bar_y)), "r"(ay) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 4) {   // the zeros behind the full vectors
+        const int n4 = at.rows / 4 * 4 + static_cast<int>(threadIdx.x), m4 = a.rows / 4 * 4 + static_cast<int>(threadIdx.x);
+        ClArray<T>{0}[n4] = T(0);
+        ClArray<T>{cl_y_offset<T>(at.rows)}[m4] = T(0);
+    }
+    __syncthreads();
+}
+
+// Deals the rows of slice `s` to the threads and lays their entries out; `vec`: where the
+// vector they multiply starts, `zero`: the index of the zero behind it.  *ok: false when they do not fit (uniform over the CTA).
+template <typename V>
+__device__ __noinline__ ClTask cl_deal(const ClMat<V>& mat, ClSlice& s, uint32_t vec, int zero, ClInfo& I, bool* ok) {
+    ClTask t{-1, 0, 0, 0};
+    *ok = false;
+    const int rows = s.rows, tid = threadIdx.x;
+    const long long e0 = s.e0;
+    const uint32_t base = (I.top + 15) / 16 * 16;
+    ClArray<int> longs{base};
+    const uint32_t mark = base + 12 * kClMaxLong;   // scratch from here on: given back below
+    ClArray<int> off{mark};
+    ClArray<uint16_t> perm{mark + 4u * (rows + 1)};
+    ClArray<int> first_pair{(mark + 6u * (rows + 1) + 3) / 4 * 4};
+    if (rows > static_cast<int>(blockDim.x) || first_pair.off + 4 * 33 > I.end) return t;
+    if (tid == 0) I.count = 0;
+    __syncthreads();
+    for (int r = tid; r <= rows; r += blockDim.x) {
+        const int64_t p = mat.ptr[s.b0 + r];
+        off[r] = static_cast<int>(p - e0);
+        const int64_t len = r < rows ? mat.ptr[s.b0 + r + 1] - p : 0;
+        if (len > mat.long_len) {
+            const int i = atomicAdd(&I.count, 1);
+            if (i < kClMaxLong) {
+                longs[3 * i] = r;
+                longs[3 * i + 1] = static_cast<int>(p - e0);
+                longs[3 * i + 2] = static_cast<int>(len);
+            }
+        }
+    }
+    __syncthreads();
+    int sh = 0;
+    while ((2 << sh) <= mat.group && (rows << (sh + 1)) <= static_cast<int>(blockDim.x)) ++sh;
+    const int chains = mat.group >> sh, tpr = 1 << sh;
+    if (I.count > kClMaxLong || chains > kClMaxChains) return t;
+    auto length = [&](int r) {   // rows for the 256 threads have no tasks
+        const int len = off[r + 1] - off[r];
+        return len > mat.long_len ? 0 : len;
+    };
+    if (tid < rows) {
+        const int len = length(tid);
+        int before = 0;
+        for (int q = 0; q < rows; ++q) {
+            const int l = length(q);
+            before += (l > len || (l == len && q < tid)) ? 1 : 0;
+        }
+        perm[before] = static_cast<uint16_t>(tid);
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    // a warp's first task is its longest; its pairs come after those of the warps before it
+    auto warp_turn = [&](int w) {
+        const int p = (32 * w) >> sh;
+        return p < rows ? ((length(perm[p]) + mat.group - 1) / mat.group + 1) / 2 : 0;
+    };
+    int len = 0, first = 0;
+    if ((tid >> sh) < rows) {
+        t.row = perm[tid >> sh];
+        len = length(t.row);
+        first = off[t.row];
+    }
+    t.turn = warp_turn(warp);
+    t.pairs = chains * t.turn;
+    if (tid == 0) {
+        int sum = 0;
+        for (int w = 0; w < warps; ++w) { first_pair[w] = sum; sum += chains * warp_turn(w); }
+        first_pair[32] = sum;
+        s.tpr_shift = sh;
+        s.n_long = I.count;
+        s.longs = longs.off;
+    }
+    __syncthreads();
+    const int64_t pairs = 32 * static_cast<int64_t>(first_pair[32]);
+    const int slot = 32 * first_pair[warp] + lane;
+    __syncthreads();   // the scratch is read
+    const uint32_t pair0 = (mark + 15) / 16 * 16;
+    const int64_t end = pair0 + pairs * static_cast<int64_t>(sizeof(ClPair<V>));
+    if (end > static_cast<int64_t>(I.end)) return t;
+    t.pair = pair0 + slot * static_cast<uint32_t>(sizeof(ClPair<V>));
+    for (int u = 0; u < t.pairs; ++u) {
+        uint32_t ii[2];
+        V vv[2];
+        int chain = 0;   // the place of u's chain, its bits reversed
+        for (int q = u / t.turn, c = 1; c < chains; c *= 2, q /= 2) chain = 2 * chain + (q & 1);
+        for (int h = 0; h < 2; ++h) {
+            const int k = (tid & (tpr - 1)) + tpr * (chain + chains * (2 * (u % t.turn) + h));
+            ii[h] = static_cast<uint32_t>(zero);
+            vv[h] = V(0);
+            if (k < len) {
+                ii[h] = static_cast<uint32_t>(mat.idx[e0 + first + k] - mat.idx_base);
+                vv[h] = mat.val[e0 + first + k];
+            }
+        }
+        ClPair<V> e;
+        e.off0 = vec + ii[0] * static_cast<uint32_t>(sizeof(V));
+        e.off1 = vec + ii[1] * static_cast<uint32_t>(sizeof(V));
+        e.val0 = vv[0];
+        e.val1 = vv[1];
+        ClArray<ClPair<V>>{t.pair}[32 * u] = e;
+    }
+    if (tid == 0) I.top = static_cast<uint32_t>(end);
+    __syncthreads();
+    *ok = true;
+    return t;
+}
+
+// My chains of my row, added up the butterfly as far as they go in this thread.  The chains lie
+// one after another in the order in which the butterfly pairs them up (0, C/2, C/4, 3C/4, ..), each
+// `turn` pairs long; finished sums wait in s0, s1, s2 for their partners like the digits of a
+// binary counter.  One form for every number of chains: a form for each, inlined twice, drove the
+// iteration's registers into local memory.
+template <typename T>
+__device__ __forceinline__ T cl_chains(const ClTask& t) {
+    constexpr int P = 4;   // pairs taken together: their loads overlap
+    const ClArray<ClPair<T>> ep{t.pair};
+    T acc = T(0), s0 = T(0), s1 = T(0), s2 = T(0), total = T(0);
+    int left = t.turn, k = 0;
+#pragma unroll 1
+    for (int u = 0; u < t.pairs; u += P) {
+        ClPair<T> e[P];
+        T xx[2 * P];
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (p == 0 || u + p < t.pairs) e[p] = ep[32 * (u + p)];
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (p == 0 || u + p < t.pairs) {
+                xx[2 * p] = *reinterpret_cast<const T*>(cl_smem + e[p].off0);
+                xx[2 * p + 1] = *reinterpret_cast<const T*>(cl_smem + e[p].off1);
+            }
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (p == 0 || u + p < t.pairs) {
+                acc = fma(e[p].val0, xx[2 * p], acc);
+                acc = fma(e[p].val1, xx[2 * p + 1], acc);
+                if (--left == 0) {   // a chain is done (the same for all of a warp)
+                    left = t.turn;
+                    total = acc;
+                    if (k & 1) {
+                        total = s0 + total;
+                        if (k & 2) {
+                            total = s1 + total;
+                            if (k & 4) total = s2 + total; else s2 = total;
+                        } else {
+                            s1 = total;
+                        }
+                    } else {
+                        s0 = total;
+                    }
+                    ++k;
+                    acc = T(0);
+                }
+            }
+    }
+    return total;
+}
+
+// The rows longer than long_len, one after another, by 256 threads each, as the grouped-lane
+// kernel sums them; their owners' tasks are empty.
+template <typename T, typename V>
+__device__ __noinline__ T cl_long_sum(const ClMat<V>& mat, const ClSlice& s, int my_row, ClArray<T> vec, T t) {
+    __shared__ T red[32];
+    __shared__ T total;
+    const ClArray<int> longs{s.longs};
+    for (int i = 0; i < s.n_long; ++i) {
+        const int row = longs[3 * i];
+        const int64_t b = s.e0 + longs[3 * i + 1], e = b + longs[3 * i + 2];
+        T acc = T(0);
+        if (threadIdx.x < kThreads)
+            for (int64_t k = b + threadIdx.x; k < e; k += kThreads)
+                acc = fma(static_cast<T>(mat.val[k]), vec[mat.idx[k] - mat.idx_base], acc);
+        T v[1] = {acc};
+        block_reduce<OpSum, T, 1>(v, red);
+        if (threadIdx.x == 0) total = v[0];
+        __syncthreads();
+        if (my_row == row) t = total;
+        __syncthreads();
+    }
+    return t;
+}
+
+// The sum of my row in FP64 from FP64 values in global memory (the checks of FP32 iterations);
+// any order will do.
+template <typename T, typename V>
+__device__ __noinline__ double cl_sum64(const ClMat<V>& mat, const ClSlice& s, int my_row, const double* val, ClArray<T> vec) {
+    const int tpr = 1 << s.tpr_shift;
+    int64_t b = 0, e = 0;
+    if (my_row >= 0) { b = mat.ptr[s.b0 + my_row]; e = mat.ptr[s.b0 + my_row + 1]; }
+    double acc = 0.0;
+#pragma unroll 4
+    for (int64_t k = b + (threadIdx.x & (tpr - 1)); k < e; k += tpr)
+        acc = fma(__ldg(val + k), static_cast<double>(vec[__ldg(mat.idx + k) - mat.idx_base]), acc);
+#pragma unroll 1
+    for (int o = tpr >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+
+// One CTA's half-iterations.  T: vector type, V: value type.  What only some steps need stays in
+// the ClInfo in shared memory: kept in registers it pushed the iteration's into local memory.
+template <typename T, typename V>
+struct ClCore {
+    ClTask tc, tr;              // my column's and my row's task
+    ClArray<T> yf;              // full y; the full x_bar is at offset 0
+    int tpr_c, tpr_r;
+    uint32_t size, rank;
+    uint32_t peer_x, peer_y, peer_bar_x, peer_bar_y;   // thread t: my slices' places and the mbarriers in CTA t
+    uint32_t par_x = 0, par_y = 0;
+    bool dead = false;          // a wait ran out: no further waiting
+
+    __device__ __forceinline__ ClArray<T> xb() const { return ClArray<T>{0}; }
+
+    // False when a slice does not fit into this CTA (uniform over the CTA).  A cluster barrier has
+    // to follow before the first exchange.
+    __device__ __forceinline__ bool begin(const ClMat<V>& a, const ClMat<V>& at, uint32_t bytes, ClInfo& I) {
+        cl_begin<T, V>(a, at, bytes, I);
+        size = I.size;
+        rank = I.rank;
+        yf = ClArray<T>{cl_y_offset<T>(I.n)};
+        bool ok = false;
+        tc = cl_deal<V>(at, I.cols, yf.off, I.m, I, &ok);
+        if (!ok) return false;
+        tr = cl_deal<V>(a, I.rows, 0u, I.n, I, &ok);
+        const uint32_t peer = threadIdx.x < size ? threadIdx.x : rank;
+        peer_x = cl_map(smem_addr(xb().ptr() + I.cols.b0), peer);
+        peer_y = cl_map(smem_addr(yf.ptr() + I.rows.b0), peer);
+        peer_bar_x = cl_map(smem_addr(&I.bar_x), peer);
+        peer_bar_y = cl_map(smem_addr(&I.bar_y), peer);
+        tpr_c = 1 << I.cols.tpr_shift;
+        tpr_r = 1 << I.rows.tpr_shift;
+        return ok;
+    }
+    // The column / row this thread owns, -1: none.
+    __device__ __forceinline__ int my_col(const ClInfo& I) const { return tc.row >= 0 && (threadIdx.x & (tpr_c - 1)) == 0 ? I.cols.b0 + tc.row : -1; }
+    __device__ __forceinline__ int my_row(const ClInfo& I) const { return tr.row >= 0 && (threadIdx.x & (tpr_r - 1)) == 0 ? I.rows.b0 + tr.row : -1; }
+
+    __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
+        if (dead) return;
+#pragma unroll 1
+        for (int t = 0; t < kClWaitTries; ++t) {
+            uint32_t ok;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+            if (ok) return;
+        }
+        dead = true;
+    }
+    __device__ __forceinline__ static void push(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+        asm volatile(
+            "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+            ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
+    }
+    // Sends my slices (of x_bar, of y) to every peer and waits for theirs, on x_bar's or y's
+    // mbarrier.  A CTA without a slice of that vector signals the peers all the same, so that
+    // nobody runs ahead of it.  All threads; the writes to my slices come before it.
+    template <bool X, bool Y>
+    __device__ __forceinline__ void exchange(ClInfo& I) {
+        if (size == 1) { __syncthreads(); return; }
+        const uint32_t bar = smem_addr(Y ? &I.bar_y : &I.bar_x);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < size) {
+            if (threadIdx.x == rank) {
+                const uint32_t expect = (X ? I.expect_x : 0u) + (Y ? I.expect_y : 0u);
+                asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(expect) : "memory");
+            } else {
+                const uint32_t there = Y ? peer_bar_y : peer_bar_x;
+                const uint32_t bx = X ? I.bytes_x : 0u, by = Y ? I.bytes_y : 0u;
+                if (X && bx) push(peer_x, smem_addr(xb().ptr() + I.cols.b0), bx, there);
+                if (Y && by) push(peer_y, smem_addr(yf.ptr() + I.rows.b0), by, there);
+                if ((Y ? by : bx) == 0u)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(there) : "memory");
+            }
+        }
+        if constexpr (Y) { wait(bar, par_y); par_y ^= 1; }
+        else { wait(bar, par_x); par_x ^= 1; }
+    }
+    __device__ __forceinline__ void exchange_x(ClInfo& I) { exchange<true, false>(I); }
+    __device__ __forceinline__ void exchange_y(ClInfo& I) { exchange<false, true>(I); }
+    // Both at once, on y's mbarrier: only between two cluster barriers.
+    __device__ __forceinline__ void exchange_both(ClInfo& I) { exchange<true, true>(I); }
+
+    // The sum of my row against `vec`, valid in the row's owner.  All threads.
+    __device__ __forceinline__ static T sum(const ClTask& task, int tpr, const ClMat<V>& mat, const ClSlice& s, ClArray<T> vec) {
+        T t = cl_chains<T>(task);
+#pragma unroll 1
+        for (int o = tpr >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (s.n_long) t = cl_long_sum<T, V>(mat, s, task.row, vec, t);
+        return t;
+    }
+    __device__ __forceinline__ T col_sum(const ClMat<V>& at, const ClInfo& I) { return sum(tc, tpr_c, at, I.cols, yf); }
+    __device__ __forceinline__ T row_sum(const ClMat<V>& a, const ClInfo& I) { return sum(tr, tpr_r, a, I.rows, xb()); }
+};
+
+// Launches `kernel` on `clusters` clusters of `ctas` CTAs; errors are left for cudaGetLastError.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_clusters(void (*kernel)(Params...), int clusters, int ctas, int threads, size_t smem,
+                                   cudaStream_t st, Args&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(clusters) * ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    note_launch();
+    return e;
+}
+// Grants a kernel the shared memory and the cluster size of a launch; an error when the device has
+// no room for one such cluster.
+template <typename... Params>
+inline cudaError_t prepare_clusters(void (*kernel)(Params...), int ctas, int threads, size_t smem) {
+    const void* f = reinterpret_cast<const void*>(kernel);
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kClSmemCap));
+    if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess || ctas == 1) return e;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    e = cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg);
+    return e != cudaSuccess ? e : fit >= 1 ? cudaSuccess : cudaErrorInvalidConfiguration;
+}
+
+}  // namespace vajra

@@ -24,6 +24,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cluster.cuh"
 #include "halpern_state.cuh"
 #include "solver.cuh"
 
@@ -48,10 +49,69 @@ __device__ __forceinline__ void store_partials(double (&v)[kQ], double (&red)[kQ
         for (int q = 0; q < kQ; ++q) part[blockIdx.x * kQ + q] = v[q];
 }
 
-// Row pass: original- and scaled-space primal residual, row part of the dual objective,
-// distance of y+ from the last restart point, NaN detection, and the guard's maxima: the
-// row violation relative to 1 + |violated bound|, its absolute size, and the row dual's sign
+// One row's terms of a check: original- and scaled-space primal residual, row part of the dual
+// objective, distance of y+ from the last restart point, NaN detection, and the guard's maxima:
+// the row violation relative to 1 + |violated bound|, its absolute size, and the row dual's sign
 // violation (verifier convention: y <= 0 on a <= row, y >= 0 on a >= row).
+// sums: rp_o^2, rp_s^2, dobj, dy^2 (restart), dy^2 (step), -; maxima: nan, p_rel, p_abs, d_abs
+__device__ __forceinline__ void kkt_row_terms(double a, double ys, double yprev, double rl_s, double ru_s, double lo,
+                                              double up, double rs, double y_last, double (&v)[kQ]) {
+    if (!isfinite(a) || !isfinite(ys)) v[kNS] = 1.0;
+    const double fy = ys - yprev;
+    v[4] += fy * fy;
+    const double ps = a - fmin(fmax(a, rl_s), ru_s);
+    const double ao = a / rs;
+    const double po = ao - fmin(fmax(ao, lo), up);
+    const double yo = -ys * rs;          // verifier sign, original space
+    double dt = 0.0;
+    if (yo > 0.0 && finite_lo(lo)) dt = yo * lo;
+    else if (yo < 0.0 && finite_up(up)) dt = yo * up;
+    const double dy = ys - y_last;
+    v[0] += po * po;
+    v[1] += ps * ps;
+    v[2] += dt;
+    v[3] += dy * dy;
+    if (po != 0.0) {
+        const double bound = po < 0.0 ? (lo > -1e19 ? fabs(lo) : 1.0) : (up < 1e19 ? fabs(up) : 1.0);
+        v[kNS + 1] = fmax(v[kNS + 1], fabs(po) / (1.0 + bound));
+        v[kNS + 2] = fmax(v[kNS + 2], fabs(po));
+    }
+    if (!finite_lo(lo) && finite_up(up) && yo > 0.0) v[kNS + 3] = fmax(v[kNS + 3], yo);
+    if (finite_lo(lo) && !finite_up(up) && yo < 0.0) v[kNS + 3] = fmax(v[kNS + 3], -yo);
+}
+
+// One column's terms: reduced cost r = c + A^T y (min form), its bound-multiplier part lambda,
+// dual residual r - lambda (original and scaled), primal objective, column part of the dual
+// objective, distance of x+ from the last restart point, and the guard's reduced-cost sign
+// violation (a column more than 1e-7 below its upper bound may not have r < 0, one more than
+// 1e-7 above its lower bound may not have r > 0).
+// sums: rd_o^2, rd_s^2, pobj, dobj, dx^2 (restart), dx^2 (step); maxima: nan, -, -, d_abs
+__device__ __forceinline__ void kkt_col_terms(double at, double xs, double xprev, double c_s, double lo, double up,
+                                              double cs, double x_last, double (&v)[kQ]) {
+    if (!isfinite(at) || !isfinite(xs)) v[kNS] = 1.0;
+    const double fx = xs - xprev;
+    v[5] += fx * fx;
+    const bool lf = finite_lo(lo), uf = finite_up(up);
+    const double r_s = c_s + at;
+    const double r_o = r_s / cs;
+    auto lam_of = [&](double r) { return (lf && uf) ? r : lf ? fmax(r, 0.0) : uf ? fmin(r, 0.0) : 0.0; };
+    const double lo_lam = lam_of(r_o), ls = lam_of(r_s);
+    const double ro = r_o - lo_lam, rsd = r_s - ls;
+    double dt = 0.0;
+    if (lo_lam > 0.0) dt = lo_lam * lo;
+    else if (lo_lam < 0.0) dt = lo_lam * up;
+    const double dx = xs - x_last;
+    v[0] += ro * ro;
+    v[1] += rsd * rsd;
+    v[2] += c_s * xs;
+    v[3] += dt;
+    v[4] += dx * dx;
+    const double xo = xs * cs;
+    if (xo < up - kGuardTol && r_o < 0.0) v[kNS + 3] = fmax(v[kNS + 3], -r_o);
+    if (xo > lo + kGuardTol && r_o > 0.0) v[kNS + 3] = fmax(v[kNS + 3], r_o);
+}
+
+// Row pass and column pass of a check: block partials of the terms above.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_kkt_rows(int m, const double* __restrict__ ax, const T* __restrict__ yc, const T* __restrict__ yprev,
@@ -60,43 +120,13 @@ k_kkt_rows(int m, const double* __restrict__ ax, const T* __restrict__ yc, const
            double* __restrict__ part, const HState* st, int phase) {
     if (st->stop || st->phase != phase) return;
     __shared__ double red[kQ * 32];
-    // sums: rp_o^2, rp_s^2, dobj, dy^2 (restart), dy^2 (step), -; maxima: nan, p_rel, p_abs, d_abs
     double v[kQ] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        const double a = ax[i];
-        const double ys = static_cast<double>(yc[i]);
-        if (!isfinite(a) || !isfinite(ys)) v[kNS] = 1.0;
-        const double fy = ys - static_cast<double>(yprev[i]);
-        v[4] += fy * fy;
-        const double ps = a - fmin(fmax(a, rl_s[i]), ru_s[i]);
-        const double ao = a / rs[i];
-        const double lo = rl_o[i], up = ru_o[i];
-        const double po = ao - fmin(fmax(ao, lo), up);
-        const double yo = -ys * rs[i];          // verifier sign, original space
-        double dt = 0.0;
-        if (yo > 0.0 && finite_lo(lo)) dt = yo * lo;
-        else if (yo < 0.0 && finite_up(up)) dt = yo * up;
-        const double dy = ys - y_last[i];
-        v[0] += po * po;
-        v[1] += ps * ps;
-        v[2] += dt;
-        v[3] += dy * dy;
-        if (po != 0.0) {
-            const double bound = po < 0.0 ? (lo > -1e19 ? fabs(lo) : 1.0) : (up < 1e19 ? fabs(up) : 1.0);
-            v[kNS + 1] = fmax(v[kNS + 1], fabs(po) / (1.0 + bound));
-            v[kNS + 2] = fmax(v[kNS + 2], fabs(po));
-        }
-        if (!finite_lo(lo) && finite_up(up) && yo > 0.0) v[kNS + 3] = fmax(v[kNS + 3], yo);
-        if (finite_lo(lo) && !finite_up(up) && yo < 0.0) v[kNS + 3] = fmax(v[kNS + 3], -yo);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+        kkt_row_terms(ax[i], static_cast<double>(yc[i]), static_cast<double>(yprev[i]), rl_s[i], ru_s[i], rl_o[i],
+                      ru_o[i], rs[i], y_last[i], v);
     store_partials(v, red, part);
 }
 
-// Column pass: reduced cost r = c + A^T y (min form), its bound-multiplier part lambda,
-// dual residual r - lambda (original and scaled), primal objective, column part of the dual
-// objective, distance of x+ from the last restart point, and the guard's reduced-cost sign
-// violation (a column more than 1e-7 below its upper bound may not have r < 0, one more than
-// 1e-7 above its lower bound may not have r > 0).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_kkt_cols(int n, const double* __restrict__ aty, const T* __restrict__ xc, const T* __restrict__ xprev,
@@ -105,34 +135,10 @@ k_kkt_cols(int n, const double* __restrict__ aty, const T* __restrict__ xc, cons
            const HState* st, int phase) {
     if (st->stop || st->phase != phase) return;
     __shared__ double red[kQ * 32];
-    // sums: rd_o^2, rd_s^2, pobj, dobj, dx^2 (restart), dx^2 (step); maxima: nan, -, -, d_abs
     double v[kQ] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const double at = aty[j];
-        const double xs = static_cast<double>(xc[j]);
-        if (!isfinite(at) || !isfinite(xs)) v[kNS] = 1.0;
-        const double fx = xs - static_cast<double>(xprev[j]);
-        v[5] += fx * fx;
-        const double lo = cl_o[j], up = cu_o[j];
-        const bool lf = finite_lo(lo), uf = finite_up(up);
-        const double r_s = c_s[j] + at;
-        const double r_o = r_s / cs[j];
-        auto lam_of = [&](double r) { return (lf && uf) ? r : lf ? fmax(r, 0.0) : uf ? fmin(r, 0.0) : 0.0; };
-        const double lo_lam = lam_of(r_o), ls = lam_of(r_s);
-        const double ro = r_o - lo_lam, rsd = r_s - ls;
-        double dt = 0.0;
-        if (lo_lam > 0.0) dt = lo_lam * lo;
-        else if (lo_lam < 0.0) dt = lo_lam * up;
-        const double dx = xs - x_last[j];
-        v[0] += ro * ro;
-        v[1] += rsd * rsd;
-        v[2] += c_s[j] * xs;
-        v[3] += dt;
-        v[4] += dx * dx;
-        const double xo = xs * cs[j];
-        if (xo < up - kGuardTol && r_o < 0.0) v[kNS + 3] = fmax(v[kNS + 3], -r_o);
-        if (xo > lo + kGuardTol && r_o > 0.0) v[kNS + 3] = fmax(v[kNS + 3], r_o);
-    }
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        kkt_col_terms(aty[j], static_cast<double>(xc[j]), static_cast<double>(xprev[j]), c_s[j], cl_o[j], cu_o[j],
+                      cs[j], x_last[j], v);
     store_partials(v, red, part);
 }
 
@@ -158,30 +164,10 @@ struct ControlParams {
 
 constexpr int kS = 2 * kNS;   // sums the control CTA combines (rows, then columns)
 
-__global__ void __launch_bounds__(1024)
-k_halpern_control(const double* __restrict__ part_r, const double* __restrict__ part_c, ControlParams cp,
-                  HState* st) {
-    if (st->stop || st->phase != cp.phase) return;
-    __shared__ double red[kS * 32];
-    double s[kS];
-#pragma unroll
-    for (int q = 0; q < kS; ++q) s[q] = 0.0;
-    for (int b = threadIdx.x; b < kCheckBlocks; b += blockDim.x) {
-        for (int q = 0; q < kNS; ++q) { s[q] += part_r[b * kQ + q]; s[kNS + q] += part_c[b * kQ + q]; }
-    }
-    block_reduce<OpSum, double, kS>(s, red);
-    // maxima: NaN flag, relative and absolute row violation, dual sign violation
-    double f[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < kCheckBlocks; b += blockDim.x) {
-        const double* r = part_r + b * kQ + kNS;
-        const double* c = part_c + b * kQ + kNS;
-        f[0] = fmax(f[0], fmax(r[0], c[0]));
-        f[1] = fmax(f[1], r[1]);
-        f[2] = fmax(f[2], r[2]);
-        f[3] = fmax(f[3], fmax(r[3], c[3]));
-    }
-    block_reduce<OpMax, double, 4>(f, red);
-    if (threadIdx.x != 0) return;
+// The decisions after a check, by one thread: `s` the combined sums (rows, then columns), `f` the
+// maxima (NaN flag, relative and absolute row violation, dual sign violation).
+__device__ __forceinline__ void halpern_decide(const double (&s)[kS], const double (&f)[4], const ControlParams& cp,
+                                               HState* st) {
     const double rp_o2 = s[0], rp_s2 = s[1], dobj_r = s[2], dy2 = s[3], fy2 = s[4];
     const double rd_o2 = s[kNS], rd_s2 = s[kNS + 1], pobj_s = s[kNS + 2], dobj_c = s[kNS + 3], dx2 = s[kNS + 4],
                  fx2 = s[kNS + 5];
@@ -266,6 +252,33 @@ k_halpern_control(const double* __restrict__ part_r, const double* __restrict__ 
     } else {
         st->k_base = k_in;
     }
+}
+
+__global__ void __launch_bounds__(1024)
+k_halpern_control(const double* __restrict__ part_r, const double* __restrict__ part_c, ControlParams cp,
+                  HState* st) {
+    if (st->stop || st->phase != cp.phase) return;
+    __shared__ double red[kS * 32];
+    double s[kS];
+#pragma unroll
+    for (int q = 0; q < kS; ++q) s[q] = 0.0;
+    for (int b = threadIdx.x; b < kCheckBlocks; b += blockDim.x) {
+        for (int q = 0; q < kNS; ++q) { s[q] += part_r[b * kQ + q]; s[kNS + q] += part_c[b * kQ + q]; }
+    }
+    block_reduce<OpSum, double, kS>(s, red);
+    // maxima: NaN flag, relative and absolute row violation, dual sign violation
+    double f[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < kCheckBlocks; b += blockDim.x) {
+        const double* r = part_r + b * kQ + kNS;
+        const double* c = part_c + b * kQ + kNS;
+        f[0] = fmax(f[0], fmax(r[0], c[0]));
+        f[1] = fmax(f[1], r[1]);
+        f[2] = fmax(f[2], r[2]);
+        f[3] = fmax(f[3], fmax(r[3], c[3]));
+    }
+    block_reduce<OpMax, double, 4>(f, red);
+    if (threadIdx.x != 0) return;
+    halpern_decide(s, f, cp, st);
 }
 
 template <typename T>
@@ -517,6 +530,250 @@ void enqueue_iteration(Phase<T>& ph, const CsrView& a, const CsrView& at, HState
     if (timed) cudaEventRecordWithFlags(ph.ev[2], st, cudaEventRecordExternal);
 }
 
+// ----- cluster-resident iterations (cluster.cuh) ------------------------------------------
+// One LP as the cluster kernel reads it: matrices in the phase's precision and in FP64 (checks),
+// the phase's vectors, the checks' vectors.
+template <typename T>
+struct ClHalpern {
+    ClMat<T> a, at;
+    const double* a64; const double* at64;
+    const T* c; const T* cl; const T* cu; const T* rl; const T* ru;
+    T* x; T* x0; T* xc; T* xprev; T* y; T* y0; T* yc; T* yprev;
+    const double* c_s; const double* cl_o; const double* cu_o; const double* cs;
+    const double* rl_s; const double* ru_s; const double* rl_o; const double* ru_o; const double* rs;
+    double* x_last; double* y_last;
+};
+constexpr int kClWeights = 128;   // Halpern weights kept ahead
+
+__device__ __forceinline__ unsigned long long ns_now() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The parts of a check outside the row sums, out of line: inlined, their registers would push
+// the iteration's into local memory.  One value of each kind per thread: the warps' partials go
+// to shared memory, and a thread per quantity adds them up.
+constexpr int kClWarps = kClThreads / 32;
+template <typename T>
+__device__ __noinline__ void cl_check_partials(const ClHalpern<T>& P, int i, double ax, int j, double aty,
+                                               double (&red)[2 * kQ * kClWarps], double* part) {
+    double v[2 * kQ];
+#pragma unroll
+    for (int q = 0; q < 2 * kQ; ++q) v[q] = 0.0;
+    if (i >= 0)
+        kkt_row_terms(ax, static_cast<double>(P.yc[i]), static_cast<double>(P.yprev[i]), P.rl_s[i], P.ru_s[i], P.rl_o[i],
+                      P.ru_o[i], P.rs[i], P.y_last[i], *reinterpret_cast<double(*)[kQ]>(v));
+    if (j >= 0)
+        kkt_col_terms(aty, static_cast<double>(P.xc[j]), static_cast<double>(P.xprev[j]), P.c_s[j], P.cl_o[j], P.cu_o[j],
+                      P.cs[j], P.x_last[j], *reinterpret_cast<double(*)[kQ]>(v + kQ));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 2 * kQ; ++q) {
+        v[q] = q % kQ < kNS ? warp_reduce<OpSum>(v[q]) : warp_reduce<OpMax>(v[q]);
+        if (lane == 0) red[q * kClWarps + warp] = v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kQ) {
+        const bool is_max = threadIdx.x % kQ >= kNS;
+        double t = 0.0;
+        for (int w = 0; w < warps; ++w) {
+            const double p = red[threadIdx.x * kClWarps + w];
+            t = is_max ? fmax(t, p) : t + p;
+        }
+        part[threadIdx.x] = t;
+    }
+}
+// Rank 0, all threads: the peers' partials combined, the decision taken on the copy `now` of
+// the state, and the state written back.
+__device__ __noinline__ void cl_decide(const double* part, int ctas, double (&red)[2 * kQ * kClWarps], ControlParams& cp, HState& now,
+                                       HState* st, double ns_primal, double ns_dual) {
+    const int tid = threadIdx.x;
+    if (tid < 2 * kQ) {   // thread q: rows' quantity q, thread kQ + q: columns'
+        const bool is_max = tid % kQ >= kNS;
+        double t = 0.0;
+        for (int r = 0; r < ctas; ++r) {
+            const double p = __ldcg(part + 2 * r * kQ + tid);
+            t = is_max ? fmax(t, p) : t + p;
+        }
+        red[tid] = t;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double s[kS], f[4];
+        for (int q = 0; q < kNS; ++q) { s[q] = red[q]; s[kNS + q] = red[kQ + q]; }
+        f[0] = fmax(red[kNS], red[kQ + kNS]);
+        f[1] = red[kNS + 1];
+        f[2] = red[kNS + 2];
+        f[3] = fmax(red[kNS + 3], red[kQ + kNS + 3]);
+        now.wait_error = *static_cast<volatile int*>(&st->wait_error);
+        halpern_decide(s, f, cp, &now);
+        if (now.wait_error) now.stop = 1;
+        if (ns_primal > 0.0) {
+            now.t_primal_ns[cp.phase] += ns_primal;
+            now.t_dual_ns[cp.phase] += ns_dual;
+            now.t_samples[cp.phase] += 1;
+        }
+    }
+    __syncthreads();
+    for (int q = tid; q < static_cast<int>(sizeof(HState) / 4); q += blockDim.x)
+        reinterpret_cast<int*>(st)[q] = reinterpret_cast<const int*>(&now)[q];
+}
+
+// Up to max_chunks chunks of `K` iterations and a check each (the last one shorter where the
+// iteration budget ends), until the LP stops or leaves the phase.  One cluster.  The arithmetic
+// is that of the kernels above: an iteration and a check differ only in where the data is and
+// in the order of the checks' FP64 sums.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_cluster_halpern(const __grid_constant__ ClHalpern<T> P, const __grid_constant__ ControlParams cp0, HState* st, double* part,
+                  int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ double red[2 * kQ * kClWarps];
+    __shared__ T hw[2 * kClWeights];
+    __shared__ HState now;
+    __shared__ ControlParams cp;
+    const int phase = cp0.phase;
+    if (st->stop || st->phase != phase) return;   // uniform over the cluster
+    ClCore<T, T> core;
+    if (!core.begin(P.a, P.at, smem_bytes, I) && threadIdx.x == 0) st->no_fit = 1;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < I.m; i += NT) core.yf[i] = P.y[i];
+    if (tid == 0) cp = cp0;
+    cl_barrier();
+    if (*static_cast<volatile int*>(&st->no_fit)) return;   // the host takes the general path
+    // My column and my row, if I own one (-1: none).
+    const int j = core.my_col(I), i = core.my_row(I);
+    T x = T(0), x0 = T(0), c = T(0), cl = T(0), cu = T(0), y0 = T(0), rl = T(0), ru = T(0);
+    if (j >= 0) { x = P.x[j]; x0 = P.x0[j]; c = P.c[j]; cl = P.cl[j]; cu = P.cu[j]; }
+    T y = T(0);
+    if (i >= 0) { y = P.y[i]; y0 = P.y0[i]; rl = P.rl[i]; ru = P.ru[i]; }
+    // The solver's state: every CTA copies it into shared memory; rank 0 decides there and
+    // writes it back (a decision that read it from global memory waited for a dozen L2 loads).
+    static_assert(sizeof(HState) % 4 == 0, "HState is copied in words");
+    auto read_state = [&]() {   // written by rank 0 before a cluster barrier, or by the host
+        for (int q = tid; q < static_cast<int>(sizeof(HState) / 4); q += NT)
+            reinterpret_cast<int*>(&now)[q] = __ldcg(reinterpret_cast<const int*>(st) + q);
+        __syncthreads();
+    };
+    read_state();
+    for (int chunk = 0; chunk < max_chunks && budget > 0; ++chunk) {
+        const int len = budget < K ? static_cast<int>(budget) : K;
+        budget -= len;
+        const T tau = static_cast<T>(now.tau), sigma = static_cast<T>(now.sigma), inv_sigma = static_cast<T>(now.inv_sigma),
+                g = static_cast<T>(now.gamma_now);
+        unsigned int t0 = 0, t1 = 0, t2 = 0;
+        // Turn kk < len is an iteration.  Turn len forms the check's products: the candidate takes
+        // the place of x_bar and y in the full vectors.
+#pragma unroll 1
+        for (int kk = 0; kk <= len; ++kk) {
+            const bool check = kk == len;
+            const int slot = kk & (kClWeights - 1);
+            if (slot == 0) {   // everyone is past the last use of the old weights
+                const long long k_base = now.k_base;
+                for (int q = tid; q < kClWeights; q += NT) {
+                    const double k = static_cast<double>(k_base + kk + q);
+                    hw[2 * q] = static_cast<T>((k + 1.0) / (k + 2.0));
+                    hw[2 * q + 1] = static_cast<T>(1.0 / (k + 2.0));
+                }
+                __syncthreads();
+            }
+            if (kk == 1) t0 = static_cast<unsigned int>(ns_now());
+            if (check) {
+                cl_barrier();   // every row sum is done with x_bar
+                if (j >= 0) core.xb()[j] = P.xc[j];
+                if (i >= 0) core.yf[i] = P.yc[i];
+                core.exchange_both(I);
+                if constexpr (sizeof(T) == 4) {   // FP64 values, from global memory
+                    const double ax = cl_sum64<T, T>(P.a, I.rows, core.tr.row, P.a64, core.xb());
+                    const double aty = cl_sum64<T, T>(P.at, I.cols, core.tc.row, P.at64, core.yf);
+                    cl_check_partials<T>(P, i, ax, j, aty, red, part + 2 * core.rank * kQ);
+                    break;
+                }
+            }
+            const T w1 = hw[2 * slot], w0 = hw[2 * slot + 1];
+            const T v = core.col_sum(P.at, I);
+            if (!check) {
+                if (j >= 0) {
+                    const T xo = x;
+                    T xp, xbn;
+                    halpern_primal(xo, v, c, cl, cu, x0, tau, w1, w0, g, &xp, &xbn, &x);
+                    core.xb()[j] = xbn;
+                    if (kk == len - 1) { P.xc[j] = xp; P.xprev[j] = xo; }
+                }
+                core.exchange_x(I);
+                if (kk == 1) t1 = static_cast<unsigned int>(ns_now());
+            }
+            const T w = core.row_sum(P.a, I);
+            if (!check) {
+                if (i >= 0) {
+                    const T yo = y;
+                    T yp;
+                    halpern_dual(yo, w, rl, ru, y0, sigma, inv_sigma, w1, w0, g, &yp, &y);
+                    core.yf[i] = y;
+                    if (kk == len - 1) { P.yc[i] = yp; P.yprev[i] = yo; }
+                }
+                if (kk < len - 1) core.exchange_y(I);
+                if (kk == 1) t2 = static_cast<unsigned int>(ns_now());
+            } else {
+                cl_check_partials<T>(P, i, static_cast<double>(w), j, static_cast<double>(v), red, part + 2 * core.rank * kQ);
+            }
+        }
+        if (core.dead) st->wait_error = 1;
+        if (tid == 0) cp.len = len;
+        cl_barrier();
+        if (core.rank == 0)
+            cl_decide(part, static_cast<int>(core.size), red, cp, now, st, len > 2 ? static_cast<double>(t1 - t0) : 0.0,
+                      static_cast<double>(t2 - t1));
+        cl_barrier();
+        read_state();
+        if (now.restart_flag) {
+            if (j >= 0) { x = x0 = P.xc[j]; P.x_last[j] = static_cast<double>(x); }
+            if (i >= 0) { y = y0 = P.yc[i]; P.y_last[i] = static_cast<double>(y); }
+        }
+        if (now.stop || now.phase != phase) break;
+        if (i >= 0) core.yf[i] = y;
+        core.exchange_y(I);
+    }
+    if (j >= 0) { P.x[j] = x; P.x0[j] = x0; }
+    if (i >= 0) { P.y[i] = y; P.y0[i] = y0; }
+    cl_barrier();   // no CTA ends while a peer may still send to it
+}
+
+// How an LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
+struct ClusterPlan { int ctas = 0, threads = 0; size_t smem = 0; };
+
+template <typename T>
+auto cluster_kernel(int threads) -> decltype(&k_cluster_halpern<T, 256>) {
+    return threads == 256 ? &k_cluster_halpern<T, 256> : &k_cluster_halpern<T, 512>;
+}
+
+// The smallest cluster whose CTAs have at most 256 rows and columns and about 1,000 entries of
+// each matrix, else 16 CTAs of up to 512.  Fewer CTAs exchange faster (0.6 us for 8, 0.8 us for
+// 16), more share the row sums; 256 threads pass a CTA's barriers faster than 512.  Microseconds
+// an iteration (FP32 / FP64; two launches an iteration: 5.5 to 6.8), checks included: 60 x 150 on
+// 1 CTA 1.2 / 1.3, on 4 1.7 / 1.7; 301 x 807 on 4 CTAs 1.9 / 2.1, on 8 1.9 / 2.1; 2000 x 5000 on
+// 16 CTAs of 512 threads 3.4 / 4.9; 5000 x 12000 (1,024 threads) 8.4 against 7.2, which is why the
+// line lies at 512.  Every thread forms at most kClMaxChains chains of a row.
+template <typename T>
+ClusterPlan plan_cluster(const CsrView& a, const CsrView& at, int64_t nnz) {
+    const auto lanes = [](const CsrView& v) { return v.group >= 1 && v.group <= 32; };
+    if (!lanes(a) || !lanes(at) || a.rows >= 65535 || at.rows >= 65535) return {};
+    for (int ctas = 1; ctas <= kClMaxCtas; ctas *= 2) {
+        const int64_t nr = cl_slice_rows(a.rows, nnz, ctas), nc = cl_slice_rows(at.rows, nnz, ctas);
+        const int threads = std::max(nr, nc) <= 256 ? 256 : 512;
+        // chains a thread forms, from an equal share (a CTA that gets more says so: no_fit)
+        const int64_t chains = std::max(a.rows / ctas * static_cast<int64_t>(a.group), at.rows / ctas * static_cast<int64_t>(at.group)) / threads;
+        if (std::max(nr, nc) > threads || chains >= kClMaxChains) continue;
+        if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
+        if (cl_smem_bytes(sizeof(T), sizeof(T), a.rows, at.rows, nnz, ctas, threads) > kClSmemCap) continue;
+        const cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
+        if (e != cudaSuccess) { cudaGetLastError(); continue; }   // no such cluster on this device
+        return ClusterPlan{ctas, threads, kClSmemCap};   // all of it: slices may be uneven
+    }
+    return {};
+}
+
 struct CheckBuffers {
     DeviceBuffer<double> ax, aty, part_r, part_c, x_last, y_last;
     DeviceBuffer<double> hw;   // Halpern weights of the current chunk (2 per iteration)
@@ -663,6 +920,16 @@ std::mutex g_tune_mutex;
 std::map<TuneKey, TuneEntry> g_tune_cache;
 
 }  // namespace
+
+// Chunks of the next launch of several: a first short launch, then what fits in the time left at
+// the rate measured so far, all that a launch may run where there is no limit to speak of.
+static int64_t launch_chunks(int64_t ran, double seconds, double left) {
+    constexpr int64_t kFirst = 16, kMost = 4096;
+    if (left > 1e9) return kMost;
+    if (ran == 0 || seconds <= 0.0) return kFirst;
+    const double fit = left * static_cast<double>(ran) / seconds;
+    return fit >= static_cast<double>(kMost) ? kMost : (fit < 1.0 ? 1 : static_cast<int64_t>(fit));
+}
 
 vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     const auto t_start = Clock::now();
@@ -917,59 +1184,109 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     cp.stall_checks = o.mixed_stall_checks < 0 ? 0 : (o.mixed_stall_checks > kHist - 1 ? kHist - 1 : o.mixed_stall_checks);
     const int64_t max_iter = o.iteration_limit;
 
+    // Small LPs: each phase runs on one thread-block cluster, many chunks a launch, unless the
+    // caller fixed a launch shape.
+    const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0 && nnz < kAutotuneMinNnz;
+    ClusterPlan cl32, cl64;
+    DeviceBuffer<double> cl_part;
+    if (may_cluster) {
+        if (mixed) cl32 = plan_cluster<float>(a32, at32, nnz);
+        cl64 = plan_cluster<double>(a64, at64, nnz);
+        if (cl32.ctas || cl64.ctas) VJ_TRY(cl_part.alloc(2 * kQ * kClMaxCtas));
+    }
+    auto cluster_chunks = [&](auto& ph, const ClusterPlan& plan, int64_t budget, int chunks) -> vajra_status {
+        using T = std::decay_t<decltype(*ph.x.get())>;
+        ClHalpern<T> P;
+        const CsrView& ia = ph.phase == 0 ? a32 : a64;
+        const CsrView& iat = ph.phase == 0 ? at32 : at64;
+        P.a = ClMat<T>{m, p.csr_ptr.get(), p.csr_idx.get(), ph.csr_val, 0, ia.group, ia.long_len};
+        P.at = ClMat<T>{n, lp.col_ptr.get(), lp.row_idx.get(), ph.csc_val, 0, iat.group, iat.long_len};
+        P.a64 = p.csr_val.get(); P.at64 = p.csc_val.get();
+        P.c = ph.c.get(); P.cl = ph.cl.get(); P.cu = ph.cu.get(); P.rl = ph.rl.get(); P.ru = ph.ru.get();
+        P.x = ph.x.get(); P.x0 = ph.x0.get(); P.xc = ph.xc.get(); P.xprev = ph.xprev.get();
+        P.y = ph.y.get(); P.y0 = ph.y0.get(); P.yc = ph.yc.get(); P.yprev = ph.yprev.get();
+        P.c_s = p.c.get(); P.cl_o = lp.col_lower.get(); P.cu_o = lp.col_upper.get(); P.cs = p.col_scale.get();
+        P.rl_s = p.row_lower.get(); P.ru_s = p.row_upper.get();
+        P.rl_o = lp.row_lower.get(); P.ru_o = lp.row_upper.get(); P.rs = p.row_scale.get();
+        P.x_last = cb.x_last.get(); P.y_last = cb.y_last.get();
+        ControlParams c2 = cp;
+        c2.phase = ph.phase;
+        VJ_CUDA(launch_clusters(cluster_kernel<T>(plan.threads), 1, plan.ctas, plan.threads, plan.smem, st, P, c2, S, cl_part.get(), K,
+                                static_cast<long long>(budget), chunks, static_cast<uint32_t>(plan.smem)));
+        return VAJRA_OK;
+    };
     const auto t_iter = Clock::now();
     int64_t launched = 0;
     int cur_phase = mixed ? 0 : 1;
     int timed_out = 0;
+    int64_t cl_chunks = 0;   // chunks the clusters of this solve have run, and their host time
+    double cl_seconds = 0.0;
     while (launched < max_iter) {
-        const int64_t remaining = max_iter - launched;
-        const int len = static_cast<int>(remaining < K ? remaining : K);
-        auto run_chunk = [&](auto& ph) -> vajra_status {
-            const CsrView& ia = ph.phase == 0 ? a32 : a64;
-            const CsrView& iat = ph.phase == 0 ? at32 : at64;
-            if (len == K) {
-                if (!ph.exec) {
-                    const auto t_graph = Clock::now();
-                    const int64_t before = launch_count();
-                    VJ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                    enqueue_chunk(ph, ia, iat, a64, at64, p, lp, cb, S, len, cp, true, st);
-                    VJ_CUDA(cudaStreamEndCapture(st, &ph.graph));
-                    VJ_CUDA(cudaGraphInstantiate(&ph.exec, ph.graph, 0));
-                    ph.graph_kernels = launch_count() - before;
-                    launch_count() = before;
-                    if (o.verbose)
-                        std::fprintf(stderr, "[vajra] chunk graph of phase %d (%lld kernels): capture + instantiate %.2f ms\n",
-                                     ph.phase, static_cast<long long>(ph.graph_kernels), 1e3 * seconds_since(t_graph));
+        const ClusterPlan& plan = cur_phase == 0 ? cl32 : cl64;
+        if (plan.ctas) {
+            const int64_t chunks = o.verbose ? 1 : launch_chunks(cl_chunks, cl_seconds, o.time_limit - seconds_since(t_start));
+            const auto t_launch = Clock::now();
+            if (cur_phase == 0) { VJ_TRY(cluster_chunks(p32, plan, max_iter - launched, static_cast<int>(chunks))); }
+            else { VJ_TRY(cluster_chunks(p64, plan, max_iter - launched, static_cast<int>(chunks))); }
+            VJ_CUDA(cudaMemcpyAsync(hs, S, sizeof(HState), cudaMemcpyDeviceToHost, st));
+            VJ_CUDA(cudaStreamSynchronize(st));
+            h->transfers++;
+            if (hs->wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
+            cl_seconds += seconds_since(t_launch);
+            cl_chunks += (hs->total - launched + K - 1) / K;
+            if (hs->no_fit) { cl32.ctas = cl64.ctas = 0; continue; }   // uneven rows: the general path
+            if (hs->total <= launched) return VAJRA_ERR_INTERNAL;   // a launch runs at least one chunk
+            launched = hs->total;
+        } else {
+            const int64_t remaining = max_iter - launched;
+            const int len = static_cast<int>(remaining < K ? remaining : K);
+            auto run_chunk = [&](auto& ph) -> vajra_status {
+                const CsrView& ia = ph.phase == 0 ? a32 : a64;
+                const CsrView& iat = ph.phase == 0 ? at32 : at64;
+                if (len == K) {
+                    if (!ph.exec) {
+                        const auto t_graph = Clock::now();
+                        const int64_t before = launch_count();
+                        VJ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+                        enqueue_chunk(ph, ia, iat, a64, at64, p, lp, cb, S, len, cp, true, st);
+                        VJ_CUDA(cudaStreamEndCapture(st, &ph.graph));
+                        VJ_CUDA(cudaGraphInstantiate(&ph.exec, ph.graph, 0));
+                        ph.graph_kernels = launch_count() - before;
+                        launch_count() = before;
+                        if (o.verbose)
+                            std::fprintf(stderr, "[vajra] chunk graph of phase %d (%lld kernels): capture + instantiate %.2f ms\n",
+                                         ph.phase, static_cast<long long>(ph.graph_kernels), 1e3 * seconds_since(t_graph));
+                    }
+                    VJ_CUDA(cudaGraphLaunch(ph.exec, st));
+                    note_launch(ph.graph_kernels);
+                } else {
+                    enqueue_chunk(ph, ia, iat, a64, at64, p, lp, cb, S, len, cp, false, st);
+                    VJ_LAUNCH_CHECK();
                 }
-                VJ_CUDA(cudaGraphLaunch(ph.exec, st));
-                note_launch(ph.graph_kernels);
-            } else {
-                enqueue_chunk(ph, ia, iat, a64, at64, p, lp, cb, S, len, cp, false, st);
-                VJ_LAUNCH_CHECK();
+                return VAJRA_OK;
+            };
+            if (cur_phase == 0) { VJ_TRY(run_chunk(p32)); } else { VJ_TRY(run_chunk(p64)); }
+            launched += len;
+            VJ_CUDA(cudaMemcpyAsync(hs, S, sizeof(HState), cudaMemcpyDeviceToHost, st));
+            VJ_CUDA(cudaStreamSynchronize(st));
+            h->transfers++;
+            // Kernel durations of this chunk's first iteration, unless that phase had stopped
+            // working before the chunk began (then its kernels returned at once).
+            if (len > 1 && (hs->phase == cur_phase || hs->switch_flag) &&
+                !(hs->stop && hs->stop_iter < launched - len + 1)) {
+                float t01 = 0.f, t12 = 0.f;
+                cudaEvent_t* ev = cur_phase == 0 ? p32.ev : p64.ev;
+                if (cudaEventElapsedTime(&t01, ev[0], ev[1]) == cudaSuccess &&
+                    cudaEventElapsedTime(&t12, ev[1], ev[2]) == cudaSuccess) {
+                    auto& ph_t = cur_phase == 0 ? p32.t_primal_ms : p64.t_primal_ms;
+                    auto& ph_d = cur_phase == 0 ? p32.t_dual_ms : p64.t_dual_ms;
+                    auto& ph_n = cur_phase == 0 ? p32.samples : p64.samples;
+                    ph_t += t01;
+                    ph_d += t12;
+                    ph_n += 1;
+                }
+                cudaGetLastError();
             }
-            return VAJRA_OK;
-        };
-        if (cur_phase == 0) { VJ_TRY(run_chunk(p32)); } else { VJ_TRY(run_chunk(p64)); }
-        launched += len;
-        VJ_CUDA(cudaMemcpyAsync(hs, S, sizeof(HState), cudaMemcpyDeviceToHost, st));
-        VJ_CUDA(cudaStreamSynchronize(st));
-        h->transfers++;
-        // Kernel durations of this chunk's first iteration, unless that phase had stopped
-        // working before the chunk began (then its kernels returned at once).
-        if (len > 1 && (hs->phase == cur_phase || hs->switch_flag) &&
-            !(hs->stop && hs->stop_iter < launched - len + 1)) {
-            float t01 = 0.f, t12 = 0.f;
-            cudaEvent_t* ev = cur_phase == 0 ? p32.ev : p64.ev;
-            if (cudaEventElapsedTime(&t01, ev[0], ev[1]) == cudaSuccess &&
-                cudaEventElapsedTime(&t12, ev[1], ev[2]) == cudaSuccess) {
-                auto& ph_t = cur_phase == 0 ? p32.t_primal_ms : p64.t_primal_ms;
-                auto& ph_d = cur_phase == 0 ? p32.t_dual_ms : p64.t_dual_ms;
-                auto& ph_n = cur_phase == 0 ? p32.samples : p64.samples;
-                ph_t += t01;
-                ph_d += t12;
-                ph_n += 1;
-            }
-            cudaGetLastError();
         }
         if (hs->stop) break;
         if (hs->phase != cur_phase) {
@@ -1088,8 +1405,11 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
         const double vs = use32 ? 4.0 : 8.0;                        // vector bytes
         const double vb = (use32 || p64.compact) ? 4.0 : 8.0;       // matrix value bytes
         const double nn = static_cast<double>(nnz), dm = m, dn = n;
-        const double t = use32 ? p32.t_primal_ms : p64.t_primal_ms, d = use32 ? p32.t_dual_ms : p64.t_dual_ms;
-        const int64_t ns = use32 ? p32.samples : p64.samples;
+        const bool on_cluster = (use32 ? cl32.ctas : cl64.ctas) > 0;
+        const int ph_i = use32 ? 0 : 1;
+        const double t = on_cluster ? 1e-6 * hs->t_primal_ns[ph_i] : use32 ? p32.t_primal_ms : p64.t_primal_ms;
+        const double d = on_cluster ? 1e-6 * hs->t_dual_ns[ph_i] : use32 ? p32.t_dual_ms : p64.t_dual_ms;
+        const int64_t ns = on_cluster ? hs->t_samples[ph_i] : use32 ? p32.samples : p64.samples;
         r->kernel_samples = ns;
         r->primal_kernel_us = ns ? 1e3 * t / ns : 0.0;
         r->dual_kernel_us = ns ? 1e3 * d / ns : 0.0;

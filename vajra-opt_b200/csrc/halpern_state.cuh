@@ -28,13 +28,40 @@ struct HState {
     int restart_count;
     int restart_flag;
     int switch_flag;
+    int wait_error;     // a bounded device wait ran out (cluster path)
+    int no_fit;         // a CTA's slices do not fit its shared memory (cluster path)
     int pad;
+    // first iteration of every chunk of the cluster path: nanoseconds of its two halves
+    double t_primal_ns[2], t_dual_ns[2];   // per phase
+    long long t_samples[2];
 };
 
 constexpr int kStatusOptimal = 1;
 constexpr int kStatusIterLimit = 6;
 constexpr int kStatusTimeLimit = 7;
 constexpr int kStatusNumerical = 9;
+
+// One column's primal half: x+ and x_bar from the row sum v = (A^T y)_j, and the Halpern step.
+template <typename T>
+__device__ __forceinline__ void halpern_primal(T xo, T v, T c, T cl, T cu, T x0, T tau, T w1, T w0, T g, T* xp_out,
+                                               T* xb_out, T* x_out) {
+    T xp = xo - tau * (c + v);
+    xp = xp < cl ? cl : (xp > cu ? cu : xp);
+    *xp_out = xp;
+    *xb_out = xp + xp - xo;
+    *x_out = w1 * ((T(1) + g) * xp - g * xo) + w0 * x0;
+}
+// One row's dual half: y+ from the row sum w = (A x_bar)_i, and the Halpern step.
+template <typename T>
+__device__ __forceinline__ void halpern_dual(T yo, T w, T rl, T ru, T y0, T sigma, T inv_sigma, T w1, T w0, T g,
+                                             T* yp_out, T* y_out) {
+    const T yh = yo + sigma * w;
+    T q = yh * inv_sigma;
+    q = q < rl ? rl : (q > ru ? ru : q);
+    const T yp = yh - sigma * q;
+    *yp_out = yp;
+    *y_out = w1 * ((T(1) + g) * yp - g * yo) + w0 * y0;
+}
 
 // At the last iteration of a chunk (write_cand) the epilogues also keep T(z) (xc, yc) and
 // the point it was taken from (xprev, yprev) for the check.
@@ -65,11 +92,10 @@ struct EpiHPrimal {
     }
     template <typename Acc>
     __device__ void operator()(int j, Acc v, const Pre& p) const {
-        const T g = p.g;
-        T xp = p.xo - p.tau * (p.c + static_cast<T>(v));
-        xp = xp < p.cl ? p.cl : (xp > p.cu ? p.cu : xp);
-        xb[j] = xp + xp - p.xo;
-        x[j] = p.w1 * ((T(1) + g) * xp - g * p.xo) + p.w0 * p.x0;
+        T xp, xbn, xn;
+        halpern_primal(p.xo, static_cast<T>(v), p.c, p.cl, p.cu, p.x0, p.tau, p.w1, p.w0, p.g, &xp, &xbn, &xn);
+        xb[j] = xbn;
+        x[j] = xn;
         if (write_cand) { xc[j] = xp; xprev[j] = p.xo; }
     }
     template <typename Acc>
@@ -100,12 +126,9 @@ struct EpiHDual {
     }
     template <typename Acc>
     __device__ void operator()(int i, Acc w, const Pre& p) const {
-        const T g = p.g;
-        const T yh = p.yo + p.sigma * static_cast<T>(w);
-        T q = yh * p.inv_sigma;
-        q = q < p.rl ? p.rl : (q > p.ru ? p.ru : q);
-        const T yp = yh - p.sigma * q;
-        y[i] = p.w1 * ((T(1) + g) * yp - g * p.yo) + p.w0 * p.y0;
+        T yp, yn;
+        halpern_dual(p.yo, static_cast<T>(w), p.rl, p.ru, p.y0, p.sigma, p.inv_sigma, p.w1, p.w0, p.g, &yp, &yn);
+        y[i] = yn;
         if (write_cand) { yc[i] = yp; yprev[i] = p.yo; }
     }
     template <typename Acc>
@@ -122,7 +145,7 @@ __device__ __forceinline__ void halpern_weights(const HState* st, int len, doubl
     }
 }
 
-__global__ void k_halpern_weights(const HState* st, int len, double* hw) {
+static __global__ void k_halpern_weights(const HState* st, int len, double* hw) {
     halpern_weights(st, len, hw, threadIdx.x, blockDim.x);
 }
 

@@ -76,3 +76,31 @@ def test_limit_in_the_middle_of_a_chunk_and_a_resident_rerun(cuda):
     assert a["iterations"] == b["iterations"] == 150 and a["status_name"] == "ITERATION_LIMIT"
     for k in ("x", "y", "row_value", "d"):
         np.testing.assert_array_equal(a[k], b[k])
+
+
+BATCHES = {"tiny": [(2, 2, 1), (60, 150, 4), (255, 256, 3)],
+           "spread": [(60, 150, 4), (301, 807, 3), (100, 400, 40), (1000, 1001, (1, 30)), (2000, 5000, 8), (4000, 9001, 6)],
+           "odd": ["one_row", "few_rows", "dense_row", "empty", (61, 149, 3)],
+           "one": [(500, 1200, 6)]}
+
+
+@pytest.mark.parametrize("limit", [1, 64])
+@pytest.mark.parametrize("prec", [V.PREC_FP64, V.PREC_MIXED])
+@pytest.mark.parametrize("kind", sorted(BATCHES))
+def test_batched_clusters_give_the_packed_iterations_bits(cuda, kind, prec, limit):
+    """Instances on clusters (alone or beside instances that are too large for one) against the
+    packed two-launch iteration (a fixed launch shape keeps the batch off the clusters)."""
+    lps = [lp_of(k) for k in BATCHES[kind]]
+    kw = dict(precision=prec, iteration_limit=limit, tolerance=1e-30, autotune=0)
+    for a, b in zip(V.solve_batch(lps, **kw), V.solve_batch(lps, spmv_shape_a=1, **kw)):
+        assert a["iterations"] == b["iterations"] == limit
+        for k in ("x", "y", "row_value", "d"):
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("prec", [V.PREC_FP64, V.PREC_MIXED])
+def test_batched_clusters_beside_larger_instances_reach_the_optima(cuda, prec):
+    lps = [lp_of(k) for k in BATCHES["spread"] if k != (100, 400, 40)]
+    for lp, r in zip(lps, V.solve_batch(lps, precision=prec, iteration_limit=40000)):
+        assert r["status_name"] == "OPTIMAL" and relative_kkt(lp, r["x"], r["y"])["rel_kkt"] <= 1.05e-6
+        assert r["fp32_iterations"] + r["fp64_iterations"] == r["iterations"]

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cluster.cuh"
 #include "halpern_state.cuh"
 #include "solver.cuh"
 
@@ -60,6 +61,8 @@ struct BatchCounters {
     int active;
     int left;
     long long chunks;
+    long long most;    // most iterations an instance has run
+    int wait_error;    // a cluster's exchange did not complete
 };
 
 // Chunks one launch of a pass graph may run before the host looks at the counters again.
@@ -241,48 +244,56 @@ struct BlockList {
 __device__ __forceinline__ bool lo_fin(double l) { return l > -1e20; }
 __device__ __forceinline__ bool up_fin(double u) { return u < 1e20; }
 
-// One CTA per instance: the same KKT terms as the single-LP row / column passes.
+// One row's and one column's terms of an instance's check, as the single-LP passes have them.
+// 0 rp_o^2, 1 rp_s^2, 2 dobj rows, 3 dy^2, 4 rd_o^2, 5 rd_s^2, 6 pobj, 7 dobj cols, 8 dx^2, 9 nan (maximum)
+__device__ __forceinline__ void bkkt_row_terms(double a, double ys, double rl_s, double ru_s, double rl_o, double ru_o,
+                                               double rs, double y_last, double (&v)[kBQ]) {
+    if (!isfinite(a) || !isfinite(ys)) v[9] = 1.0;
+    const double ps = a - fmin(fmax(a, rl_s), ru_s);
+    const double ao = a / rs;
+    const double po = ao - fmin(fmax(ao, rl_o), ru_o);
+    const double yo = -ys * rs;
+    double dt = 0.0;
+    if (yo > 0.0 && lo_fin(rl_o)) dt = yo * rl_o;
+    else if (yo < 0.0 && up_fin(ru_o)) dt = yo * ru_o;
+    const double dy = ys - y_last;
+    v[0] += po * po; v[1] += ps * ps; v[2] += dt; v[3] += dy * dy;
+}
+__device__ __forceinline__ void bkkt_col_terms(double at, double xs, double c_s, double cl_o, double cu_o, double cs,
+                                               double x_last, double (&v)[kBQ]) {
+    if (!isfinite(at) || !isfinite(xs)) v[9] = 1.0;
+    const bool lf = lo_fin(cl_o), uf = up_fin(cu_o);
+    const double r_s = c_s + at, r_o = r_s / cs;
+    auto lam_of = [&](double r) { return (lf && uf) ? r : lf ? fmax(r, 0.0) : uf ? fmin(r, 0.0) : 0.0; };
+    const double lo = lam_of(r_o), ls = lam_of(r_s);
+    double dt = 0.0;
+    if (lo > 0.0) dt = lo * cl_o;
+    else if (lo < 0.0) dt = lo * cu_o;
+    const double dx = xs - x_last;
+    v[4] += (r_o - lo) * (r_o - lo); v[5] += (r_s - ls) * (r_s - ls);
+    v[6] += c_s * xs; v[7] += dt; v[8] += dx * dx;
+}
+// The checks' vectors of the packed LPs.
+struct BKktVectors {
+    const double* rl_s; const double* ru_s; const double* rl_o; const double* ru_o; const double* rs;
+    const double* c_s; const double* cl_o; const double* cu_o; const double* cs;
+};
+
+// One CTA per instance: its check sums.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_bkkt(const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, const double* __restrict__ ax,
-       const double* __restrict__ aty, const T* __restrict__ xc, const T* __restrict__ yc,
-       const double* __restrict__ rl_s, const double* __restrict__ ru_s, const double* __restrict__ rl_o,
-       const double* __restrict__ ru_o, const double* __restrict__ rs, const double* __restrict__ c_s,
-       const double* __restrict__ cl_o, const double* __restrict__ cu_o, const double* __restrict__ cs,
+       const double* __restrict__ aty, const T* __restrict__ xc, const T* __restrict__ yc, BKktVectors V,
        const double* __restrict__ x_last, const double* __restrict__ y_last, double* __restrict__ part,
        BatchArrays S) {
     const int inst = blockIdx.x;
     if (S.done[inst]) return;
     __shared__ double red[kBQ * 32];
     double v[kBQ] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    // 0 rp_o^2, 1 rp_s^2, 2 dobj rows, 3 dy^2, 4 rd_o^2, 5 rd_s^2, 6 pobj, 7 dobj cols, 8 dx^2, 9 nan
-    for (int64_t i = roff[inst] + threadIdx.x; i < roff[inst + 1]; i += blockDim.x) {
-        const double a = ax[i], ys = static_cast<double>(yc[i]);
-        if (!isfinite(a) || !isfinite(ys)) v[9] = 1.0;
-        const double ps = a - fmin(fmax(a, rl_s[i]), ru_s[i]);
-        const double ao = a / rs[i];
-        const double po = ao - fmin(fmax(ao, rl_o[i]), ru_o[i]);
-        const double yo = -ys * rs[i];
-        double dt = 0.0;
-        if (yo > 0.0 && lo_fin(rl_o[i])) dt = yo * rl_o[i];
-        else if (yo < 0.0 && up_fin(ru_o[i])) dt = yo * ru_o[i];
-        const double dy = ys - y_last[i];
-        v[0] += po * po; v[1] += ps * ps; v[2] += dt; v[3] += dy * dy;
-    }
-    for (int64_t j = coff[inst] + threadIdx.x; j < coff[inst + 1]; j += blockDim.x) {
-        const double at = aty[j], xs = static_cast<double>(xc[j]);
-        if (!isfinite(at) || !isfinite(xs)) v[9] = 1.0;
-        const bool lf = lo_fin(cl_o[j]), uf = up_fin(cu_o[j]);
-        const double r_s = c_s[j] + at, r_o = r_s / cs[j];
-        auto lam_of = [&](double r) { return (lf && uf) ? r : lf ? fmax(r, 0.0) : uf ? fmin(r, 0.0) : 0.0; };
-        const double lo = lam_of(r_o), ls = lam_of(r_s);
-        double dt = 0.0;
-        if (lo > 0.0) dt = lo * cl_o[j];
-        else if (lo < 0.0) dt = lo * cu_o[j];
-        const double dx = xs - x_last[j];
-        v[4] += (r_o - lo) * (r_o - lo); v[5] += (r_s - ls) * (r_s - ls);
-        v[6] += c_s[j] * xs; v[7] += dt; v[8] += dx * dx;
-    }
+    for (int64_t i = roff[inst] + threadIdx.x; i < roff[inst + 1]; i += blockDim.x)
+        bkkt_row_terms(ax[i], static_cast<double>(yc[i]), V.rl_s[i], V.ru_s[i], V.rl_o[i], V.ru_o[i], V.rs[i], y_last[i], v);
+    for (int64_t j = coff[inst] + threadIdx.x; j < coff[inst + 1]; j += blockDim.x)
+        bkkt_col_terms(aty[j], static_cast<double>(xc[j]), V.c_s[j], V.cl_o[j], V.cu_o[j], V.cs[j], x_last[j], v);
     double f[1] = {v[9]};
     block_reduce<OpSum, double, kBQ - 1>(*reinterpret_cast<double(*)[kBQ - 1]>(v), red);
     block_reduce<OpMax, double, 1>(f, red);
@@ -303,71 +314,219 @@ struct BControl {
     double gamma32;
 };
 
-// One thread per instance: the single-LP control rules (halpern_mode.cu) per instance.
-__global__ void k_bcontrol(const double* __restrict__ part, BControl cp, BatchArrays S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cp.count || S.done[i]) return;
-    const double* s = part + i * kBQ;
-    S.total[i] += cp.len;
-    S.restart_flag[i] = 0;
+// One instance's state, and its place in the arrays.
+struct BInstance {
+    double omega, eta, tau, sigma, inv_sigma, gamma, kkt_start, kkt_prev;
+    double rel_p, rel_d, rel_gap, rel_kkt, pobj, dobj, bnorm, cnorm, offset_min;
+    double* hist;
+    long long k_base, total;
+    int done, status, restart_count, restart_flag, hist_n;
+};
+__device__ __forceinline__ BInstance binst_load(const BatchArrays& S, int i) {
+    BInstance b;
+    b.omega = S.omega[i]; b.eta = S.eta[i]; b.tau = S.tau[i]; b.sigma = S.sigma[i]; b.inv_sigma = S.inv_sigma[i];
+    b.gamma = S.gamma[i]; b.kkt_start = S.kkt_start[i]; b.kkt_prev = S.kkt_prev[i];
+    b.rel_p = S.rel_p[i]; b.rel_d = S.rel_d[i]; b.rel_gap = S.rel_gap[i]; b.rel_kkt = S.rel_kkt[i];
+    b.pobj = S.pobj[i]; b.dobj = S.dobj[i];
+    b.bnorm = S.bnorm[i]; b.cnorm = S.cnorm[i]; b.offset_min = S.offset_min[i];
+    b.hist = S.hist + static_cast<size_t>(i) * kBHist;
+    b.k_base = S.k_base[i]; b.total = S.total[i];
+    b.done = S.done[i]; b.status = S.status[i]; b.restart_count = S.restart_count[i];
+    b.restart_flag = S.restart_flag[i]; b.hist_n = S.hist_n[i];
+    return b;
+}
+__device__ __forceinline__ void binst_store(const BatchArrays& S, int i, const BInstance& b) {
+    S.omega[i] = b.omega; S.tau[i] = b.tau; S.sigma[i] = b.sigma; S.inv_sigma[i] = b.inv_sigma;
+    S.gamma[i] = b.gamma; S.kkt_start[i] = b.kkt_start; S.kkt_prev[i] = b.kkt_prev;
+    S.rel_p[i] = b.rel_p; S.rel_d[i] = b.rel_d; S.rel_gap[i] = b.rel_gap; S.rel_kkt[i] = b.rel_kkt;
+    S.pobj[i] = b.pobj; S.dobj[i] = b.dobj;
+    S.k_base[i] = b.k_base; S.total[i] = b.total;
+    S.done[i] = b.done; S.status[i] = b.status; S.restart_count[i] = b.restart_count;
+    S.restart_flag[i] = b.restart_flag; S.hist_n[i] = b.hist_n;
+}
+
+// The single-LP control rules (halpern_mode.cu) for one instance; `s`: its check sums.
+__device__ __forceinline__ void binst_decide(BInstance& b, const double* s, const BControl& cp) {
+    b.total += cp.len;
+    b.restart_flag = 0;
     if (s[9] > 0.0 || isnan(s[0]) || isnan(s[4])) {
-        S.done[i] = 1;
-        S.status[i] = 9;
+        b.done = 1;
+        b.status = 9;
         return;
     }
-    const double pobj = s[6] + S.offset_min[i];
-    const double dobj = s[2] + s[7] + S.offset_min[i];
-    const double rel_p = sqrt(s[0]) / (1.0 + S.bnorm[i]);
-    const double rel_d = sqrt(s[4]) / (1.0 + S.cnorm[i]);
+    const double pobj = s[6] + b.offset_min;
+    const double dobj = s[2] + s[7] + b.offset_min;
+    const double rel_p = sqrt(s[0]) / (1.0 + b.bnorm);
+    const double rel_d = sqrt(s[4]) / (1.0 + b.cnorm);
     const double gap = fabs(pobj - dobj) / (1.0 + fabs(pobj) + fabs(dobj));
     const double rel = fmax(rel_p, fmax(rel_d, gap));
-    S.rel_p[i] = rel_p; S.rel_d[i] = rel_d; S.rel_gap[i] = gap; S.rel_kkt[i] = rel;
-    S.pobj[i] = pobj; S.dobj[i] = dobj;
+    b.rel_p = rel_p; b.rel_d = rel_d; b.rel_gap = gap; b.rel_kkt = rel;
+    b.pobj = pobj; b.dobj = dobj;
     if (rel <= cp.tol) {
-        S.done[i] = 1;
-        S.status[i] = 1;
+        b.done = 1;
+        b.status = 1;
         return;
     }
     if (cp.pass32) {
-        const int hn = S.hist_n[i];
-        double* hist = S.hist + static_cast<size_t>(i) * kBHist;
+        const int hn = b.hist_n;
         const int w = cp.stall_checks;
-        const bool stalled = w > 0 && hn >= w && rel > 0.98 * hist[(hn - w) % kBHist];
-        hist[hn % kBHist] = rel;
-        S.hist_n[i] = hn + 1;
-        if (rel <= cp.early_tol) S.gamma[i] = cp.gamma32;
+        const bool stalled = w > 0 && hn >= w && rel > 0.98 * b.hist[(hn - w) % kBHist];
+        b.hist[hn % kBHist] = rel;
+        b.hist_n = hn + 1;
+        if (rel <= cp.early_tol) b.gamma = cp.gamma32;
         if (rel <= cp.switch_tol || stalled) {   // leaves the FP32 pass; the FP64 pass takes it over
-            S.done[i] = 1;
-            S.status[i] = kBHandover;
+            b.done = 1;
+            b.status = kBHandover;
             return;
         }
     }
-    const double omega = S.omega[i];
+    const double omega = b.omega;
     const double wk = sqrt(omega * s[1] + s[5] / omega + gap * gap);
-    if (S.kkt_start[i] < 0.0) { S.kkt_start[i] = wk; S.kkt_prev[i] = wk; }
-    const long long k_in = S.k_base[i] + cp.len;
-    const bool restart = (wk <= cp.beta_sufficient * S.kkt_start[i]) ||
-                         (wk <= cp.beta_necessary * S.kkt_start[i] && wk > S.kkt_prev[i]) ||
-                         (static_cast<double>(k_in) >= cp.beta_artificial * static_cast<double>(S.total[i]));
-    S.kkt_prev[i] = wk;
+    if (b.kkt_start < 0.0) { b.kkt_start = wk; b.kkt_prev = wk; }
+    const long long k_in = b.k_base + cp.len;
+    const bool restart = (wk <= cp.beta_sufficient * b.kkt_start) ||
+                         (wk <= cp.beta_necessary * b.kkt_start && wk > b.kkt_prev) ||
+                         (static_cast<double>(k_in) >= cp.beta_artificial * static_cast<double>(b.total));
+    b.kkt_prev = wk;
     if (restart) {
         const double dx = sqrt(s[8]), dy = sqrt(s[3]);
         if (dx > 1e-10 && dy > 1e-10) {
             const double th = cp.pw_smoothing;
-            S.omega[i] = exp(th * log(dy / dx) + (1.0 - th) * log(omega));
-            S.tau[i] = S.eta[i] / S.omega[i];
-            S.sigma[i] = S.eta[i] * S.omega[i];
-            S.inv_sigma[i] = 1.0 / S.sigma[i];
+            b.omega = exp(th * log(dy / dx) + (1.0 - th) * log(omega));
+            b.tau = b.eta / b.omega;
+            b.sigma = b.eta * b.omega;
+            b.inv_sigma = 1.0 / b.sigma;
         }
-        S.k_base[i] = 0;
-        S.kkt_start[i] = wk;
-        S.kkt_prev[i] = wk;
-        S.restart_count[i] += 1;
-        S.restart_flag[i] = 1;
+        b.k_base = 0;
+        b.kkt_start = wk;
+        b.kkt_prev = wk;
+        b.restart_count += 1;
+        b.restart_flag = 1;
     } else {
-        S.k_base[i] = k_in;
+        b.k_base = k_in;
     }
-    instance_weights(S, i);
+}
+
+// One thread per instance.
+__global__ void k_bcontrol(const double* __restrict__ part, BControl cp, BatchArrays S) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cp.count || S.done[i]) return;
+    BInstance b = binst_load(S, i);
+    binst_decide(b, part + i * kBQ, cp);
+    binst_store(S, i, b);
+    if (!b.done) instance_weights(S, i);
+}
+
+// ----- small instances on clusters (cluster.cuh) -------------------------------------------
+// The packed matrices as the clusters read them.
+template <typename T>
+struct BMats {
+    const int64_t* a_ptr; const int32_t* a_idx; const T* a_val;
+    const int64_t* at_ptr; const int32_t* at_idx; const T* at_val;
+    int group_a, group_at;
+    int64_t long_a, long_at;
+};
+// Instance `inst` of them, by thread 0.
+template <typename T>
+__device__ __forceinline__ void bmats_of(const BMats<T>& M, const int64_t* roff, const int64_t* coff, int inst, ClMats<T>& out) {
+    const int r0 = static_cast<int>(roff[inst]), c0 = static_cast<int>(coff[inst]);
+    out.a = ClMat<T>{static_cast<int>(roff[inst + 1]) - r0, M.a_ptr + r0, M.a_idx, M.a_val, c0, M.group_a, M.long_a};
+    out.at = ClMat<T>{static_cast<int>(coff[inst + 1]) - c0, M.at_ptr + c0, M.at_idx, M.at_val, r0, M.group_at, M.long_at};
+}
+
+constexpr uint32_t kBMaxes = 1u << 9;
+template <typename T>
+__device__ __noinline__ void cl_bkkt_partials(const ClVectors<T>& P, const BKktVectors& V, int i, double ax, int j, double aty,
+                                              double* red, double* part) {
+    double v[kBQ] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (i >= 0)
+        bkkt_row_terms(ax, static_cast<double>(P.yc[i]), V.rl_s[i], V.ru_s[i], V.rl_o[i], V.ru_o[i], V.rs[i], P.y_last[i], v);
+    if (j >= 0)
+        bkkt_col_terms(aty, static_cast<double>(P.xc[j]), V.c_s[j], V.cl_o[j], V.cu_o[j], V.cs[j], P.x_last[j], v);
+    cl_reduce<kBQ, kBMaxes>(v, red, part);
+}
+__device__ __noinline__ void cl_bkkt_decide(const double* part, int ctas, double* red, const BControl& cp, BInstance& b) {
+    cl_combine<kBQ, kBMaxes>(part, ctas, red);
+    if (threadIdx.x == 0) binst_decide(b, red, cp);
+}
+
+template <typename T>
+struct BatchClusterControl {
+    const ClVectors<T>& P;
+    const BKktVectors& V;
+    const BatchArrays& S;   // `done` here is the clusters' own array
+    int inst;
+    BInstance& b;           // rank 0's copy, in shared memory
+    BControl& cp;
+    double* red;
+    double* part;
+    __device__ void control(ClControl& c) const {
+        c.tau = b.tau; c.sigma = b.sigma; c.inv_sigma = b.inv_sigma; c.gamma = b.gamma;
+        c.k_base = b.k_base; c.stop = b.done; c.restart = b.restart_flag;
+    }
+    __device__ void start(ClControl& c) const {
+        if (threadIdx.x != 0) return;
+        b = binst_load(S, inst);
+        control(c);
+    }
+    __device__ void partials(int i, double ax, int j, double aty, uint32_t rank) const {
+        cl_bkkt_partials<T>(P, V, i, ax, j, aty, red, part + rank * kBQ);
+    }
+    __device__ void decide(int ctas, int len, double, double, ClControl& c) const {
+        if (threadIdx.x == 0) cp.len = len;
+        cl_bkkt_decide(part, ctas, red, cp, b);
+        if (threadIdx.x == 0) control(c);
+    }
+    __device__ void finish() const {
+        if (threadIdx.x != 0) return;
+        b.restart_flag = 0;   // done here: the general path's restart pass leaves the instance alone
+        binst_store(S, inst, b);
+    }
+};
+
+// Cluster q runs instance insts[q]: chunks until it is done or the budget ends.  128 registers a
+// thread, so that two CTAs of 256 threads share an SM.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ BKktVectors V, const __grid_constant__ BMats<T> M,
+                const int* __restrict__ insts, const int64_t* __restrict__ roff, const int64_t* __restrict__ coff,
+                const __grid_constant__ BatchArrays S, const __grid_constant__ BControl cp0, double* part, ClControl* shared,
+                int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+    __shared__ double red[kBQ * kClWarps];
+    __shared__ BInstance b;
+    __shared__ BControl cp;
+    __shared__ ClMats<T> mats;
+    const int cluster = blockIdx.x / cl_size(), inst = insts[cluster];
+    if (S.done[inst]) return;   // uniform over the cluster
+    if (threadIdx.x == 0) {
+        cp = cp0;
+        bmats_of(M, roff, coff, inst, mats);
+    }
+    __syncthreads();
+    BatchClusterControl<T> pol{P, V, S, inst, b, cp, red, part + static_cast<size_t>(cluster) * kClMaxCtas * kBQ};
+    cl_run<T, NT>(P, mats, static_cast<int>(roff[inst]), static_cast<int>(coff[inst]), pol, shared + cluster, K, budget, max_chunks,
+                  smem_bytes);
+}
+
+// nofit[insts[q]] = 1 where the slices of cluster q do not fit its CTAs.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+k_cluster_fit(const __grid_constant__ BMats<T> M, const int* __restrict__ insts, const int64_t* __restrict__ roff,
+              const int64_t* __restrict__ coff, int* __restrict__ nofit, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ ClMats<T> mats;
+    const int inst = insts[blockIdx.x / cl_size()];
+    if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
+    __syncthreads();
+    ClCore<T, T> core;
+    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) nofit[inst] = 1;
+}
+
+// done = 1 for the instances that a path does not run: `on` (null: none) marks those on clusters,
+// `want` is the path's mark; an instance that has finished (status set) is run by neither.
+__global__ void k_bassign(int count, const int* __restrict__ on, int want, const int* __restrict__ status, int* __restrict__ done) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) done[i] = (on && on[i] != 0) == (want != 0) && status[i] == 0 ? 0 : 1;
 }
 
 // Counts the unfinished instances.  Inside the WHILE body of a pass graph (`loop` = 1) it also
@@ -381,13 +540,33 @@ __global__ void __launch_bounds__(1024) k_bcount(int count, const int* __restric
     block_reduce<OpSum, double, 1>(v, red);
     if (threadIdx.x == 0) {
         const int active = static_cast<int>(v[0]);
-        out->active = active;
         if (loop) {
             const int left = out->left - 1;
             out->left = left;
             out->chunks += 1;
             cudaGraphSetConditional(again, active > 0 && left > 0 ? 1u : 0u);
         }
+    }
+}
+
+// After a launch: the unfinished instances of both paths, the most iterations an instance has run,
+// and whether a cluster's exchange did not complete.
+__global__ void __launch_bounds__(1024) k_btotals(int count, const int* __restrict__ done, const int* __restrict__ done_cl,
+                                                  const long long* __restrict__ total, const ClControl* __restrict__ shared,
+                                                  int clusters, BatchCounters* out) {
+    __shared__ double red[2 * 32];
+    double v[1] = {0.0}, f[2] = {0.0, 0.0};
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        v[0] += (done[i] ? 0.0 : 1.0) + (done_cl[i] ? 0.0 : 1.0);
+        f[0] = fmax(f[0], static_cast<double>(total[i]));
+    }
+    for (int q = threadIdx.x; q < clusters; q += blockDim.x) f[1] = fmax(f[1], shared[q].wait_error ? 1.0 : 0.0);
+    block_reduce<OpSum, double, 1>(v, red);
+    block_reduce<OpMax, double, 2>(f, red);
+    if (threadIdx.x == 0) {
+        out->active = static_cast<int>(v[0]);
+        out->most = static_cast<long long>(f[0]);
+        out->wait_error = f[1] > 0.0 ? 1 : 0;
     }
 }
 
@@ -431,7 +610,6 @@ __global__ void k_bhandover_state(int count, double gamma64, BatchArrays S) {
     if (i >= count) return;
     S.total32[i] = S.total[i];
     if (S.status[i] != kBHandover) return;
-    S.done[i] = 0;
     S.status[i] = 0;
     S.k_base[i] = 0;
     S.kkt_start[i] = -1.0;
@@ -584,6 +762,127 @@ template <typename T>
 vajra_status up(DeviceBuffer<T>& d, const std::vector<T>& h, cudaStream_t st) {
     VJ_TRY(d.alloc(h.size()));
     if (!h.empty()) VJ_CUDA(cudaMemcpyAsync(d.get(), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+    return VAJRA_OK;
+}
+
+// The instances that run on clusters, by cluster size and threads.
+struct ClusterClass {
+    int ctas = 0, threads = 0, first = 0, clusters = 0;   // its part of the instance list
+    size_t smem = 0;
+};
+struct ClusterBatch {
+    std::vector<int> least;              // per instance: CTAs of its smallest cluster, 0: it has none
+    std::vector<int> insts;              // the instances of the present plan, by class, largest first
+    std::vector<ClusterClass> classes;   // widest clusters first
+    DeviceBuffer<int> d_insts, d_on;     // the same list; per instance: runs on a cluster
+};
+
+template <typename T>
+auto batch_kernel(int threads) -> decltype(&k_cluster_batch<T, 256>) {
+    return threads == 256 ? &k_cluster_batch<T, 256> : &k_cluster_batch<T, 512>;
+}
+template <typename T>
+auto fit_kernel(int threads) -> decltype(&k_cluster_fit<T, 256>) {
+    return threads == 256 ? &k_cluster_fit<T, 256> : &k_cluster_fit<T, 512>;
+}
+
+// The smallest cluster that holds an instance takes the least of the GPU, since an exchange costs
+// no less with more CTAs: 256 threads on one CTA, else CTAs of 512 with at most 4,096 entries of each
+// matrix.
+template <typename T>
+int least_cluster(const vajra_lp& L, int group_a, int group_at) {
+    auto fits = [&](int c, int t) { return cl_fits(sizeof(T), L.num_rows, L.num_cols, L.nnz, group_a, group_at, c, t); };
+    for (int c = 1; c <= kClMaxCtas; c *= 2)
+        if (fits(c, 512) && (L.nnz <= 4096 * static_cast<int64_t>(c) || c == kClMaxCtas)) return c;
+    return 0;
+}
+
+// Entries of unfinished instances too large for a cluster up to which the others go to clusters.
+// Above it the packed iteration is bound by bandwidth (18 ps an entry in FP64, so 70 us here) and
+// takes the small instances along at no worse a rate than clusters beside it do (256 LPs of 100 to
+// 20,000 rows: 477 ms packed, 526 ms with the small ones on clusters).  Below it an iteration costs
+// its launches (9 to 20 us) and the small instances finish sooner by themselves (96 LPs of 100 to
+// 2,000 rows: 43.8 -> 30.6 ms).
+constexpr int64_t kClBatchEntries = int64_t(4) << 20;
+
+// Plans the unfinished instances (open[i] != 0) of a launch.  A plan that leaves half of the SMs
+// idle gets clusters of twice the size, as far as their CTAs keep 512 entries.
+template <typename T>
+vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, const BMats<T>& M, const int64_t* roff,
+                           const int64_t* coff, ClusterBatch& out, cudaStream_t st) {
+    DeviceBuffer<int> nofit;
+    VJ_TRY(nofit.alloc(count));
+    VJ_TRY(out.d_insts.alloc(count));
+    VJ_TRY(out.d_on.alloc(count));
+    std::vector<int> ctas(count), threads(count), on(count), h(count);
+    auto fits = [&](int i, int c, int t) {
+        return cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, M.group_a, M.group_at, c, t);
+    };
+    for (bool again = true; again;) {
+        again = false;
+        int64_t outside = 0, sms_used = 0;
+        for (int i = 0; i < count; ++i) if (open[i] && !out.least[i]) outside += lps[i].nnz;
+        for (int i = 0; i < count; ++i) {
+            ctas[i] = open[i] && outside <= kClBatchEntries ? out.least[i] : 0;
+            sms_used += ctas[i];
+        }
+        while (sms_used > 0 && 2 * sms_used <= sm_count()) {
+            int64_t used = 0;
+            for (int i = 0; i < count; ++i) {
+                if (ctas[i] > 0 && ctas[i] < kClMaxCtas && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
+                    ctas[i] *= 2;
+                used += ctas[i];
+            }
+            if (used == sms_used) break;
+            sms_used = used;
+        }
+        for (int i = 0; i < count; ++i)
+            threads[i] = ctas[i] && fits(i, ctas[i], 256) && lps[i].nnz <= 2048 * static_cast<int64_t>(ctas[i]) ? 256 : 512;
+        out.classes.clear();
+        out.insts.clear();
+        for (int c = kClMaxCtas; c >= 1; c /= 2)
+            for (int t : {512, 256}) {
+                ClusterClass k;
+                k.ctas = c;
+                k.threads = t;
+                k.first = static_cast<int>(out.insts.size());
+                size_t most = 0;
+                for (int i = 0; i < count; ++i)
+                    if (ctas[i] == c && threads[i] == t) {
+                        out.insts.push_back(i);
+                        most = std::max(most, cl_smem_bytes(sizeof(T), sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, c, t));
+                    }
+                k.clusters = static_cast<int>(out.insts.size()) - k.first;
+                if (!k.clusters) continue;
+                std::stable_sort(out.insts.begin() + k.first, out.insts.end(), [&](int x, int y) { return lps[x].nnz > lps[y].nnz; });
+                // two CTAs of 256 threads fit an SM when each takes half of its shared memory
+                k.smem = t == 256 && most <= kClSmemCap / 2 - 4096 ? kClSmemCap / 2 - 4096 : kClSmemCap;
+                out.classes.push_back(k);
+            }
+        if (out.insts.empty()) break;
+        // Instances whose uneven rows do not fit after all go to the packed iteration.
+        VJ_CUDA(cudaMemcpyAsync(out.d_insts.get(), out.insts.data(), sizeof(int) * out.insts.size(), cudaMemcpyHostToDevice, st));
+        VJ_CUDA(cudaMemsetAsync(nofit.get(), 0, sizeof(int) * count, st));
+        for (const ClusterClass& k : out.classes) {
+            cudaError_t e = prepare_clusters(batch_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
+            if (e == cudaSuccess) e = prepare_clusters(fit_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
+            if (e != cudaSuccess) {   // no such cluster on this device
+                cudaGetLastError();
+                for (int q = k.first; q < k.first + k.clusters; ++q) out.least[out.insts[q]] = 0;
+                again = true;
+                continue;
+            }
+            VJ_CUDA(launch_clusters(fit_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, st, M, out.d_insts.get() + k.first,
+                                    roff, coff, nofit.get(), static_cast<uint32_t>(k.smem)));
+        }
+        VJ_CUDA(cudaMemcpyAsync(h.data(), nofit.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
+        VJ_CUDA(cudaStreamSynchronize(st));
+        for (int q : out.insts)
+            if (h[q]) { out.least[q] = 0; again = true; }
+    }
+    for (int q : out.insts) on[q] = 1;
+    VJ_CUDA(cudaMemcpyAsync(out.d_on.get(), on.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
+    VJ_CUDA(cudaStreamSynchronize(st));   // host vectors above
     return VAJRA_OK;
 }
 
@@ -775,9 +1074,36 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         VJ_LAUNCH_CHECK();
     }
 
+    // ---- small instances on clusters ---------------------------------------------------------
+    const BKktVectors kv{p.row_lower.get(), p.row_upper.get(), lp.row_lower.get(), lp.row_upper.get(), p.row_scale.get(),
+                         p.c.get(), lp.col_lower.get(), lp.col_upper.get(), p.col_scale.get()};
+    auto mats = [&](auto tag) {
+        using T = decltype(tag);
+        const T* csr; const T* csc;
+        if constexpr (sizeof(T) == 4) { csr = p.csr_val32.get(); csc = p.csc_val32.get(); }
+        else { csr = p.csr_val.get(); csc = p.csc_val.get(); }
+        return BMats<T>{p.csr_ptr.get(), p.csr_idx.get(), csr, lp.col_ptr.get(), lp.row_idx.get(), csc,
+                        p.a.group, p.at.group, p.a.long_len, p.at.long_len};
+    };
+    ClusterBatch clus32, clus64;
+    bool all_fit = true;
+    const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0;   // as for a single LP
+    for (int i = 0; i < count; ++i) {
+        clus32.least.push_back(may_cluster && mixed ? least_cluster<float>(lps[i], p.a.group, p.at.group) : 0);
+        clus64.least.push_back(may_cluster ? least_cluster<double>(lps[i], p.a.group, p.at.group) : 0);
+        all_fit = all_fit && clus64.least[i] > 0;   // FP32 vectors are smaller
+    }
+    DeviceBuffer<double> cl_part;
+    DeviceBuffer<ClControl> cl_shared;
+    DeviceBuffer<int> done_cl;
+    VJ_TRY(cl_part.alloc(static_cast<size_t>(count) * kClMaxCtas * kBQ));
+    VJ_TRY(cl_shared.alloc(static_cast<size_t>(count)));
+    VJ_TRY(done_cl.alloc(count));
+
+
     // autotune the packed SpMVs (store epilogue, no skipping)
     CsrView a = p.a, at = p.at;
-    if (o.autotune) {
+    if (o.autotune && !all_fit) {
         cudaEvent_t e0, e1;
         VJ_CUDA(cudaEventCreate(&e0));
         VJ_CUDA(cudaEventCreate(&e1));
@@ -881,11 +1207,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         }
         launch_spmv_t<double, T, double>(a_it, p.csr_val.get(), xcv, EpiBStore{ax.get(), row_inst.get(), S.done}, st);
         launch_spmv_t<double, T, double>(at_it, p.csc_val.get(), ycv, EpiBStore{aty.get(), col_inst.get(), S.done}, st);
-        k_bkkt<T><<<count, kThreads, 0, st>>>(d_roff.get(), d_coff.get(), ax.get(), aty.get(), xcv, ycv,
-                                              p.row_lower.get(), p.row_upper.get(), lp.row_lower.get(),
-                                              lp.row_upper.get(), p.row_scale.get(), p.c.get(), lp.col_lower.get(),
-                                              lp.col_upper.get(), p.col_scale.get(), x_last.get(), y_last.get(),
-                                              part.get(), S);
+        k_bkkt<T><<<count, kThreads, 0, st>>>(d_roff.get(), d_coff.get(), ax.get(), aty.get(), xcv, ycv, kv, x_last.get(),
+                                              y_last.get(), part.get(), S);
         BControl c2 = bc;
         c2.len = len;
         c2.pass32 = sizeof(T) == 4 ? 1 : 0;
@@ -896,21 +1219,109 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         note_launch(4);
     };
 
+    // One launch of the clusters of a pass: every class on a stream of its own, joined into `st`.
+    struct Side {
+        std::vector<cudaStream_t> streams;
+        std::vector<cudaEvent_t> events;
+        cudaEvent_t ready = nullptr;
+        ~Side() {
+            for (auto& e : events) cudaEventDestroy(e);
+            for (auto& s : streams) cudaStreamDestroy(s);
+            if (ready) cudaEventDestroy(ready);
+        }
+    } side;
+    auto want_streams = [&](size_t k) -> vajra_status {
+        if (!side.ready) VJ_CUDA(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
+        while (side.streams.size() < k) {
+            cudaStream_t s = nullptr;
+            cudaEvent_t e = nullptr;
+            VJ_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            side.streams.push_back(s);
+            VJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            side.events.push_back(e);
+        }
+        return VAJRA_OK;
+    };
+    BatchArrays Scl = S;
+    Scl.done = done_cl.get();
+    auto fork_clusters = [&](auto tag, const ClusterBatch& cl, int64_t iters) -> vajra_status {
+        using T = decltype(tag);
+        if (cl.insts.empty()) return VAJRA_OK;
+        VJ_TRY(want_streams(cl.classes.size()));
+        const PassBuffers& b = sizeof(T) == 4 ? pb32 : pb64;
+        const ClVectors<T> P{static_cast<const T*>(b.c), static_cast<const T*>(b.cl), static_cast<const T*>(b.cu),
+                             static_cast<const T*>(b.rl), static_cast<const T*>(b.ru), static_cast<T*>(b.x), static_cast<T*>(b.x0),
+                             static_cast<T*>(b.xc), nullptr, static_cast<T*>(b.y), static_cast<T*>(b.y0), static_cast<T*>(b.yc),
+                             nullptr, x_last.get(), y_last.get(), p.csr_val.get(), p.csc_val.get()};
+        BControl c2 = bc;
+        c2.pass32 = sizeof(T) == 4 ? 1 : 0;
+        VJ_CUDA(cudaEventRecord(side.ready, st));
+        for (size_t q = 0; q < cl.classes.size(); ++q) {
+            const ClusterClass& k = cl.classes[q];
+            VJ_CUDA(cudaStreamWaitEvent(side.streams[q], side.ready, 0));
+            VJ_CUDA(launch_clusters(batch_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, side.streams[q], P, kv,
+                                    mats(tag), cl.d_insts.get() + k.first, d_roff.get(), d_coff.get(), Scl, c2,
+                                    cl_part.get() + static_cast<size_t>(k.first) * kClMaxCtas * kBQ, cl_shared.get() + k.first, K,
+                                    static_cast<long long>(iters), static_cast<int>((iters + K - 1) / K), static_cast<uint32_t>(k.smem)));
+            VJ_CUDA(cudaEventRecord(side.events[q], side.streams[q]));
+        }
+        return VAJRA_OK;
+    };
+    auto join_clusters = [&](const ClusterBatch& cl) -> vajra_status {
+        for (size_t q = 0; q < cl.classes.size(); ++q) VJ_CUDA(cudaStreamWaitEvent(st, side.events[q], 0));
+        return VAJRA_OK;
+    };
+
     const int64_t max_iter = o.iteration_limit;
     int64_t launched = 0;
     bool time_out = false;
-    // Runs one pass until no instance is left in it or a limit is reached.  Full chunks run in
-    // the pass graph: a WHILE node whose body is one chunk, repeated on the device while an
-    // instance is active, at most `left` times a launch.  A last partial chunk (iteration
-    // limit not a multiple of K) is launched directly.
+    const bool timed = o.time_limit < 1e9;
+    // Runs one pass until no instance is left in it or a limit is reached: the clusters on their
+    // streams, the other instances on `st`.  Those run full chunks in the pass graph: a WHILE node
+    // whose body is one chunk, repeated on the device while an instance is active, at most `left`
+    // times a launch.  A last partial chunk (iteration limit not a multiple of K) is launched
+    // directly.
     auto run_pass = [&](auto tag) -> vajra_status {
         using T = decltype(tag);
         const int k = sizeof(T) == 4 ? 0 : 1;
+        ClusterBatch& cl = k == 0 ? clus32 : clus64;
+        std::vector<int> open(count), status(count);
+        int64_t first = kFirstLaunchChunks;
         long long pass_chunks = 0;   // chunks this pass has run, and the host time they took
         double pass_seconds = 0.0;
         while (launched < max_iter) {
             const int64_t remaining = max_iter - launched;
+            // which instances are unfinished, and which of them go to clusters now
+            VJ_CUDA(cudaMemcpyAsync(status.data(), S.status, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
+            VJ_CUDA(cudaStreamSynchronize(st));
+            for (int i = 0; i < count; ++i) open[i] = status[i] == 0 ? 1 : 0;
+            VJ_TRY(plan_clusters(lps, count, open, mats(tag), d_roff.get(), d_coff.get(), cl, st));
+            bool general = false;
+            for (int i = 0, q = 0; i < count; ++i) q += open[i], general = general || q > static_cast<int>(cl.insts.size());
+            const unsigned cg = (count + 127) / 128;
+            k_bassign<<<cg, 128, 0, st>>>(count, cl.d_on.get(), 0, S.status, S.done);
+            k_bassign<<<cg, 128, 0, st>>>(count, cl.d_on.get(), 1, S.status, done_cl.get());
+            note_launch(2);
+            if (!cl.insts.empty()) VJ_CUDA(cudaMemsetAsync(cl_shared.get(), 0, sizeof(ClControl) * cl.insts.size(), st));
+            int64_t budget = 1;   // chunks of this launch
             if (remaining >= K) {
+                // without a time limit: launches of growing length, each planned for what is left
+                budget = first;
+                first = std::min<int64_t>(2 * first, kMaxLaunchChunks);
+                if (timed && pass_chunks > 0) {
+                    // chunks that fit in the time left at this pass's measured rate (at least one)
+                    const double per_chunk = pass_seconds / static_cast<double>(pass_chunks);
+                    const double left_s = o.time_limit - seconds_since(t_start);
+                    const double fit = per_chunk > 0.0 ? left_s / per_chunk : static_cast<double>(kMaxLaunchChunks);
+                    budget = fit >= kMaxLaunchChunks ? kMaxLaunchChunks : (fit < 1.0 ? 1 : static_cast<int64_t>(fit));
+                }
+                if (remaining / K < budget) budget = remaining / K;
+            }
+            const int64_t iters = remaining >= K ? budget * K : remaining;
+            const auto t_launch = Clock::now();
+            const long long chunks_before = hc->chunks;
+            VJ_TRY(fork_clusters(tag, cl, iters));
+            if (general && remaining >= K) {
                 if (!guard.e[k]) {
                     VJ_CUDA(cudaGraphCreate(&guard.g[k], 0));
                     cudaGraphConditionalHandle again;
@@ -932,39 +1343,31 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                     graph_kernels[k] = launch_count() - before;
                     launch_count() = before;
                 }
-                int64_t budget = kFirstLaunchChunks;
-                if (pass_chunks > 0) {
-                    // chunks that fit in the time left at this pass's measured rate (at least one)
-                    const double per_chunk = pass_seconds / static_cast<double>(pass_chunks);
-                    const double left_s = o.time_limit - seconds_since(t_start);
-                    const double fit = per_chunk > 0.0 ? left_s / per_chunk : static_cast<double>(kMaxLaunchChunks);
-                    budget = fit >= kMaxLaunchChunks ? kMaxLaunchChunks : (fit < 1.0 ? 1 : static_cast<int64_t>(fit));
-                }
-                if (remaining / K < budget) budget = remaining / K;
-                const long long chunks_before = hc->chunks;
-                const auto t_launch = Clock::now();
                 hc->left = static_cast<int>(budget);
                 VJ_CUDA(cudaMemcpyAsync(&counters.get()->left, &hc->left, sizeof(int), cudaMemcpyHostToDevice, st));
                 VJ_CUDA(cudaGraphLaunch(guard.e[k], st));
-                VJ_CUDA(cudaMemcpyAsync(hc, counters.get(), sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
-                VJ_CUDA(cudaStreamSynchronize(st));
-                const long long ran = hc->chunks - chunks_before;
-                pass_chunks += ran;
-                pass_seconds += seconds_since(t_launch);
-                note_launch(graph_kernels[k] * ran);
-                launched += ran * K;
-                if (o.verbose)
-                    std::fprintf(stderr, "[vajra] batch %s pass: %lld chunks to iteration %lld, %d active, %.1f ms\n",
-                                 k == 0 ? "FP32" : "FP64", ran, static_cast<long long>(launched), hc->active,
-                                 1e3 * seconds_since(t_start));
-                if (ran < 1 || ran > budget) return VAJRA_ERR_INTERNAL;   // the loop runs 1..budget chunks
-            } else {
+            } else if (general) {
                 chunk(tag, static_cast<int>(remaining), cudaGraphConditionalHandle{}, 0);
                 VJ_LAUNCH_CHECK();
-                launched += remaining;
-                VJ_CUDA(cudaMemcpyAsync(hc, counters.get(), sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
-                VJ_CUDA(cudaStreamSynchronize(st));
             }
+            VJ_TRY(join_clusters(cl));
+            k_btotals<<<1, 1024, 0, st>>>(count, S.done, done_cl.get(), S.total, cl_shared.get(), static_cast<int>(cl.insts.size()), counters.get());
+            VJ_LAUNCH_CHECK();
+            note_launch(1);
+            VJ_CUDA(cudaMemcpyAsync(hc, counters.get(), sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
+            VJ_CUDA(cudaStreamSynchronize(st));
+            if (hc->wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
+            const long long ran = hc->chunks - chunks_before;
+            note_launch(graph_kernels[k] * ran);
+            if (general && remaining >= K && (ran < 1 || ran > budget)) return VAJRA_ERR_INTERNAL;   // the loop runs 1..budget chunks
+            pass_chunks += budget;
+            pass_seconds += seconds_since(t_launch);
+            // an unfinished instance has run all of it; else the pass is as long as its longest instance
+            launched = hc->active > 0 || k == 1 ? launched + iters : hc->most;
+            if (o.verbose)
+                std::fprintf(stderr, "[vajra] batch %s pass: %lld chunks outside clusters, to iteration %lld, %d active, %.1f ms\n",
+                             k == 0 ? "FP32" : "FP64", ran, static_cast<long long>(launched), hc->active,
+                             1e3 * seconds_since(t_start));
             if (hc->active == 0) break;
             if (seconds_since(t_start) > o.time_limit) { time_out = true; break; }
         }
@@ -976,9 +1379,11 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                                                        x.get(), x0.get(), xc.get(), x_last.get(), y.get(), y0.get(),
                                                        yc.get(), y_last.get(), S.status);
         k_bhandover_state<<<(count + 127) / 128, 128, 0, st>>>(count, o.reflection, S);
-        k_bcount<<<1, 1024, 0, st>>>(count, S.done, counters.get(), cudaGraphConditionalHandle{}, 0);
+        k_bassign<<<(count + 127) / 128, 128, 0, st>>>(count, nullptr, 0, S.status, S.done);
+        k_bassign<<<(count + 127) / 128, 128, 0, st>>>(count, nullptr, 1, S.status, done_cl.get());
+        k_btotals<<<1, 1024, 0, st>>>(count, S.done, done_cl.get(), S.total, cl_shared.get(), 0, counters.get());
         VJ_LAUNCH_CHECK();
-        note_launch(3);
+        note_launch(5);
         VJ_CUDA(cudaMemcpyAsync(hc, counters.get(), sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
     }

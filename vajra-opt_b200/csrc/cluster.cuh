@@ -27,6 +27,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "halpern_state.cuh"
 #include "spmv.cuh"
 
 namespace vajra {
@@ -106,6 +107,16 @@ inline int64_t pad4(int64_t v) { return (v + 3) / 4 * 4; }
 inline size_t cl_smem_bytes(size_t t, size_t value, int64_t m, int64_t n, int64_t nnz, int parts, int threads) {
     const size_t share = static_cast<size_t>(nnz + nnz / 2) / parts + 2 * threads;
     return t * (pad4(n + 1) + pad4(m + 1)) + 2 * share * (value + 4) + 8 * threads + 24 * kClMaxLong + 1024;
+}
+
+// Whether an LP can go to a cluster of `ctas` CTAs: indices of 16 bits, lane-group row sums, at most
+// `threads` rows and columns and kClMaxChains chains a thread in every CTA (from equal shares; a
+// CTA that gets more says so when it deals its slices), and the entries in shared memory.
+inline bool cl_fits(size_t t, int64_t m, int64_t n, int64_t nnz, int group_a, int group_at, int ctas, int threads) {
+    if (group_a < 1 || group_a > 32 || group_at < 1 || group_at > 32 || m >= 65535 || n >= 65535) return false;
+    if (std::max(cl_slice_rows(m, nnz, ctas), cl_slice_rows(n, nnz, ctas)) > threads) return false;
+    if (std::max(m / ctas * group_a, n / ctas * group_at) / threads >= kClMaxChains) return false;
+    return cl_smem_bytes(t, t, m, n, nnz, ctas, threads) <= kClSmemCap;
 }
 
 // The dynamic shared memory of a cluster kernel and an array in it.  Arrays are kept as offsets,
@@ -505,6 +516,204 @@ struct ClCore {
     __device__ __forceinline__ T col_sum(const ClMat<V>& at, const ClInfo& I) { return sum(tc, tpr_c, at, I.cols, yf); }
     __device__ __forceinline__ T row_sum(const ClMat<V>& a, const ClInfo& I) { return sum(tr, tpr_r, a, I.rows, xb()); }
 };
+
+// ----- chunks of Halpern iterations ----------------------------------------------------------
+// What an iteration and a check need to know of the solver's state, by chunk.
+struct ClControl {
+    double tau, sigma, inv_sigma, gamma;
+    long long k_base;
+    int stop;       // no further chunk
+    int restart;    // the candidate becomes iterate and anchor
+    int wait_error; // a bounded wait ran out somewhere in the cluster
+    int no_fit;     // a CTA's slices do not fit its shared memory: nothing was done
+};
+// The vectors of the LP(s); an instance's rows / columns start at the offsets its runner is given.
+template <typename T>
+struct ClVectors {
+    const T* c; const T* cl; const T* cu; const T* rl; const T* ru;
+    T* x; T* x0; T* xc; T* xprev; T* y; T* y0; T* yc; T* yprev;   // xprev, yprev may be null
+    double* x_last; double* y_last;
+    const double* a64; const double* at64;   // the matrices' FP64 values (entry by entry as V)
+};
+template <typename T>
+struct ClMats { ClMat<T> a, at; };   // in shared memory
+
+constexpr int kClWeights = 128;   // Halpern weights kept ahead
+
+__device__ __forceinline__ unsigned long long ns_now() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Sums / maxima (MAXES: bit q set) of Q values a thread over the CTA, into part[0, Q): the warps'
+// values go to shared memory, then a thread per quantity adds them up.  In a fixed order.
+constexpr int kClWarps = kClThreads / 32;
+template <int Q, uint32_t MAXES>
+__device__ __forceinline__ void cl_reduce(double (&v)[Q], double* red, double* part) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        v[q] = (MAXES >> q & 1u) ? warp_reduce<OpMax>(v[q]) : warp_reduce<OpSum>(v[q]);
+        if (lane == 0) red[q * kClWarps + warp] = v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < Q) {
+        const bool is_max = MAXES >> threadIdx.x & 1u;
+        double t = 0.0;
+        for (int w = 0; w < warps; ++w) {
+            const double p = red[threadIdx.x * kClWarps + w];
+            t = is_max ? fmax(t, p) : t + p;
+        }
+        part[threadIdx.x] = t;
+    }
+}
+// The same over the CTAs' partials (Q each, in global memory), into red[0, Q).
+template <int Q, uint32_t MAXES>
+__device__ __forceinline__ void cl_combine(const double* part, int ctas, double* red) {
+    if (threadIdx.x < Q) {
+        const bool is_max = MAXES >> threadIdx.x & 1u;
+        double t = 0.0;
+        for (int r = 0; r < ctas; ++r) {
+            const double p = __ldcg(part + r * Q + threadIdx.x);
+            t = is_max ? fmax(t, p) : t + p;
+        }
+        red[threadIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+// Up to max_chunks chunks of `K` iterations and a check each (the last one shorter where the
+// iteration budget ends), until the solver's control stops the LP.  The arithmetic is that of the
+// two-launch iteration: only where the data is differs, and the order of the checks' FP64 sums.
+// Pol: `start(ctl)` gives the control of the first chunk (rank 0, all threads), `partials(i, ax,
+// j, aty, rank)` stores this CTA's part of a check (i / j: this thread's row / column, -1: none),
+// `decide(ctas, len, ns_primal, ns_dual, ctl)` takes the decision (rank 0, all threads) and
+// `finish()` puts the state back (rank 0).  Rank 0 hands the control to its peers through *shared,
+// in global memory.  Returns false when a slice does not fit.
+template <typename T, int NT, class Pol>
+__device__ __forceinline__ bool cl_run(const ClVectors<T>& P, const ClMats<T>& M, int row0, int col0, Pol& pol,
+                                       ClControl* shared, int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ T hw[2 * kClWeights];
+    __shared__ ClControl now;
+    const int tid = threadIdx.x;
+    ClCore<T, T> core;
+    const bool fits = core.begin(M.a, M.at, smem_bytes, I);
+    for (int i = tid; i < I.m; i += NT) core.yf[i] = P.y[row0 + i];
+    if (core.rank == 0) {
+        if (tid == 0) now.wait_error = now.no_fit = now.restart = 0;
+        __syncthreads();
+        pol.start(now);
+        __syncthreads();
+        if (tid == 0) *shared = now;
+    }
+    cl_barrier();
+    if (!fits && tid == 0) shared->no_fit = 1;
+    cl_barrier();
+    auto read_control = [&]() {   // written before a cluster barrier
+        constexpr int kWords = sizeof(ClControl) / 4;
+        static_assert(sizeof(ClControl) % 4 == 0 && kWords <= NT, "ClControl is copied in words");
+        if (tid < kWords) reinterpret_cast<int*>(&now)[tid] = __ldcg(reinterpret_cast<const int*>(shared) + tid);
+        __syncthreads();
+    };
+    read_control();
+    if (now.no_fit) return false;
+    // My column and my row, if I own one (-1: none).
+    const int jl = core.my_col(I), il = core.my_row(I);
+    const int j = jl < 0 ? -1 : col0 + jl, i = il < 0 ? -1 : row0 + il;
+    T x = T(0), x0 = T(0), c = T(0), cl = T(0), cu = T(0), y = T(0), y0 = T(0), rl = T(0), ru = T(0);
+    if (j >= 0) { x = P.x[j]; x0 = P.x0[j]; c = P.c[j]; cl = P.cl[j]; cu = P.cu[j]; }
+    if (i >= 0) { y = P.y[i]; y0 = P.y0[i]; rl = P.rl[i]; ru = P.ru[i]; }
+    for (int chunk = 0; chunk < max_chunks && budget > 0 && !now.stop; ++chunk) {
+        const int len = budget < K ? static_cast<int>(budget) : K;
+        budget -= len;
+        const T tau = static_cast<T>(now.tau), sigma = static_cast<T>(now.sigma), inv_sigma = static_cast<T>(now.inv_sigma),
+                g = static_cast<T>(now.gamma);
+        unsigned int t0 = 0, t1 = 0, t2 = 0;
+        // Turn kk < len is an iteration.  Turn len forms the check's products: the candidate takes
+        // the place of x_bar and y in the full vectors.
+#pragma unroll 1
+        for (int kk = 0; kk <= len; ++kk) {
+            const bool check = kk == len;
+            const int slot = kk & (kClWeights - 1);
+            if (slot == 0) {   // everyone is past the last use of the old weights
+                const long long k_base = now.k_base;
+                for (int q = tid; q < kClWeights; q += NT) {
+                    const double k = static_cast<double>(k_base + kk + q);
+                    hw[2 * q] = static_cast<T>((k + 1.0) / (k + 2.0));
+                    hw[2 * q + 1] = static_cast<T>(1.0 / (k + 2.0));
+                }
+                __syncthreads();
+            }
+            if (kk == 1) t0 = static_cast<unsigned int>(ns_now());
+            if (check) {
+                cl_barrier();   // every row sum is done with x_bar
+                if (j >= 0) core.xb()[jl] = P.xc[j];
+                if (i >= 0) core.yf[il] = P.yc[i];
+                core.exchange_both(I);
+                if constexpr (sizeof(T) == 4) {   // FP64 values, from global memory
+                    const double ax = cl_sum64<T, T>(M.a, I.rows, core.tr.row, P.a64, core.xb());
+                    const double aty = cl_sum64<T, T>(M.at, I.cols, core.tc.row, P.at64, core.yf);
+                    pol.partials(i, ax, j, aty, core.rank);
+                    break;
+                }
+            }
+            const T w1 = hw[2 * slot], w0 = hw[2 * slot + 1];
+            const T v = core.col_sum(M.at, I);
+            if (!check) {
+                if (j >= 0) {
+                    const T xo = x;
+                    T xp, xbn;
+                    halpern_primal(xo, v, c, cl, cu, x0, tau, w1, w0, g, &xp, &xbn, &x);
+                    core.xb()[jl] = xbn;
+                    if (kk == len - 1) { P.xc[j] = xp; if (P.xprev) P.xprev[j] = xo; }
+                }
+                core.exchange_x(I);
+                if (kk == 1) t1 = static_cast<unsigned int>(ns_now());
+            }
+            const T w = core.row_sum(M.a, I);
+            if (!check) {
+                if (i >= 0) {
+                    const T yo = y;
+                    T yp;
+                    halpern_dual(yo, w, rl, ru, y0, sigma, inv_sigma, w1, w0, g, &yp, &y);
+                    core.yf[il] = y;
+                    if (kk == len - 1) { P.yc[i] = yp; if (P.yprev) P.yprev[i] = yo; }
+                }
+                if (kk < len - 1) core.exchange_y(I);
+                if (kk == 1) t2 = static_cast<unsigned int>(ns_now());
+            } else {
+                pol.partials(i, static_cast<double>(w), j, static_cast<double>(v), core.rank);
+            }
+        }
+        if (core.dead) shared->wait_error = 1;
+        cl_barrier();
+        if (core.rank == 0) {
+            if (tid == 0) now.wait_error = *static_cast<volatile int*>(&shared->wait_error);
+            pol.decide(static_cast<int>(core.size), len, len > 2 ? static_cast<double>(t1 - t0) : 0.0, static_cast<double>(t2 - t1), now);
+            __syncthreads();
+            if (tid == 0) {
+                if (now.wait_error) now.stop = 1;
+                *shared = now;
+            }
+        }
+        cl_barrier();
+        read_control();
+        if (now.restart) {
+            if (j >= 0) { x = x0 = P.xc[j]; P.x_last[j] = static_cast<double>(x); }
+            if (i >= 0) { y = y0 = P.yc[i]; P.y_last[i] = static_cast<double>(y); }
+        }
+        if (now.stop) break;
+        if (i >= 0) core.yf[il] = y;
+        core.exchange_y(I);
+    }
+    if (j >= 0) { P.x[j] = x; P.x0[j] = x0; }
+    if (i >= 0) { P.y[i] = y; P.y0[i] = y0; }
+    if (core.rank == 0) pol.finish();
+    cl_barrier();   // no CTA ends while a peer may still send to it
+    return true;
+}
 
 // Launches `kernel` on `clusters` clusters of `ctas` CTAs; errors are left for cudaGetLastError.
 template <typename... Params, typename... Args>

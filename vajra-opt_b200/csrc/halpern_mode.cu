@@ -531,213 +531,97 @@ void enqueue_iteration(Phase<T>& ph, const CsrView& a, const CsrView& at, HState
 }
 
 // ----- cluster-resident iterations (cluster.cuh) ------------------------------------------
-// One LP as the cluster kernel reads it: matrices in the phase's precision and in FP64 (checks),
-// the phase's vectors, the checks' vectors.
-template <typename T>
-struct ClHalpern {
-    ClMat<T> a, at;
-    const double* a64; const double* at64;
-    const T* c; const T* cl; const T* cu; const T* rl; const T* ru;
-    T* x; T* x0; T* xc; T* xprev; T* y; T* y0; T* yc; T* yprev;
+// The checks' vectors of the LP.
+struct KktVectors {
     const double* c_s; const double* cl_o; const double* cu_o; const double* cs;
     const double* rl_s; const double* ru_s; const double* rl_o; const double* ru_o; const double* rs;
-    double* x_last; double* y_last;
 };
-constexpr int kClWeights = 128;   // Halpern weights kept ahead
-
-__device__ __forceinline__ unsigned long long ns_now() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
+constexpr uint32_t kKktMaxes = ((1u << kQ) - (1u << kNS)) | (((1u << kQ) - (1u << kNS)) << kQ);   // rows' values, then columns'
 
 // The parts of a check outside the row sums, out of line: inlined, their registers would push
-// the iteration's into local memory.  One value of each kind per thread: the warps' partials go
-// to shared memory, and a thread per quantity adds them up.
-constexpr int kClWarps = kClThreads / 32;
+// the iteration's into local memory.
 template <typename T>
-__device__ __noinline__ void cl_check_partials(const ClHalpern<T>& P, int i, double ax, int j, double aty,
-                                               double (&red)[2 * kQ * kClWarps], double* part) {
+__device__ __noinline__ void cl_kkt_partials(const ClVectors<T>& P, const KktVectors& V, int i, double ax, int j, double aty,
+                                             double* red, double* part) {
     double v[2 * kQ];
 #pragma unroll
     for (int q = 0; q < 2 * kQ; ++q) v[q] = 0.0;
     if (i >= 0)
-        kkt_row_terms(ax, static_cast<double>(P.yc[i]), static_cast<double>(P.yprev[i]), P.rl_s[i], P.ru_s[i], P.rl_o[i],
-                      P.ru_o[i], P.rs[i], P.y_last[i], *reinterpret_cast<double(*)[kQ]>(v));
+        kkt_row_terms(ax, static_cast<double>(P.yc[i]), static_cast<double>(P.yprev[i]), V.rl_s[i], V.ru_s[i], V.rl_o[i],
+                      V.ru_o[i], V.rs[i], P.y_last[i], *reinterpret_cast<double(*)[kQ]>(v));
     if (j >= 0)
-        kkt_col_terms(aty, static_cast<double>(P.xc[j]), static_cast<double>(P.xprev[j]), P.c_s[j], P.cl_o[j], P.cu_o[j],
-                      P.cs[j], P.x_last[j], *reinterpret_cast<double(*)[kQ]>(v + kQ));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < 2 * kQ; ++q) {
-        v[q] = q % kQ < kNS ? warp_reduce<OpSum>(v[q]) : warp_reduce<OpMax>(v[q]);
-        if (lane == 0) red[q * kClWarps + warp] = v[q];
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 * kQ) {
-        const bool is_max = threadIdx.x % kQ >= kNS;
-        double t = 0.0;
-        for (int w = 0; w < warps; ++w) {
-            const double p = red[threadIdx.x * kClWarps + w];
-            t = is_max ? fmax(t, p) : t + p;
-        }
-        part[threadIdx.x] = t;
-    }
+        kkt_col_terms(aty, static_cast<double>(P.xc[j]), static_cast<double>(P.xprev[j]), V.c_s[j], V.cl_o[j], V.cu_o[j],
+                      V.cs[j], P.x_last[j], *reinterpret_cast<double(*)[kQ]>(v + kQ));
+    cl_reduce<2 * kQ, kKktMaxes>(v, red, part);
 }
-// Rank 0, all threads: the peers' partials combined, the decision taken on the copy `now` of
-// the state, and the state written back.
-__device__ __noinline__ void cl_decide(const double* part, int ctas, double (&red)[2 * kQ * kClWarps], ControlParams& cp, HState& now,
-                                       HState* st, double ns_primal, double ns_dual) {
-    const int tid = threadIdx.x;
-    if (tid < 2 * kQ) {   // thread q: rows' quantity q, thread kQ + q: columns'
-        const bool is_max = tid % kQ >= kNS;
-        double t = 0.0;
-        for (int r = 0; r < ctas; ++r) {
-            const double p = __ldcg(part + 2 * r * kQ + tid);
-            t = is_max ? fmax(t, p) : t + p;
-        }
-        red[tid] = t;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double s[kS], f[4];
-        for (int q = 0; q < kNS; ++q) { s[q] = red[q]; s[kNS + q] = red[kQ + q]; }
-        f[0] = fmax(red[kNS], red[kQ + kNS]);
-        f[1] = red[kNS + 1];
-        f[2] = red[kNS + 2];
-        f[3] = fmax(red[kNS + 3], red[kQ + kNS + 3]);
-        now.wait_error = *static_cast<volatile int*>(&st->wait_error);
-        halpern_decide(s, f, cp, &now);
-        if (now.wait_error) now.stop = 1;
-        if (ns_primal > 0.0) {
-            now.t_primal_ns[cp.phase] += ns_primal;
-            now.t_dual_ns[cp.phase] += ns_dual;
-            now.t_samples[cp.phase] += 1;
-        }
-    }
-    __syncthreads();
-    for (int q = tid; q < static_cast<int>(sizeof(HState) / 4); q += blockDim.x)
-        reinterpret_cast<int*>(st)[q] = reinterpret_cast<const int*>(&now)[q];
+__device__ __noinline__ void cl_kkt_decide(const double* part, int ctas, double* red, ControlParams& cp, HState& hs) {
+    cl_combine<2 * kQ, kKktMaxes>(part, ctas, red);
+    if (threadIdx.x != 0) return;
+    double s[kS], f[4];
+    for (int q = 0; q < kNS; ++q) { s[q] = red[q]; s[kNS + q] = red[kQ + q]; }
+    f[0] = fmax(red[kNS], red[kQ + kNS]);
+    f[1] = red[kNS + 1];
+    f[2] = red[kNS + 2];
+    f[3] = fmax(red[kNS + 3], red[kQ + kNS + 3]);
+    halpern_decide(s, f, cp, &hs);
 }
 
-// Up to max_chunks chunks of `K` iterations and a check each (the last one shorter where the
-// iteration budget ends), until the LP stops or leaves the phase.  One cluster.  The arithmetic
-// is that of the kernels above: an iteration and a check differ only in where the data is and
-// in the order of the checks' FP64 sums.
+// The single LP's control: rank 0 keeps the solver's state in shared memory between the chunks
+// (read from global memory, a decision waited for a dozen L2 loads).
+template <typename T>
+struct HalpernControl {
+    const ClVectors<T>& P;
+    const KktVectors& V;
+    HState* st;        // in global memory
+    HState& hs;        // rank 0's copy
+    ControlParams& cp; // in shared memory
+    double* red;
+    double* part;
+    __device__ void control(ClControl& c) const {
+        c.tau = hs.tau; c.sigma = hs.sigma; c.inv_sigma = hs.inv_sigma; c.gamma = hs.gamma_now;
+        c.k_base = hs.k_base; c.stop = hs.stop || hs.phase != cp.phase; c.restart = hs.restart_flag;
+    }
+    __device__ void start(ClControl& c) const {
+        static_assert(sizeof(HState) % 4 == 0, "HState is copied in words");
+        for (int q = threadIdx.x; q < static_cast<int>(sizeof(HState) / 4); q += blockDim.x)
+            reinterpret_cast<int*>(&hs)[q] = reinterpret_cast<const int*>(st)[q];
+        __syncthreads();
+        if (threadIdx.x == 0) control(c);
+    }
+    __device__ void partials(int i, double ax, int j, double aty, uint32_t rank) const {
+        cl_kkt_partials<T>(P, V, i, ax, j, aty, red, part + rank * 2 * kQ);
+    }
+    __device__ void decide(int ctas, int len, double ns_primal, double ns_dual, ClControl& c) const {
+        if (threadIdx.x == 0) cp.len = len;
+        cl_kkt_decide(part, ctas, red, cp, hs);
+        if (threadIdx.x != 0) return;
+        if (ns_primal > 0.0) {
+            hs.t_primal_ns[cp.phase] += ns_primal;
+            hs.t_dual_ns[cp.phase] += ns_dual;
+            hs.t_samples[cp.phase] += 1;
+        }
+        control(c);
+    }
+    __device__ void finish() const {
+        __syncthreads();
+        for (int q = threadIdx.x; q < static_cast<int>(sizeof(HState) / 4); q += blockDim.x)
+            reinterpret_cast<int*>(st)[q] = reinterpret_cast<const int*>(&hs)[q];
+    }
+};
+
+// One cluster, one LP.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, 1)
-k_cluster_halpern(const __grid_constant__ ClHalpern<T> P, const __grid_constant__ ControlParams cp0, HState* st, double* part,
-                  int K, long long budget, int max_chunks, uint32_t smem_bytes) {
-    __shared__ ClInfo I;
+k_cluster_halpern(const __grid_constant__ ClVectors<T> P, const __grid_constant__ KktVectors V,
+                  const __grid_constant__ ClMats<T> M, const __grid_constant__ ControlParams cp0, HState* st, double* part,
+                  ClControl* shared, int K, long long budget, int max_chunks, uint32_t smem_bytes) {
     __shared__ double red[2 * kQ * kClWarps];
-    __shared__ T hw[2 * kClWeights];
-    __shared__ HState now;
+    __shared__ HState hs;
     __shared__ ControlParams cp;
-    const int phase = cp0.phase;
-    if (st->stop || st->phase != phase) return;   // uniform over the cluster
-    ClCore<T, T> core;
-    if (!core.begin(P.a, P.at, smem_bytes, I) && threadIdx.x == 0) st->no_fit = 1;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < I.m; i += NT) core.yf[i] = P.y[i];
-    if (tid == 0) cp = cp0;
-    cl_barrier();
-    if (*static_cast<volatile int*>(&st->no_fit)) return;   // the host takes the general path
-    // My column and my row, if I own one (-1: none).
-    const int j = core.my_col(I), i = core.my_row(I);
-    T x = T(0), x0 = T(0), c = T(0), cl = T(0), cu = T(0), y0 = T(0), rl = T(0), ru = T(0);
-    if (j >= 0) { x = P.x[j]; x0 = P.x0[j]; c = P.c[j]; cl = P.cl[j]; cu = P.cu[j]; }
-    T y = T(0);
-    if (i >= 0) { y = P.y[i]; y0 = P.y0[i]; rl = P.rl[i]; ru = P.ru[i]; }
-    // The solver's state: every CTA copies it into shared memory; rank 0 decides there and
-    // writes it back (a decision that read it from global memory waited for a dozen L2 loads).
-    static_assert(sizeof(HState) % 4 == 0, "HState is copied in words");
-    auto read_state = [&]() {   // written by rank 0 before a cluster barrier, or by the host
-        for (int q = tid; q < static_cast<int>(sizeof(HState) / 4); q += NT)
-            reinterpret_cast<int*>(&now)[q] = __ldcg(reinterpret_cast<const int*>(st) + q);
-        __syncthreads();
-    };
-    read_state();
-    for (int chunk = 0; chunk < max_chunks && budget > 0; ++chunk) {
-        const int len = budget < K ? static_cast<int>(budget) : K;
-        budget -= len;
-        const T tau = static_cast<T>(now.tau), sigma = static_cast<T>(now.sigma), inv_sigma = static_cast<T>(now.inv_sigma),
-                g = static_cast<T>(now.gamma_now);
-        unsigned int t0 = 0, t1 = 0, t2 = 0;
-        // Turn kk < len is an iteration.  Turn len forms the check's products: the candidate takes
-        // the place of x_bar and y in the full vectors.
-#pragma unroll 1
-        for (int kk = 0; kk <= len; ++kk) {
-            const bool check = kk == len;
-            const int slot = kk & (kClWeights - 1);
-            if (slot == 0) {   // everyone is past the last use of the old weights
-                const long long k_base = now.k_base;
-                for (int q = tid; q < kClWeights; q += NT) {
-                    const double k = static_cast<double>(k_base + kk + q);
-                    hw[2 * q] = static_cast<T>((k + 1.0) / (k + 2.0));
-                    hw[2 * q + 1] = static_cast<T>(1.0 / (k + 2.0));
-                }
-                __syncthreads();
-            }
-            if (kk == 1) t0 = static_cast<unsigned int>(ns_now());
-            if (check) {
-                cl_barrier();   // every row sum is done with x_bar
-                if (j >= 0) core.xb()[j] = P.xc[j];
-                if (i >= 0) core.yf[i] = P.yc[i];
-                core.exchange_both(I);
-                if constexpr (sizeof(T) == 4) {   // FP64 values, from global memory
-                    const double ax = cl_sum64<T, T>(P.a, I.rows, core.tr.row, P.a64, core.xb());
-                    const double aty = cl_sum64<T, T>(P.at, I.cols, core.tc.row, P.at64, core.yf);
-                    cl_check_partials<T>(P, i, ax, j, aty, red, part + 2 * core.rank * kQ);
-                    break;
-                }
-            }
-            const T w1 = hw[2 * slot], w0 = hw[2 * slot + 1];
-            const T v = core.col_sum(P.at, I);
-            if (!check) {
-                if (j >= 0) {
-                    const T xo = x;
-                    T xp, xbn;
-                    halpern_primal(xo, v, c, cl, cu, x0, tau, w1, w0, g, &xp, &xbn, &x);
-                    core.xb()[j] = xbn;
-                    if (kk == len - 1) { P.xc[j] = xp; P.xprev[j] = xo; }
-                }
-                core.exchange_x(I);
-                if (kk == 1) t1 = static_cast<unsigned int>(ns_now());
-            }
-            const T w = core.row_sum(P.a, I);
-            if (!check) {
-                if (i >= 0) {
-                    const T yo = y;
-                    T yp;
-                    halpern_dual(yo, w, rl, ru, y0, sigma, inv_sigma, w1, w0, g, &yp, &y);
-                    core.yf[i] = y;
-                    if (kk == len - 1) { P.yc[i] = yp; P.yprev[i] = yo; }
-                }
-                if (kk < len - 1) core.exchange_y(I);
-                if (kk == 1) t2 = static_cast<unsigned int>(ns_now());
-            } else {
-                cl_check_partials<T>(P, i, static_cast<double>(w), j, static_cast<double>(v), red, part + 2 * core.rank * kQ);
-            }
-        }
-        if (core.dead) st->wait_error = 1;
-        if (tid == 0) cp.len = len;
-        cl_barrier();
-        if (core.rank == 0)
-            cl_decide(part, static_cast<int>(core.size), red, cp, now, st, len > 2 ? static_cast<double>(t1 - t0) : 0.0,
-                      static_cast<double>(t2 - t1));
-        cl_barrier();
-        read_state();
-        if (now.restart_flag) {
-            if (j >= 0) { x = x0 = P.xc[j]; P.x_last[j] = static_cast<double>(x); }
-            if (i >= 0) { y = y0 = P.yc[i]; P.y_last[i] = static_cast<double>(y); }
-        }
-        if (now.stop || now.phase != phase) break;
-        if (i >= 0) core.yf[i] = y;
-        core.exchange_y(I);
-    }
-    if (j >= 0) { P.x[j] = x; P.x0[j] = x0; }
-    if (i >= 0) { P.y[i] = y; P.y0[i] = y0; }
-    cl_barrier();   // no CTA ends while a peer may still send to it
+    if (st->stop || st->phase != cp0.phase) return;   // uniform over the cluster
+    if (threadIdx.x == 0) cp = cp0;
+    HalpernControl<T> pol{P, V, st, hs, cp, red, part};
+    cl_run<T, NT>(P, M, 0, 0, pol, shared, K, budget, max_chunks, smem_bytes);
 }
 
 // How an LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
@@ -757,16 +641,10 @@ auto cluster_kernel(int threads) -> decltype(&k_cluster_halpern<T, 256>) {
 // line lies at 512.  Every thread forms at most kClMaxChains chains of a row.
 template <typename T>
 ClusterPlan plan_cluster(const CsrView& a, const CsrView& at, int64_t nnz) {
-    const auto lanes = [](const CsrView& v) { return v.group >= 1 && v.group <= 32; };
-    if (!lanes(a) || !lanes(at) || a.rows >= 65535 || at.rows >= 65535) return {};
     for (int ctas = 1; ctas <= kClMaxCtas; ctas *= 2) {
-        const int64_t nr = cl_slice_rows(a.rows, nnz, ctas), nc = cl_slice_rows(at.rows, nnz, ctas);
-        const int threads = std::max(nr, nc) <= 256 ? 256 : 512;
-        // chains a thread forms, from an equal share (a CTA that gets more says so: no_fit)
-        const int64_t chains = std::max(a.rows / ctas * static_cast<int64_t>(a.group), at.rows / ctas * static_cast<int64_t>(at.group)) / threads;
-        if (std::max(nr, nc) > threads || chains >= kClMaxChains) continue;
+        const int threads = cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, 256) ? 256 : 512;
+        if (!cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, threads)) continue;
         if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
-        if (cl_smem_bytes(sizeof(T), sizeof(T), a.rows, at.rows, nnz, ctas, threads) > kClSmemCap) continue;
         const cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
         if (e != cudaSuccess) { cudaGetLastError(); continue; }   // no such cluster on this device
         return ClusterPlan{ctas, threads, kClSmemCap};   // all of it: slices may be uneven
@@ -1158,9 +1036,10 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
 
     HState* S = dstate.get();
     HState* hs = nullptr;
-    hs = static_cast<HState*>(pinned_scratch(sizeof(HState)));
+    hs = static_cast<HState*>(pinned_scratch(sizeof(HState) + sizeof(ClControl)));
     if (!hs) { set_error("page-locked host memory for the solver state"); return VAJRA_ERR_OUT_OF_MEMORY; }
 
+    ClControl* hc = reinterpret_cast<ClControl*>(hs + 1);   // what a cluster launch reports
     ControlParams cp{};
     cp.tol = o.tolerance;
     cp.switch_tol = o.mixed_switch_tolerance;
@@ -1189,30 +1068,31 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0 && nnz < kAutotuneMinNnz;
     ClusterPlan cl32, cl64;
     DeviceBuffer<double> cl_part;
+    DeviceBuffer<ClControl> cl_shared;
     if (may_cluster) {
         if (mixed) cl32 = plan_cluster<float>(a32, at32, nnz);
         cl64 = plan_cluster<double>(a64, at64, nnz);
-        if (cl32.ctas || cl64.ctas) VJ_TRY(cl_part.alloc(2 * kQ * kClMaxCtas));
+        if (cl32.ctas || cl64.ctas) {
+            VJ_TRY(cl_part.alloc(2 * kQ * kClMaxCtas));
+            VJ_TRY(cl_shared.alloc(1));
+        }
     }
     auto cluster_chunks = [&](auto& ph, const ClusterPlan& plan, int64_t budget, int chunks) -> vajra_status {
         using T = std::decay_t<decltype(*ph.x.get())>;
-        ClHalpern<T> P;
         const CsrView& ia = ph.phase == 0 ? a32 : a64;
         const CsrView& iat = ph.phase == 0 ? at32 : at64;
-        P.a = ClMat<T>{m, p.csr_ptr.get(), p.csr_idx.get(), ph.csr_val, 0, ia.group, ia.long_len};
-        P.at = ClMat<T>{n, lp.col_ptr.get(), lp.row_idx.get(), ph.csc_val, 0, iat.group, iat.long_len};
-        P.a64 = p.csr_val.get(); P.at64 = p.csc_val.get();
-        P.c = ph.c.get(); P.cl = ph.cl.get(); P.cu = ph.cu.get(); P.rl = ph.rl.get(); P.ru = ph.ru.get();
-        P.x = ph.x.get(); P.x0 = ph.x0.get(); P.xc = ph.xc.get(); P.xprev = ph.xprev.get();
-        P.y = ph.y.get(); P.y0 = ph.y0.get(); P.yc = ph.yc.get(); P.yprev = ph.yprev.get();
-        P.c_s = p.c.get(); P.cl_o = lp.col_lower.get(); P.cu_o = lp.col_upper.get(); P.cs = p.col_scale.get();
-        P.rl_s = p.row_lower.get(); P.ru_s = p.row_upper.get();
-        P.rl_o = lp.row_lower.get(); P.ru_o = lp.row_upper.get(); P.rs = p.row_scale.get();
-        P.x_last = cb.x_last.get(); P.y_last = cb.y_last.get();
+        const ClMats<T> M{ClMat<T>{m, p.csr_ptr.get(), p.csr_idx.get(), ph.csr_val, 0, ia.group, ia.long_len},
+                          ClMat<T>{n, lp.col_ptr.get(), lp.row_idx.get(), ph.csc_val, 0, iat.group, iat.long_len}};
+        const ClVectors<T> P{ph.c.get(), ph.cl.get(), ph.cu.get(), ph.rl.get(), ph.ru.get(), ph.x.get(), ph.x0.get(),
+                             ph.xc.get(), ph.xprev.get(), ph.y.get(), ph.y0.get(), ph.yc.get(), ph.yprev.get(),
+                             cb.x_last.get(), cb.y_last.get(), p.csr_val.get(), p.csc_val.get()};
+        const KktVectors kv{p.c.get(), lp.col_lower.get(), lp.col_upper.get(), p.col_scale.get(), p.row_lower.get(),
+                            p.row_upper.get(), lp.row_lower.get(), lp.row_upper.get(), p.row_scale.get()};
         ControlParams c2 = cp;
         c2.phase = ph.phase;
-        VJ_CUDA(launch_clusters(cluster_kernel<T>(plan.threads), 1, plan.ctas, plan.threads, plan.smem, st, P, c2, S, cl_part.get(), K,
-                                static_cast<long long>(budget), chunks, static_cast<uint32_t>(plan.smem)));
+        VJ_CUDA(launch_clusters(cluster_kernel<T>(plan.threads), 1, plan.ctas, plan.threads, plan.smem, st, P, kv, M, c2, S,
+                                cl_part.get(), cl_shared.get(), K, static_cast<long long>(budget), chunks,
+                                static_cast<uint32_t>(plan.smem)));
         return VAJRA_OK;
     };
     const auto t_iter = Clock::now();
@@ -1229,12 +1109,13 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
             if (cur_phase == 0) { VJ_TRY(cluster_chunks(p32, plan, max_iter - launched, static_cast<int>(chunks))); }
             else { VJ_TRY(cluster_chunks(p64, plan, max_iter - launched, static_cast<int>(chunks))); }
             VJ_CUDA(cudaMemcpyAsync(hs, S, sizeof(HState), cudaMemcpyDeviceToHost, st));
+            VJ_CUDA(cudaMemcpyAsync(hc, cl_shared.get(), sizeof(ClControl), cudaMemcpyDeviceToHost, st));
             VJ_CUDA(cudaStreamSynchronize(st));
             h->transfers++;
-            if (hs->wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
+            if (hc->wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
             cl_seconds += seconds_since(t_launch);
             cl_chunks += (hs->total - launched + K - 1) / K;
-            if (hs->no_fit) { cl32.ctas = cl64.ctas = 0; continue; }   // uneven rows: the general path
+            if (hc->no_fit) { cl32.ctas = cl64.ctas = 0; continue; }   // uneven rows: the general path
             if (hs->total <= launched) return VAJRA_ERR_INTERNAL;   // a launch runs at least one chunk
             launched = hs->total;
         } else {

@@ -28,8 +28,6 @@ struct HState {
     int restart_count;
     int restart_flag;
     int switch_flag;
-    int wait_error;     // a bounded device wait ran out (cluster path)
-    int no_fit;         // a CTA's slices do not fit its shared memory (cluster path)
     int pad;
     // first iteration of every chunk of the cluster path: nanoseconds of its two halves
     double t_primal_ns[2], t_dual_ns[2];   // per phase

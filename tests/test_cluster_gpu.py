@@ -104,3 +104,29 @@ def test_batched_clusters_beside_larger_instances_reach_the_optima(cuda, prec):
     for lp, r in zip(lps, V.solve_batch(lps, precision=prec, iteration_limit=40000)):
         assert r["status_name"] == "OPTIMAL" and relative_kkt(lp, r["x"], r["y"])["rel_kkt"] <= 1.05e-6
         assert r["fp32_iterations"] + r["fp64_iterations"] == r["iterations"]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("every", [7, 100])
+def test_unrolled_on_clusters_matches_the_packed_map(cuda, prec, every):
+    """Alone, every instance fits a cluster; beside one of 7,000 x 20,000 all run packed.  Same row
+    sums in the same order only where the packed matrices have the same mean row length, so the
+    bound is rounding: 30 nonexpansive steps and their reverse, sums of at most 64 products, error
+    <= 2 * 30 * 64 eps of the largest entry, eps the precision of the pass (the gradients of the
+    mixed form come from FP32)."""
+    from vajra_pdhg.autograd import PREC_FP32, PREC_FP64, PREC_MIXED, unrolled
+    p = {"fp64": PREC_FP64, "mixed": PREC_MIXED, "fp32": PREC_FP32}[prec]
+    lps = [W.random_planted(m, n, 6, seed=90 + m) for m, n in ((60, 150), (301, 807), (1000, 3000))]
+    big = W.random_planted(7000, 20000, 6, seed=9)
+    n = sum(lp.num_cols for lp in lps)
+    m = sum(lp.num_rows for lp in lps)
+    w = np.random.default_rng(3).standard_normal(n + big.num_cols)
+    a = unrolled(lps, w[:n], iterations=30, checkpoint_every=every, precision=p, enable_scaling=0)
+    b = unrolled(lps + [big], w, iterations=30, checkpoint_every=every, precision=p, enable_scaling=0)
+    for key, size, eps in (("x", n, 2.0 ** -24 if prec == "fp32" else 2.0 ** -53),
+                           ("loss", len(lps), 2.0 ** -24 if prec == "fp32" else 2.0 ** -53),
+                           ("grad_c", n, 2.0 ** -53 if prec == "fp64" else 2.0 ** -24),
+                           ("grad_row_lower", m, 2.0 ** -53 if prec == "fp64" else 2.0 ** -24),
+                           ("grad_row_upper", m, 2.0 ** -53 if prec == "fp64" else 2.0 ** -24)):
+        u, v = a[key], b[key][:size]
+        np.testing.assert_allclose(u, v, rtol=0, atol=2 * 30 * 64 * eps * (1.0 + np.abs(v).max()), err_msg=key)

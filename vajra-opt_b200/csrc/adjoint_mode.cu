@@ -20,10 +20,30 @@
 #include <vector>
 
 #include "batch_common.cuh"
+#include "cluster_batch.cuh"
 #include "solver.cuh"
 
 namespace vajra {
 namespace {
+
+// One column's and one row's step of the map.
+template <typename T>
+__device__ __forceinline__ void fwd_primal(T xo, T v, T c, T cl, T cu, T tau, T* xn_out, T* xb_out, uint8_t* inside) {
+    const T pre = xo - tau * (c + v);
+    const T xn = pre < cl ? cl : (pre > cu ? cu : pre);
+    *inside = (pre > cl && pre < cu) ? 1 : 0;
+    *xb_out = xn + xn - xo;
+    *xn_out = xn;
+}
+template <typename T>
+__device__ __forceinline__ void fwd_dual(T yo, T w, T rl, T ru, T sg, T* y_out, uint8_t* code_out) {
+    const T q = yo + sg * w;
+    const T t = q / sg;
+    const uint8_t code = t < rl ? 1 : (t > ru ? 2 : 0);
+    const T cl = code == 1 ? rl : (code == 2 ? ru : t);
+    *code_out = code;
+    *y_out = q - sg * cl;
+}
 
 template <typename T>
 struct EpiFwdPrimal {
@@ -33,12 +53,11 @@ struct EpiFwdPrimal {
     uint8_t* mask;   // may be null
     __device__ bool active() const { return true; }
     template <typename Acc> __device__ void operator()(int j, Acc v) const {
-        const T tau = static_cast<T>(step[col_inst[j]]);
-        const T xo = x[j];
-        const T pre = xo - tau * (c[j] + static_cast<T>(v));
-        const T xn = pre < cl[j] ? cl[j] : (pre > cu[j] ? cu[j] : pre);
-        if (mask) mask[j] = (pre > cl[j] && pre < cu[j]) ? 1 : 0;
-        xb[j] = xn + xn - xo;
+        T xn, xbn;
+        uint8_t inside;
+        fwd_primal(x[j], static_cast<T>(v), c[j], cl[j], cu[j], static_cast<T>(step[col_inst[j]]), &xn, &xbn, &inside);
+        if (mask) mask[j] = inside;
+        xb[j] = xbn;
         x[j] = xn;
     }
 };
@@ -51,13 +70,11 @@ struct EpiFwdDual {
     uint8_t* mask;
     __device__ bool active() const { return true; }
     template <typename Acc> __device__ void operator()(int i, Acc w) const {
-        const T sg = static_cast<T>(step[row_inst[i]]);
-        const T q = y[i] + sg * static_cast<T>(w);
-        const T t = q / sg;
-        const uint8_t code = t < rl[i] ? 1 : (t > ru[i] ? 2 : 0);
-        const T cl = code == 1 ? rl[i] : (code == 2 ? ru[i] : t);
+        T yn;
+        uint8_t code;
+        fwd_dual(y[i], static_cast<T>(w), rl[i], ru[i], static_cast<T>(step[row_inst[i]]), &yn, &code);
         if (mask) mask[i] = code;
-        y[i] = q - sg * cl;
+        y[i] = yn;
     }
 };
 
@@ -103,6 +120,161 @@ struct EpiBwdDual {
         yh[i] = yh[i] - static_cast<T>(step[row_inst[i]]) * static_cast<T>(s);
     }
 };
+
+// ----- instances on clusters (cluster.cuh) --------------------------------------------------
+// A step was five launches of a few microseconds' work; here a whole segment (or the whole
+// forward pass) of an instance is one launch, and a step waits for two exchanges.
+template <typename T>
+struct FwdVectors {
+    const T* c; const T* cl; const T* cu; const T* rl; const T* ru;
+    T* x; T* y;
+    const double* step;
+    int n, m;        // of the packed problem
+    T* ckpt;         // null, or (x, y) before the steps 0, every, 2 every, ..
+    int every;
+    uint8_t* pmask; uint8_t* dmask;   // null, or the active sets of every step
+};
+template <typename T>
+struct BwdVectors {
+    T* xh; T* yh;
+    double* g_c; double* g_rl; double* g_ru;
+    const double* step;
+    int n, m;
+    const uint8_t* pmask; const uint8_t* dmask;
+};
+
+// Cluster q: `steps` steps of the map for instance insts[q].
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+k_cluster_forward(const __grid_constant__ FwdVectors<T> F, const __grid_constant__ BMats<T> M, const int* __restrict__ insts,
+                  const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ ClMats<T> mats;
+    const int inst = insts[blockIdx.x / cl_size()];
+    const int r0 = static_cast<int>(roff[inst]), c0 = static_cast<int>(coff[inst]);
+    if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
+    __syncthreads();
+    ClCore<T, T> core;
+    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
+    for (int i = threadIdx.x; i < I.m; i += NT) core.yf[i] = F.y[r0 + i];
+    cl_barrier();
+    if (*static_cast<volatile int*>(failed + inst)) return;   // uniform over the cluster
+    const int jl = core.my_col(I), il = core.my_row(I);
+    const int j = jl < 0 ? -1 : c0 + jl, i = il < 0 ? -1 : r0 + il;
+    const T step = static_cast<T>(F.step[inst]);
+    T x = T(0), c = T(0), cl = T(0), cu = T(0), y = T(0), rl = T(0), ru = T(0);
+    if (j >= 0) { x = F.x[j]; c = F.c[j]; cl = F.cl[j]; cu = F.cu[j]; }
+    if (i >= 0) { y = F.y[i]; rl = F.rl[i]; ru = F.ru[i]; }
+    int to_ckpt = 0;
+    T* ck = F.ckpt;
+#pragma unroll 1
+    for (int k = 0; k < steps; ++k) {
+        if (ck && to_ckpt == 0) {
+            if (j >= 0) ck[j] = x;
+            if (i >= 0) ck[F.n + i] = y;
+            ck += static_cast<size_t>(F.n) + F.m;
+            to_ckpt = F.every;
+        }
+        --to_ckpt;
+        const T v = core.col_sum(mats.at, I);
+        if (j >= 0) {
+            T xn, xbn;
+            uint8_t inside;
+            fwd_primal(x, v, c, cl, cu, step, &xn, &xbn, &inside);
+            if (F.pmask) F.pmask[static_cast<size_t>(k) * F.n + j] = inside;
+            core.xb()[jl] = xbn;
+            x = xn;
+        }
+        core.exchange_x(I);
+        const T w = core.row_sum(mats.a, I);
+        if (i >= 0) {
+            T yn;
+            uint8_t code;
+            fwd_dual(y, w, rl, ru, step, &yn, &code);
+            if (F.dmask) F.dmask[static_cast<size_t>(k) * F.m + i] = code;
+            core.yf[il] = yn;
+            y = yn;
+        }
+        core.exchange_y(I);
+    }
+    if (j >= 0) F.x[j] = x;
+    if (i >= 0) F.y[i] = y;
+    if (core.dead) failed[inst] = 2;
+    cl_barrier();   // no CTA ends while a peer may still send to it
+}
+
+// Cluster q: the reverse of `steps` steps for instance insts[q].  The full y holds w^ = sigma q^,
+// the full x_bar pre^.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+k_cluster_backward(const __grid_constant__ BwdVectors<T> B, const __grid_constant__ BMats<T> M, const int* __restrict__ insts,
+                   const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ ClMats<T> mats;
+    const int inst = insts[blockIdx.x / cl_size()];
+    const int r0 = static_cast<int>(roff[inst]), c0 = static_cast<int>(coff[inst]);
+    if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
+    __syncthreads();
+    ClCore<T, T> core;
+    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
+    cl_barrier();
+    if (*static_cast<volatile int*>(failed + inst)) return;   // uniform over the cluster
+    const int jl = core.my_col(I), il = core.my_row(I);
+    const int j = jl < 0 ? -1 : c0 + jl, i = il < 0 ? -1 : r0 + il;
+    const double sg = B.step[inst];
+    T xh = T(0), yh = T(0);
+    double g_c = 0.0, g_rl = 0.0, g_ru = 0.0;
+    uint8_t code = 0, inside = 0;   // of the step to come: loaded a step ahead
+    if (j >= 0) { xh = B.xh[j]; g_c = B.g_c[j]; if (steps > 0) inside = B.pmask[static_cast<size_t>(steps - 1) * B.n + j]; }
+    if (i >= 0) { yh = B.yh[i]; g_rl = B.g_rl[i]; g_ru = B.g_ru[i]; if (steps > 0) code = B.dmask[static_cast<size_t>(steps - 1) * B.m + i]; }
+#pragma unroll 1
+    for (int k = steps - 1; k >= 0; --k) {
+        const uint8_t code_k = code, inside_k = inside;
+        if (k > 0) {
+            if (j >= 0) inside = B.pmask[static_cast<size_t>(k - 1) * B.n + j];
+            if (i >= 0) code = B.dmask[static_cast<size_t>(k - 1) * B.m + i];
+        }
+        if (i >= 0) {
+            if (code_k == 1) g_rl -= sg * static_cast<double>(yh);
+            if (code_k == 2) g_ru -= sg * static_cast<double>(yh);
+            yh = code_k != 0 ? yh : T(0);
+            core.yf[il] = static_cast<T>(sg) * yh;
+        }
+        core.exchange_y(I);
+        const T xbh = core.col_sum(mats.at, I);
+        if (j >= 0) {
+            const T p = inside_k ? xh + xbh + xbh : T(0);
+            g_c -= sg * static_cast<double>(p);
+            xh = p - xbh;
+            core.xb()[jl] = p;
+        }
+        core.exchange_x(I);
+        const T s = core.row_sum(mats.a, I);
+        if (i >= 0) yh = yh - static_cast<T>(sg) * s;
+    }
+    if (j >= 0) { B.xh[j] = xh; B.g_c[j] = g_c; }
+    if (i >= 0) { B.yh[i] = yh; B.g_rl[i] = g_rl; B.g_ru[i] = g_ru; }
+    if (core.dead) failed[inst] = 2;
+    cl_barrier();
+}
+
+// (x, y) of the instances insts[0, gridDim.y) from a checkpoint.
+template <typename T>
+__global__ void k_load_checkpoint(const int* __restrict__ insts, const int64_t* __restrict__ roff, const int64_t* __restrict__ coff,
+                                  int n, const T* __restrict__ ckpt, T* __restrict__ x, T* __restrict__ y) {
+    const int inst = insts[blockIdx.y], stride = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t j = coff[inst] + t; j < coff[inst + 1]; j += stride) x[j] = ckpt[j];
+    for (int64_t i = roff[inst] + t; i < roff[inst + 1]; i += stride) y[i] = ckpt[n + i];
+}
+
+template <typename T>
+auto forward_kernel(int threads) -> decltype(&k_cluster_forward<T, 256>) {
+    return threads == 256 ? &k_cluster_forward<T, 256> : &k_cluster_forward<T, 512>;
+}
+template <typename T>
+auto backward_kernel(int threads) -> decltype(&k_cluster_backward<T, 256>) {
+    return threads == 256 ? &k_cluster_backward<T, 256> : &k_cluster_backward<T, 512>;
+}
 
 template <typename T>
 __global__ void k_adj_init(int m, int n, const double* __restrict__ cl, const double* __restrict__ cu,
@@ -208,7 +380,7 @@ void values_of(Prepared& p, const T** csr, const T** csc) {
 }
 
 template <typename TF, typename TB>
-vajra_status run_unrolled_t(const PackedHost& P, const vajra_unrolled_opts& o, Prepared& p, const DeviceLp& lp,
+vajra_status run_unrolled_t(const vajra_lp* lps, const int64_t* d_roff, const PackedHost& P, const vajra_unrolled_opts& o, Prepared& p, const DeviceLp& lp,
                             const int* row_inst, const int* col_inst, const int64_t* d_coff, const double* step,
                             const DeviceBuffer<double>& d_w, const double* c_orig_dev, double* h_loss, double* h_x,
                             double* h_gc, double* h_grl, double* h_gru, cudaStream_t st) {
@@ -248,8 +420,64 @@ vajra_status run_unrolled_t(const PackedHost& P, const vajra_unrolled_opts& o, P
     VJ_LAUNCH_CHECK();
     auto ck_x = [&](int s) { return U.ckpt.get() + static_cast<size_t>(s) * (static_cast<size_t>(n) + m); };
     auto ck_y = [&](int s) { return ck_x(s) + n; };
+    // Where every instance fits a cluster, each runs on its own; else all run packed.
+    // TF's vectors are no smaller than TB's, so one plan serves both passes.
+    auto mats = [&](auto tag) {
+        using T = decltype(tag);
+        const T* csr; const T* csc;
+        values_of<T>(p, &csr, &csc);
+        return BMats<T>{p.csr_ptr.get(), p.csr_idx.get(), csr, lp.col_ptr.get(), lp.row_idx.get(), csc,
+                        p.a.group, p.at.group, p.a.long_len, p.at.long_len};
+    };
+    static_assert(sizeof(TF) >= sizeof(TB), "the plan is made for the forward type");
+    ClusterBatch cl;
+    bool clusters = K > 0;
+    for (int i = 0; i < count; ++i) {
+        cl.least.push_back(least_cluster<TF>(lps[i], p.a.group, p.at.group, 1));
+        clusters = clusters && cl.least[i] > 0;
+    }
+    DeviceBuffer<int> failed;
+    VJ_TRY(failed.alloc(count));
+    VJ_CUDA(cudaMemsetAsync(failed.get(), 0, sizeof(int) * count, st));
+    if (clusters) {
+        VJ_TRY(plan_clusters(lps, count, std::vector<int>(count, 1), 0, mats(TF{}), d_roff, d_coff, cl,
+                             [](const ClusterClass& q) {
+                                 cudaError_t e = prepare_clusters(forward_kernel<TF>(q.threads), q.ctas, q.threads, q.smem);
+                                 return e != cudaSuccess ? e : prepare_clusters(backward_kernel<TB>(q.threads), q.ctas, q.threads, q.smem);
+                             }, st));
+        clusters = static_cast<int>(cl.insts.size()) == count;
+        // At most kAtOnce clusters a stream: the GPU holds 15 clusters of 8 CTAs, and 32 of them in one
+        // launch after another would take three rounds each, the last one nearly empty; launches
+        // of several streams fill each other's rounds.
+        constexpr int kAtOnce = 4;
+        std::vector<ClusterClass> parts;
+        for (const ClusterClass& q : cl.classes) {
+            const int cut = std::max(kAtOnce, (q.clusters + 15) / 16);
+            for (int f = 0; f < q.clusters; f += cut) {
+                parts.push_back(q);
+                parts.back().first = q.first + f;
+                parts.back().clusters = std::min(cut, q.clusters - f);
+            }
+        }
+        cl.classes = parts;
+    }
+    DeviceBuffer<double> loss, x_out, g_c, g_rl, g_ru;
+    ClusterStreams side;   // after the buffers its kernels use
+    if (clusters) VJ_TRY(side.create(cl.classes.size()));
+    auto forward_cluster = [&](const ClusterClass& q, int steps, TF* ckpt, uint8_t* pm, uint8_t* dm, cudaStream_t s) -> vajra_status {
+        const FwdVectors<TF> F{U.c.get(), U.cl.get(), U.cu.get(), U.rl.get(), U.ru.get(), U.x.get(), U.y.get(), step, n, m, ckpt, C, pm, dm};
+        VJ_CUDA(launch_clusters(forward_kernel<TF>(q.threads), q.clusters, q.ctas, q.threads, q.smem, s, F, mats(TF{}),
+                                cl.d_insts.get() + q.first, d_roff, d_coff, steps, failed.get(), static_cast<uint32_t>(q.smem)));
+        return VAJRA_OK;
+    };
     // forward, with checkpoints
-    for (int s = 0; s < nseg; ++s) {
+    if (clusters) {
+        VJ_TRY(side.fork(st));
+        for (size_t q = 0; q < cl.classes.size(); ++q)
+            VJ_TRY(forward_cluster(cl.classes[q], K, want_grad ? U.ckpt.get() : nullptr, nullptr, nullptr, side.streams[q]));
+        VJ_TRY(side.join(st));
+    }
+    for (int s = 0; s < nseg && !clusters; ++s) {
         const int len = (s + 1) * C <= K ? C : K - s * C;
         if (want_grad) {
             VJ_CUDA(cudaMemcpyAsync(ck_x(s), U.x.get(), sizeof(TF) * n, cudaMemcpyDeviceToDevice, st));
@@ -257,7 +485,6 @@ vajra_status run_unrolled_t(const PackedHost& P, const vajra_unrolled_opts& o, P
         }
         for (int k = 0; k < len; ++k) U.forward_step(nullptr, nullptr, st);
     }
-    DeviceBuffer<double> loss, x_out, g_c, g_rl, g_ru;
     VJ_TRY(loss.alloc(count));
     VJ_TRY(x_out.alloc(n));
     k_adj_loss<TF><<<count, kThreads, 0, st>>>(d_coff, U.x.get(), p.col_scale.get(), d_w.get(), c_orig_dev, x_out.get(),
@@ -274,7 +501,24 @@ vajra_status run_unrolled_t(const PackedHost& P, const vajra_unrolled_opts& o, P
         k_adj_seed<TB><<<grid_for(mx), kThreads, 0, st>>>(m, n, p.col_scale.get(), d_w.get(), c_orig_dev, U.xh.get(),
                                                          U.yh.get(), g_c.get(), g_rl.get(), g_ru.get());
         note_launch(1);
-        for (int s = nseg - 1; s >= 0; --s) {
+        if (clusters) VJ_TRY(side.fork(st));
+        for (int s = nseg - 1; s >= 0 && clusters; --s) {
+            const int len = (s + 1) * C <= K ? C : K - s * C;
+            // every class goes through its segments by itself: the step vectors of an instance are its own
+            for (size_t q = 0; q < cl.classes.size(); ++q) {
+                const ClusterClass& k = cl.classes[q];
+                const cudaStream_t ss = side.streams[q];
+                k_load_checkpoint<TF><<<dim3(8, k.clusters), kThreads, 0, ss>>>(cl.d_insts.get() + k.first, d_roff, d_coff, n, ck_x(s),
+                                                                               U.x.get(), U.y.get());
+                note_launch(1);
+                VJ_TRY(forward_cluster(k, len, nullptr, U.pmask.get(), U.dmask.get(), ss));
+                const BwdVectors<TB> B{U.xh.get(), U.yh.get(), g_c.get(), g_rl.get(), g_ru.get(), step, n, m, U.pmask.get(), U.dmask.get()};
+                VJ_CUDA(launch_clusters(backward_kernel<TB>(k.threads), k.clusters, k.ctas, k.threads, k.smem, ss, B, mats(TB{}),
+                                        cl.d_insts.get() + k.first, d_roff, d_coff, len, failed.get(), static_cast<uint32_t>(k.smem)));
+            }
+        }
+        if (clusters) VJ_TRY(side.join(st));
+        for (int s = nseg - 1; s >= 0 && !clusters; --s) {
             const int len = (s + 1) * C <= K ? C : K - s * C;
             VJ_CUDA(cudaMemcpyAsync(U.x.get(), ck_x(s), sizeof(TF) * n, cudaMemcpyDeviceToDevice, st));
             VJ_CUDA(cudaMemcpyAsync(U.y.get(), ck_y(s), sizeof(TF) * m, cudaMemcpyDeviceToDevice, st));
@@ -294,9 +538,16 @@ vajra_status run_unrolled_t(const PackedHost& P, const vajra_unrolled_opts& o, P
         if (h_gru) VJ_CUDA(cudaMemcpyAsync(h_gru, g_ru.get(), sizeof(double) * m, cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
     }
+    std::vector<int> h_failed(count);
+    VJ_CUDA(cudaMemcpyAsync(h_failed.data(), failed.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
     if (h_loss) VJ_CUDA(cudaMemcpyAsync(h_loss, loss.get(), sizeof(double) * count, cudaMemcpyDeviceToHost, st));
     if (h_x) VJ_CUDA(cudaMemcpyAsync(h_x, x_out.get(), sizeof(double) * n, cudaMemcpyDeviceToHost, st));
     VJ_CUDA(cudaStreamSynchronize(st));
+    for (int i = 0; i < count; ++i)
+        if (h_failed[i]) {
+            set_error("instance %d: its cluster did not complete (%d)", i, h_failed[i]);
+            return h_failed[i] == 2 ? VAJRA_ERR_WAIT_TIMEOUT : VAJRA_ERR_INTERNAL;
+        }
     return VAJRA_OK;
 }
 
@@ -348,12 +599,12 @@ vajra_status run_unrolled(int count, const vajra_lp* lps, const vajra_unrolled_o
     // FP64: FP64 map and reverse pass.  MIXED: the FP64 map (forward, checkpoints and the
     // recomputed active sets), reverse pass in FP32.  FP32: the FP32 map and reverse pass.
     if (o.precision == VAJRA_PREC_FP64)
-        return run_unrolled_t<double, double>(P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
+        return run_unrolled_t<double, double>(lps, d_roff.get(), P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
                                               lp.c.get(), h_loss, h_x, h_gc, h_grl, h_gru, st);
     if (o.precision == VAJRA_PREC_FP32)
-        return run_unrolled_t<float, float>(P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
+        return run_unrolled_t<float, float>(lps, d_roff.get(), P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
                                             lp.c.get(), h_loss, h_x, h_gc, h_grl, h_gru, st);
-    return run_unrolled_t<double, float>(P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
+    return run_unrolled_t<double, float>(lps, d_roff.get(), P, o, p, lp, row_inst.get(), col_inst.get(), d_coff.get(), step.get(), w,
                                          lp.c.get(), h_loss, h_x, h_gc, h_grl, h_gru, st);
 }
 

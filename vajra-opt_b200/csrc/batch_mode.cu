@@ -26,7 +26,7 @@
 #include <cstring>
 #include <vector>
 
-#include "cluster.cuh"
+#include "cluster_batch.cuh"
 #include "halpern_state.cuh"
 #include "solver.cuh"
 
@@ -418,22 +418,6 @@ __global__ void k_bcontrol(const double* __restrict__ part, BControl cp, BatchAr
 }
 
 // ----- small instances on clusters (cluster.cuh) -------------------------------------------
-// The packed matrices as the clusters read them.
-template <typename T>
-struct BMats {
-    const int64_t* a_ptr; const int32_t* a_idx; const T* a_val;
-    const int64_t* at_ptr; const int32_t* at_idx; const T* at_val;
-    int group_a, group_at;
-    int64_t long_a, long_at;
-};
-// Instance `inst` of them, by thread 0.
-template <typename T>
-__device__ __forceinline__ void bmats_of(const BMats<T>& M, const int64_t* roff, const int64_t* coff, int inst, ClMats<T>& out) {
-    const int r0 = static_cast<int>(roff[inst]), c0 = static_cast<int>(coff[inst]);
-    out.a = ClMat<T>{static_cast<int>(roff[inst + 1]) - r0, M.a_ptr + r0, M.a_idx, M.a_val, c0, M.group_a, M.long_a};
-    out.at = ClMat<T>{static_cast<int>(coff[inst + 1]) - c0, M.at_ptr + c0, M.at_idx, M.at_val, r0, M.group_at, M.long_at};
-}
-
 constexpr uint32_t kBMaxes = 1u << 9;
 template <typename T>
 __device__ __noinline__ void cl_bkkt_partials(const ClVectors<T>& P, const BKktVectors& V, int i, double ax, int j, double aty,
@@ -487,7 +471,7 @@ struct BatchClusterControl {
 // Cluster q runs instance insts[q]: chunks until it is done or the budget ends.  128 registers a
 // thread, so that two CTAs of 256 threads share an SM.
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT)
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ BKktVectors V, const __grid_constant__ BMats<T> M,
                 const int* __restrict__ insts, const int64_t* __restrict__ roff, const int64_t* __restrict__ coff,
                 const __grid_constant__ BatchArrays S, const __grid_constant__ BControl cp0, double* part, ClControl* shared,
@@ -506,20 +490,6 @@ k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ 
     BatchClusterControl<T> pol{P, V, S, inst, b, cp, red, part + static_cast<size_t>(cluster) * kClMaxCtas * kBQ};
     cl_run<T, NT>(P, mats, static_cast<int>(roff[inst]), static_cast<int>(coff[inst]), pol, shared + cluster, K, budget, max_chunks,
                   smem_bytes);
-}
-
-// nofit[insts[q]] = 1 where the slices of cluster q do not fit its CTAs.
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT)
-k_cluster_fit(const __grid_constant__ BMats<T> M, const int* __restrict__ insts, const int64_t* __restrict__ roff,
-              const int64_t* __restrict__ coff, int* __restrict__ nofit, uint32_t smem_bytes) {
-    __shared__ ClInfo I;
-    __shared__ ClMats<T> mats;
-    const int inst = insts[blockIdx.x / cl_size()];
-    if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
-    __syncthreads();
-    ClCore<T, T> core;
-    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) nofit[inst] = 1;
 }
 
 // done = 1 for the instances that a path does not run: `on` (null: none) marks those on clusters,
@@ -765,36 +735,9 @@ vajra_status up(DeviceBuffer<T>& d, const std::vector<T>& h, cudaStream_t st) {
     return VAJRA_OK;
 }
 
-// The instances that run on clusters, by cluster size and threads.
-struct ClusterClass {
-    int ctas = 0, threads = 0, first = 0, clusters = 0;   // its part of the instance list
-    size_t smem = 0;
-};
-struct ClusterBatch {
-    std::vector<int> least;              // per instance: CTAs of its smallest cluster, 0: it has none
-    std::vector<int> insts;              // the instances of the present plan, by class, largest first
-    std::vector<ClusterClass> classes;   // widest clusters first
-    DeviceBuffer<int> d_insts, d_on;     // the same list; per instance: runs on a cluster
-};
-
 template <typename T>
 auto batch_kernel(int threads) -> decltype(&k_cluster_batch<T, 256>) {
     return threads == 256 ? &k_cluster_batch<T, 256> : &k_cluster_batch<T, 512>;
-}
-template <typename T>
-auto fit_kernel(int threads) -> decltype(&k_cluster_fit<T, 256>) {
-    return threads == 256 ? &k_cluster_fit<T, 256> : &k_cluster_fit<T, 512>;
-}
-
-// The smallest cluster that holds an instance takes the least of the GPU, since an exchange costs
-// no less with more CTAs: 256 threads on one CTA, else CTAs of 512 with at most 4,096 entries of each
-// matrix.
-template <typename T>
-int least_cluster(const vajra_lp& L, int group_a, int group_at) {
-    auto fits = [&](int c, int t) { return cl_fits(sizeof(T), L.num_rows, L.num_cols, L.nnz, group_a, group_at, c, t); };
-    for (int c = 1; c <= kClMaxCtas; c *= 2)
-        if (fits(c, 512) && (L.nnz <= 4096 * static_cast<int64_t>(c) || c == kClMaxCtas)) return c;
-    return 0;
 }
 
 // Entries of unfinished instances too large for a cluster up to which the others go to clusters.
@@ -804,87 +747,6 @@ int least_cluster(const vajra_lp& L, int group_a, int group_at) {
 // its launches (9 to 20 us) and the small instances finish sooner by themselves (96 LPs of 100 to
 // 2,000 rows: 43.8 -> 30.6 ms).
 constexpr int64_t kClBatchEntries = int64_t(4) << 20;
-
-// Plans the unfinished instances (open[i] != 0) of a launch.  A plan that leaves half of the SMs
-// idle gets clusters of twice the size, as far as their CTAs keep 512 entries.
-template <typename T>
-vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, const BMats<T>& M, const int64_t* roff,
-                           const int64_t* coff, ClusterBatch& out, cudaStream_t st) {
-    DeviceBuffer<int> nofit;
-    VJ_TRY(nofit.alloc(count));
-    VJ_TRY(out.d_insts.alloc(count));
-    VJ_TRY(out.d_on.alloc(count));
-    std::vector<int> ctas(count), threads(count), on(count), h(count);
-    auto fits = [&](int i, int c, int t) {
-        return cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, M.group_a, M.group_at, c, t);
-    };
-    for (bool again = true; again;) {
-        again = false;
-        int64_t outside = 0, sms_used = 0;
-        for (int i = 0; i < count; ++i) if (open[i] && !out.least[i]) outside += lps[i].nnz;
-        for (int i = 0; i < count; ++i) {
-            ctas[i] = open[i] && outside <= kClBatchEntries ? out.least[i] : 0;
-            sms_used += ctas[i];
-        }
-        while (sms_used > 0 && 2 * sms_used <= sm_count()) {
-            int64_t used = 0;
-            for (int i = 0; i < count; ++i) {
-                if (ctas[i] > 0 && ctas[i] < kClMaxCtas && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
-                    ctas[i] *= 2;
-                used += ctas[i];
-            }
-            if (used == sms_used) break;
-            sms_used = used;
-        }
-        for (int i = 0; i < count; ++i)
-            threads[i] = ctas[i] && fits(i, ctas[i], 256) && lps[i].nnz <= 2048 * static_cast<int64_t>(ctas[i]) ? 256 : 512;
-        out.classes.clear();
-        out.insts.clear();
-        for (int c = kClMaxCtas; c >= 1; c /= 2)
-            for (int t : {512, 256}) {
-                ClusterClass k;
-                k.ctas = c;
-                k.threads = t;
-                k.first = static_cast<int>(out.insts.size());
-                size_t most = 0;
-                for (int i = 0; i < count; ++i)
-                    if (ctas[i] == c && threads[i] == t) {
-                        out.insts.push_back(i);
-                        most = std::max(most, cl_smem_bytes(sizeof(T), sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, c, t));
-                    }
-                k.clusters = static_cast<int>(out.insts.size()) - k.first;
-                if (!k.clusters) continue;
-                std::stable_sort(out.insts.begin() + k.first, out.insts.end(), [&](int x, int y) { return lps[x].nnz > lps[y].nnz; });
-                // two CTAs of 256 threads fit an SM when each takes half of its shared memory
-                k.smem = t == 256 && most <= kClSmemCap / 2 - 4096 ? kClSmemCap / 2 - 4096 : kClSmemCap;
-                out.classes.push_back(k);
-            }
-        if (out.insts.empty()) break;
-        // Instances whose uneven rows do not fit after all go to the packed iteration.
-        VJ_CUDA(cudaMemcpyAsync(out.d_insts.get(), out.insts.data(), sizeof(int) * out.insts.size(), cudaMemcpyHostToDevice, st));
-        VJ_CUDA(cudaMemsetAsync(nofit.get(), 0, sizeof(int) * count, st));
-        for (const ClusterClass& k : out.classes) {
-            cudaError_t e = prepare_clusters(batch_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
-            if (e == cudaSuccess) e = prepare_clusters(fit_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
-            if (e != cudaSuccess) {   // no such cluster on this device
-                cudaGetLastError();
-                for (int q = k.first; q < k.first + k.clusters; ++q) out.least[out.insts[q]] = 0;
-                again = true;
-                continue;
-            }
-            VJ_CUDA(launch_clusters(fit_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, st, M, out.d_insts.get() + k.first,
-                                    roff, coff, nofit.get(), static_cast<uint32_t>(k.smem)));
-        }
-        VJ_CUDA(cudaMemcpyAsync(h.data(), nofit.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
-        VJ_CUDA(cudaStreamSynchronize(st));
-        for (int q : out.insts)
-            if (h[q]) { out.least[q] = 0; again = true; }
-    }
-    for (int q : out.insts) on[q] = 1;
-    VJ_CUDA(cudaMemcpyAsync(out.d_on.get(), on.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
-    VJ_CUDA(cudaStreamSynchronize(st));   // host vectors above
-    return VAJRA_OK;
-}
 
 }  // namespace
 
@@ -1089,8 +951,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     bool all_fit = true;
     const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0;   // as for a single LP
     for (int i = 0; i < count; ++i) {
-        clus32.least.push_back(may_cluster && mixed ? least_cluster<float>(lps[i], p.a.group, p.at.group) : 0);
-        clus64.least.push_back(may_cluster ? least_cluster<double>(lps[i], p.a.group, p.at.group) : 0);
+        clus32.least.push_back(may_cluster && mixed ? least_cluster<float>(lps[i], p.a.group, p.at.group, 1) : 0);
+        clus64.least.push_back(may_cluster ? least_cluster<double>(lps[i], p.a.group, p.at.group, 1) : 0);
         all_fit = all_fit && clus64.least[i] > 0;   // FP32 vectors are smaller
     }
     DeviceBuffer<double> cl_part;
@@ -1220,34 +1082,13 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     };
 
     // One launch of the clusters of a pass: every class on a stream of its own, joined into `st`.
-    struct Side {
-        std::vector<cudaStream_t> streams;
-        std::vector<cudaEvent_t> events;
-        cudaEvent_t ready = nullptr;
-        ~Side() {
-            for (auto& e : events) cudaEventDestroy(e);
-            for (auto& s : streams) cudaStreamDestroy(s);
-            if (ready) cudaEventDestroy(ready);
-        }
-    } side;
-    auto want_streams = [&](size_t k) -> vajra_status {
-        if (!side.ready) VJ_CUDA(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
-        while (side.streams.size() < k) {
-            cudaStream_t s = nullptr;
-            cudaEvent_t e = nullptr;
-            VJ_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-            side.streams.push_back(s);
-            VJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            side.events.push_back(e);
-        }
-        return VAJRA_OK;
-    };
+    ClusterStreams side;
     BatchArrays Scl = S;
     Scl.done = done_cl.get();
     auto fork_clusters = [&](auto tag, const ClusterBatch& cl, int64_t iters) -> vajra_status {
         using T = decltype(tag);
         if (cl.insts.empty()) return VAJRA_OK;
-        VJ_TRY(want_streams(cl.classes.size()));
+        VJ_TRY(side.create(cl.classes.size()));
         const PassBuffers& b = sizeof(T) == 4 ? pb32 : pb64;
         const ClVectors<T> P{static_cast<const T*>(b.c), static_cast<const T*>(b.cl), static_cast<const T*>(b.cu),
                              static_cast<const T*>(b.rl), static_cast<const T*>(b.ru), static_cast<T*>(b.x), static_cast<T*>(b.x0),
@@ -1255,20 +1096,14 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                              nullptr, x_last.get(), y_last.get(), p.csr_val.get(), p.csc_val.get()};
         BControl c2 = bc;
         c2.pass32 = sizeof(T) == 4 ? 1 : 0;
-        VJ_CUDA(cudaEventRecord(side.ready, st));
+        VJ_TRY(side.fork(st));
         for (size_t q = 0; q < cl.classes.size(); ++q) {
             const ClusterClass& k = cl.classes[q];
-            VJ_CUDA(cudaStreamWaitEvent(side.streams[q], side.ready, 0));
             VJ_CUDA(launch_clusters(batch_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, side.streams[q], P, kv,
                                     mats(tag), cl.d_insts.get() + k.first, d_roff.get(), d_coff.get(), Scl, c2,
                                     cl_part.get() + static_cast<size_t>(k.first) * kClMaxCtas * kBQ, cl_shared.get() + k.first, K,
                                     static_cast<long long>(iters), static_cast<int>((iters + K - 1) / K), static_cast<uint32_t>(k.smem)));
-            VJ_CUDA(cudaEventRecord(side.events[q], side.streams[q]));
         }
-        return VAJRA_OK;
-    };
-    auto join_clusters = [&](const ClusterBatch& cl) -> vajra_status {
-        for (size_t q = 0; q < cl.classes.size(); ++q) VJ_CUDA(cudaStreamWaitEvent(st, side.events[q], 0));
         return VAJRA_OK;
     };
 
@@ -1295,7 +1130,10 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
             VJ_CUDA(cudaMemcpyAsync(status.data(), S.status, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
             VJ_CUDA(cudaStreamSynchronize(st));
             for (int i = 0; i < count; ++i) open[i] = status[i] == 0 ? 1 : 0;
-            VJ_TRY(plan_clusters(lps, count, open, mats(tag), d_roff.get(), d_coff.get(), cl, st));
+            VJ_TRY(plan_clusters(lps, count, open, kClBatchEntries, mats(tag), d_roff.get(), d_coff.get(), cl,
+                                 [](const ClusterClass& q) {
+                                     return prepare_clusters(batch_kernel<T>(q.threads), q.ctas, q.threads, q.smem);
+                                 }, st));
             bool general = false;
             for (int i = 0, q = 0; i < count; ++i) q += open[i], general = general || q > static_cast<int>(cl.insts.size());
             const unsigned cg = (count + 127) / 128;
@@ -1350,7 +1188,7 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                 chunk(tag, static_cast<int>(remaining), cudaGraphConditionalHandle{}, 0);
                 VJ_LAUNCH_CHECK();
             }
-            VJ_TRY(join_clusters(cl));
+            if (!cl.insts.empty()) VJ_TRY(side.join(st));
             k_btotals<<<1, 1024, 0, st>>>(count, S.done, done_cl.get(), S.total, cl_shared.get(), static_cast<int>(cl.insts.size()), counters.get());
             VJ_LAUNCH_CHECK();
             note_launch(1);

@@ -92,13 +92,6 @@ __host__ __device__ inline int cl_bound(int rows, const int64_t* ptr, int r, int
     }
     return 4 * lo < rows ? 4 * lo : rows;
 }
-// No slice has more rows than this (its weight is at most a part plus the last four rows').
-inline int64_t cl_slice_rows(int64_t rows, int64_t nnz, int parts) {
-    if (parts == 1) return rows;
-    const int64_t b = (nnz + kClRowWeight * rows) / (static_cast<int64_t>(kClRowWeight) * parts) + 8;
-    return b < rows ? b : rows;
-}
-
 inline int64_t pad4(int64_t v) { return (v + 3) / 4 * 4; }
 
 // Shared memory of a CTA: the two full vectors, the larger scratch of dealing a slice, and both
@@ -109,12 +102,14 @@ inline size_t cl_smem_bytes(size_t t, size_t value, int64_t m, int64_t n, int64_
     return t * (pad4(n + 1) + pad4(m + 1)) + 2 * share * (value + 4) + 8 * threads + 24 * kClMaxLong + 1024;
 }
 
-// Whether an LP can go to a cluster of `ctas` CTAs: indices of 16 bits, lane-group row sums, at most
-// `threads` rows and columns and kClMaxChains chains a thread in every CTA (from equal shares; a
-// CTA that gets more says so when it deals its slices), and the entries in shared memory.
+// Whether an LP should fit a cluster of `ctas` CTAs: indices of 16 bits, lane-group row sums, at
+// most `threads` rows and columns and kClMaxChains chains a thread in every CTA, and the entries in
+// shared memory.  From equal shares and a tenth: a CTA that gets more says so when it deals its
+// slices.
 inline bool cl_fits(size_t t, int64_t m, int64_t n, int64_t nnz, int group_a, int group_at, int ctas, int threads) {
     if (group_a < 1 || group_a > 32 || group_at < 1 || group_at > 32 || m >= 65535 || n >= 65535) return false;
-    if (std::max(cl_slice_rows(m, nnz, ctas), cl_slice_rows(n, nnz, ctas)) > threads) return false;
+    const int64_t most = std::max(m, n);
+    if (ctas == 1 ? most > threads : (most + most / 10) / ctas + 8 > threads) return false;
     if (std::max(m / ctas * group_a, n / ctas * group_at) / threads >= kClMaxChains) return false;
     return cl_smem_bytes(t, t, m, n, nnz, ctas, threads) <= kClSmemCap;
 }

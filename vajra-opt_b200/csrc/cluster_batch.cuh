@@ -1,0 +1,193 @@
+// Many LPs packed block-diagonally, each on a thread-block cluster of its own (cluster.cuh): which
+// instances go to clusters of which size.
+#pragma once
+
+#include <algorithm>
+#include <vector>
+
+#include "cluster.cuh"
+
+namespace vajra {
+namespace {
+
+// The packed matrices as the clusters read them.
+template <typename T>
+struct BMats {
+    const int64_t* a_ptr; const int32_t* a_idx; const T* a_val;
+    const int64_t* at_ptr; const int32_t* at_idx; const T* at_val;
+    int group_a, group_at;
+    int64_t long_a, long_at;
+};
+// Instance `inst` of them, by thread 0.
+template <typename T>
+__device__ __forceinline__ void bmats_of(const BMats<T>& M, const int64_t* roff, const int64_t* coff, int inst, ClMats<T>& out) {
+    const int r0 = static_cast<int>(roff[inst]), c0 = static_cast<int>(coff[inst]);
+    out.a = ClMat<T>{static_cast<int>(roff[inst + 1]) - r0, M.a_ptr + r0, M.a_idx, M.a_val, c0, M.group_a, M.long_a};
+    out.at = ClMat<T>{static_cast<int>(coff[inst + 1]) - c0, M.at_ptr + c0, M.at_idx, M.at_val, r0, M.group_at, M.long_at};
+}
+
+// nofit[insts[q]] = 1 where the slices of cluster q do not fit its CTAs.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+k_cluster_fit(const __grid_constant__ BMats<T> M, const int* __restrict__ insts, const int64_t* __restrict__ roff,
+              const int64_t* __restrict__ coff, int* __restrict__ nofit, uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ ClMats<T> mats;
+    const int inst = insts[blockIdx.x / cl_size()];
+    if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
+    __syncthreads();
+    ClCore<T, T> core;
+    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) nofit[inst] = 1;
+}
+
+// The instances that run on clusters, by cluster size and threads.
+struct ClusterClass {
+    int ctas = 0, threads = 0, first = 0, clusters = 0;   // its part of the instance list
+    size_t smem = 0;
+};
+struct ClusterBatch {
+    std::vector<int> least;              // per instance: CTAs of its smallest cluster, 0: it has none
+    std::vector<int> insts;              // the instances of the present plan, by class, largest first
+    std::vector<ClusterClass> classes;   // widest clusters first
+    DeviceBuffer<int> d_insts, d_on;     // the same list; per instance: runs on a cluster
+};
+
+// A stream for every class of a launch, forked from and joined into the caller's.
+struct ClusterStreams {
+    std::vector<cudaStream_t> streams;
+    std::vector<cudaEvent_t> events;
+    cudaEvent_t ready = nullptr;
+    size_t used = 0;
+    ~ClusterStreams() {   // (a failed call may leave work on them; buffers declared before outlive it)
+        for (auto& s : streams) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
+        for (auto& e : events) cudaEventDestroy(e);
+        if (ready) cudaEventDestroy(ready);
+    }
+    vajra_status create(size_t k) {
+        used = k;
+        if (!ready) VJ_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        while (streams.size() < k) {
+            cudaStream_t s = nullptr;
+            cudaEvent_t e = nullptr;
+            VJ_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            streams.push_back(s);
+            VJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            events.push_back(e);
+        }
+        return VAJRA_OK;
+    }
+    vajra_status fork(cudaStream_t st) {
+        VJ_CUDA(cudaEventRecord(ready, st));
+        for (size_t q = 0; q < used; ++q) VJ_CUDA(cudaStreamWaitEvent(streams[q], ready, 0));
+        return VAJRA_OK;
+    }
+    vajra_status join(cudaStream_t st) {
+        for (size_t q = 0; q < used; ++q) {
+            VJ_CUDA(cudaEventRecord(events[q], streams[q]));
+            VJ_CUDA(cudaStreamWaitEvent(st, events[q], 0));
+        }
+        return VAJRA_OK;
+    }
+};
+
+template <typename T>
+auto fit_kernel(int threads) -> decltype(&k_cluster_fit<T, 256>) {
+    return threads == 256 ? &k_cluster_fit<T, 256> : &k_cluster_fit<T, 512>;
+}
+
+// The smallest cluster that holds an instance takes the least of the GPU, since an exchange costs
+// no less with more CTAs: 256 threads on one CTA, else CTAs of 512 with at most 4,096 entries of each
+// matrix.  `from`: CTAs it has at least.
+template <typename T>
+int least_cluster(const vajra_lp& L, int group_a, int group_at, int from) {
+    auto fits = [&](int c, int t) { return cl_fits(sizeof(T), L.num_rows, L.num_cols, L.nnz, group_a, group_at, c, t); };
+    for (int c = from; c <= kClMaxCtas; c *= 2)
+        if (fits(c, 512) && (L.nnz <= 4096 * static_cast<int64_t>(c) || c == kClMaxCtas)) return c;
+    return 0;
+}
+
+// Plans the instances with open[i] != 0 for a launch, unless those that no cluster holds have more
+// than `most_outside` entries.  A plan that leaves half of the SMs idle gets clusters of twice the
+// size, as far as their CTAs keep 512 entries.  `prepare`: what a class's launch needs (an error:
+// there is no such cluster on this device).
+template <typename T, class Prepare>
+vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, int64_t most_outside, const BMats<T>& M,
+                           const int64_t* roff, const int64_t* coff, ClusterBatch& out, Prepare prepare, cudaStream_t st) {
+    DeviceBuffer<int> nofit;
+    VJ_TRY(nofit.alloc(count));
+    VJ_TRY(out.d_insts.alloc(count));
+    VJ_TRY(out.d_on.alloc(count));
+    std::vector<int> ctas(count), threads(count), on(count), h(count);
+    auto fits = [&](int i, int c, int t) {
+        return cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, M.group_a, M.group_at, c, t);
+    };
+    for (bool again = true; again;) {
+        again = false;
+        int64_t outside = 0, sms_used = 0;
+        for (int i = 0; i < count; ++i) if (open[i] && !out.least[i]) outside += lps[i].nnz;
+        for (int i = 0; i < count; ++i) {
+            ctas[i] = open[i] && outside <= most_outside ? out.least[i] : 0;
+            sms_used += ctas[i];
+        }
+        while (sms_used > 0 && 2 * sms_used <= sm_count()) {
+            int64_t used = 0;
+            for (int i = 0; i < count; ++i) {
+                if (ctas[i] > 0 && ctas[i] < kClMaxCtas && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
+                    ctas[i] *= 2;
+                used += ctas[i];
+            }
+            if (used == sms_used) break;
+            sms_used = used;
+        }
+        for (int i = 0; i < count; ++i)
+            threads[i] = ctas[i] && fits(i, ctas[i], 256) && lps[i].nnz <= 2048 * static_cast<int64_t>(ctas[i]) ? 256 : 512;
+        out.classes.clear();
+        out.insts.clear();
+        for (int c = kClMaxCtas; c >= 1; c /= 2)
+            for (int t : {512, 256}) {
+                ClusterClass k;
+                k.ctas = c;
+                k.threads = t;
+                k.first = static_cast<int>(out.insts.size());
+                size_t most = 0;
+                for (int i = 0; i < count; ++i)
+                    if (ctas[i] == c && threads[i] == t) {
+                        out.insts.push_back(i);
+                        most = std::max(most, cl_smem_bytes(sizeof(T), sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, c, t));
+                    }
+                k.clusters = static_cast<int>(out.insts.size()) - k.first;
+                if (!k.clusters) continue;
+                std::stable_sort(out.insts.begin() + k.first, out.insts.end(), [&](int x, int y) { return lps[x].nnz > lps[y].nnz; });
+                // two CTAs of 256 threads fit an SM when each takes half of its shared memory
+                k.smem = t == 256 && most <= kClSmemCap / 2 - 4096 ? kClSmemCap / 2 - 4096 : kClSmemCap;
+                out.classes.push_back(k);
+            }
+        if (out.insts.empty()) break;
+        // Instances whose uneven rows do not fit after all get a wider cluster, at last none.
+        VJ_CUDA(cudaMemcpyAsync(out.d_insts.get(), out.insts.data(), sizeof(int) * out.insts.size(), cudaMemcpyHostToDevice, st));
+        VJ_CUDA(cudaMemsetAsync(nofit.get(), 0, sizeof(int) * count, st));
+        for (const ClusterClass& k : out.classes) {
+            cudaError_t e = prepare(k);
+            if (e == cudaSuccess) e = prepare_clusters(fit_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
+            if (e != cudaSuccess) {   // no such cluster on this device
+                cudaGetLastError();
+                for (int q = k.first; q < k.first + k.clusters; ++q) out.least[out.insts[q]] = 0;
+                again = true;
+                continue;
+            }
+            VJ_CUDA(launch_clusters(fit_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, st, M, out.d_insts.get() + k.first,
+                                    roff, coff, nofit.get(), static_cast<uint32_t>(k.smem)));
+        }
+        VJ_CUDA(cudaMemcpyAsync(h.data(), nofit.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
+        VJ_CUDA(cudaStreamSynchronize(st));
+        for (int q : out.insts)
+            if (h[q]) { out.least[q] = least_cluster<T>(lps[q], M.group_a, M.group_at, 2 * ctas[q]); again = true; }
+    }
+    for (int q : out.insts) on[q] = 1;
+    VJ_CUDA(cudaMemcpyAsync(out.d_on.get(), on.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
+    VJ_CUDA(cudaStreamSynchronize(st));   // host vectors above
+    return VAJRA_OK;
+}
+
+}  // namespace
+}  // namespace vajra

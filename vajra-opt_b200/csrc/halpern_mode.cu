@@ -624,6 +624,61 @@ k_cluster_halpern(const __grid_constant__ ClVectors<T> P, const __grid_constant_
     cl_run<T, NT>(P, M, 0, 0, pol, shared, K, budget, max_chunks, smem_bytes);
 }
 
+// The power iteration of spectral_norm_fast (setup.cu) on one cluster: sst->spectral_norm after at
+// most max_iter rounds.  The set-up's loop launches five kernels a round, 1.9 ms of a small LP's
+// 2.6 ms of set-up; here a round is two row sums, two exchanges and a reduction.  `part`: 16 values.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_cluster_norm(const __grid_constant__ ClMats<double> M, int max_iter, double tol, SetupState* sst, double* part, ClControl* shared,
+               uint32_t smem_bytes) {
+    __shared__ ClInfo I;
+    __shared__ double red[kClWarps];
+    __shared__ double sum;
+    const int tid = threadIdx.x;
+    ClCore<double, double> core;
+    if (!core.begin(M.a, M.at, smem_bytes, I) && tid == 0) shared->no_fit = 1;
+    for (int j = tid; j < I.n; j += NT) core.xb()[j] = 1.0 / sqrt(static_cast<double>(I.n));
+    cl_barrier();
+    if (*static_cast<volatile int*>(&shared->no_fit)) return;   // the host takes the set-up's loop
+    const int jl = core.my_col(I), il = core.my_row(I);
+    double lambda = 1.0, prev = 0.0, norm = 0.0;
+    bool done = false;   // uniform over the cluster: every CTA adds the same partials in the same order
+#pragma unroll 1
+    for (int it = 0; it < max_iter && !done; ++it) {
+        const double w = core.row_sum(M.a, I);
+        if (il >= 0) core.yf[il] = w;
+        core.exchange_y(I);
+        const double u = core.col_sum(M.at, I);
+        double v[1] = {jl >= 0 ? u * u : 0.0};
+        cl_reduce<1, 0u>(v, red, part + core.rank);
+        cl_barrier();
+        if (tid == 0) {
+            double t = 0.0;
+            for (uint32_t r = 0; r < core.size; ++r) t += __ldcg(part + r);
+            sum = t;
+        }
+        __syncthreads();
+        norm = sqrt(sum);
+        if (norm < 1e-15 || isnan(norm) || isinf(norm)) {
+            norm = lambda > 1e-6 ? sqrt(lambda) : 1e-3;
+            if (core.rank == 0 && tid == 0) sst->spectral_norm = norm;
+            cl_barrier();
+            return;
+        }
+        lambda = norm;
+        done = it > 0 && fabs(norm - prev) <= tol * norm;
+        prev = norm;
+        if (jl >= 0) core.xb()[jl] = u / norm;
+        core.exchange_x(I);
+    }
+    if (core.dead) shared->wait_error = 1;
+    if (core.rank == 0 && tid == 0) {
+        const double s = sqrt(lambda);
+        sst->spectral_norm = s > 1e-12 ? s : 1e-6;
+    }
+    cl_barrier();   // no CTA ends while a peer may still send to it
+}
+
 // How an LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
 struct ClusterPlan { int ctas = 0, threads = 0; size_t smem = 0; };
 
@@ -639,13 +694,16 @@ auto cluster_kernel(int threads) -> decltype(&k_cluster_halpern<T, 256>) {
 // 1 CTA 1.2 / 1.3, on 4 1.7 / 1.7; 301 x 807 on 4 CTAs 1.9 / 2.1, on 8 1.9 / 2.1; 2000 x 5000 on
 // 16 CTAs of 512 threads 3.4 / 4.9; 5000 x 12000 (1,024 threads) 8.4 against 7.2, which is why the
 // line lies at 512.  Every thread forms at most kClMaxChains chains of a row.
+// `from`: CTAs it has at least.
 template <typename T>
-ClusterPlan plan_cluster(const CsrView& a, const CsrView& at, int64_t nnz) {
-    for (int ctas = 1; ctas <= kClMaxCtas; ctas *= 2) {
+ClusterPlan plan_cluster(const CsrView& a, const CsrView& at, int64_t nnz, int from) {
+    for (int ctas = from; ctas <= kClMaxCtas; ctas *= 2) {
         const int threads = cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, 256) ? 256 : 512;
         if (!cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, threads)) continue;
         if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
-        const cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
+        cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
+        if (sizeof(T) == 8 && e == cudaSuccess)
+            e = prepare_clusters(threads == 256 ? &k_cluster_norm<256> : &k_cluster_norm<512>, ctas, threads, kClSmemCap);
         if (e != cudaSuccess) { cudaGetLastError(); continue; }   // no such cluster on this device
         return ClusterPlan{ctas, threads, kClSmemCap};   // all of it: slices may be uneven
     }
@@ -822,6 +880,9 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     // Degree ordering (built once per handle); the result vectors go back to the caller's
     // numbering at the end.  Below ~1M entries the vectors stay in cache anyway.
     constexpr int64_t kOrderMinNnz = int64_t(1) << 20;
+    // Below ~1M entries a solve is launch-bound and the timing runs would cost more than any
+    // shape saves: the set-up heuristic (lanes per row from the mean row length) stays.
+    constexpr int64_t kAutotuneMinNnz = int64_t(1) << 20;
     const bool ordered = o.degree_order > 0 || (o.degree_order == 0 && nnz >= kOrderMinNnz);
     // verbose: host time of each set-up step (the stream drained at each mark)
     auto mark = [&](const char* what) {
@@ -870,11 +931,42 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
         if (mixed) VJ_TRY(prepare_hot_kernels<float>());
         VJ_TRY(prepare_hot_kernels<double>());
     }
-    VJ_TRY(spectral_norm_fast(p, m, n, 100, 1e-5, sst.get(), st));
-    mark("norm estimate");
+    // Small LPs (below ~1M entries, where the shapes are the heuristic's): the norm estimate and, unless
+    // the caller fixed a launch shape, the iterations run on a thread-block cluster.
+    ClusterPlan cl32, cl64;
+    DeviceBuffer<double> cl_part;
+    DeviceBuffer<ClControl> cl_shared;
+    if (nnz < kAutotuneMinNnz) {
+        cl64 = plan_cluster<double>(p.a, p.at, nnz, 1);
+        if (mixed) cl32 = plan_cluster<float>(p.a, p.at, nnz, 1);
+    }
     SetupState hss{};
-    VJ_CUDA(cudaMemcpyAsync(&hss, sst.get(), sizeof(hss), cudaMemcpyDeviceToHost, st));
-    VJ_CUDA(cudaStreamSynchronize(st));
+    bool normed = false;
+    if (cl32.ctas || cl64.ctas) {
+        VJ_TRY(cl_part.alloc(2 * kQ * kClMaxCtas));
+        VJ_TRY(cl_shared.alloc(1));
+    }
+    if (cl64.ctas) {
+        const ClMats<double> M{ClMat<double>{m, p.csr_ptr.get(), p.csr_idx.get(), p.csr_val.get(), 0, p.a.group, p.a.long_len},
+                               ClMat<double>{n, lp.col_ptr.get(), lp.row_idx.get(), p.csc_val.get(), 0, p.at.group, p.at.long_len}};
+        ClControl hc{};
+        VJ_CUDA(cudaMemsetAsync(cl_shared.get(), 0, sizeof(ClControl), st));
+        VJ_CUDA(launch_clusters(cl64.threads == 256 ? &k_cluster_norm<256> : &k_cluster_norm<512>, 1, cl64.ctas, cl64.threads, cl64.smem,
+                                st, M, 100, 1e-5, sst.get(), cl_part.get(), cl_shared.get(), static_cast<uint32_t>(cl64.smem)));
+        VJ_CUDA(cudaMemcpyAsync(&hss, sst.get(), sizeof(hss), cudaMemcpyDeviceToHost, st));
+        VJ_CUDA(cudaMemcpyAsync(&hc, cl_shared.get(), sizeof(hc), cudaMemcpyDeviceToHost, st));
+        VJ_CUDA(cudaStreamSynchronize(st));
+        if (hc.wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
+        if (hc.no_fit) cl64 = plan_cluster<double>(p.a, p.at, nnz, 2 * cl64.ctas);   // uneven rows
+        else normed = true;
+    }
+    if (!normed) {
+        VJ_TRY(spectral_norm_fast(p, m, n, 100, 1e-5, sst.get(), st));
+        VJ_CUDA(cudaMemcpyAsync(&hss, sst.get(), sizeof(hss), cudaMemcpyDeviceToHost, st));
+        VJ_CUDA(cudaStreamSynchronize(st));
+    }
+    mark("norm estimate");
+    if (o.spmv_shape_a != 0 || o.spmv_shape_at != 0) cl32 = cl64 = ClusterPlan{};   // shapes the caller fixed
     const double spectral_norm = hss.spectral_norm;
     if (!(spectral_norm > 1e-12) || !std::isfinite(spectral_norm)) {
         r->status = kStatusNumerical;
@@ -962,9 +1054,6 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     init.gamma_now = gamma;   // the FP32 phase starts with the full step too
     CsrView a64 = p.a, at64 = p.at;
     CsrView a32 = p.a, at32 = p.at;
-    // Below ~1M entries a solve is launch-bound and the timing runs would cost more than any
-    // shape saves: the set-up heuristic (lanes per row from the mean row length) stays.
-    constexpr int64_t kAutotuneMinNnz = int64_t(1) << 20;
     const TuneKey tkey{h->device, m, n, nnz, ordered ? 1 : 0, compact ? 1 : 0};
     if (o.autotune) {   // shapes another handle already tuned for this LP
         std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -1063,20 +1152,6 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     cp.stall_checks = o.mixed_stall_checks < 0 ? 0 : (o.mixed_stall_checks > kHist - 1 ? kHist - 1 : o.mixed_stall_checks);
     const int64_t max_iter = o.iteration_limit;
 
-    // Small LPs: each phase runs on one thread-block cluster, many chunks a launch, unless the
-    // caller fixed a launch shape.
-    const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0 && nnz < kAutotuneMinNnz;
-    ClusterPlan cl32, cl64;
-    DeviceBuffer<double> cl_part;
-    DeviceBuffer<ClControl> cl_shared;
-    if (may_cluster) {
-        if (mixed) cl32 = plan_cluster<float>(a32, at32, nnz);
-        cl64 = plan_cluster<double>(a64, at64, nnz);
-        if (cl32.ctas || cl64.ctas) {
-            VJ_TRY(cl_part.alloc(2 * kQ * kClMaxCtas));
-            VJ_TRY(cl_shared.alloc(1));
-        }
-    }
     auto cluster_chunks = [&](auto& ph, const ClusterPlan& plan, int64_t budget, int chunks) -> vajra_status {
         using T = std::decay_t<decltype(*ph.x.get())>;
         const CsrView& ia = ph.phase == 0 ? a32 : a64;
@@ -1115,7 +1190,11 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
             if (hc->wait_error) { set_error("an exchange between the CTAs of a cluster did not complete"); return VAJRA_ERR_WAIT_TIMEOUT; }
             cl_seconds += seconds_since(t_launch);
             cl_chunks += (hs->total - launched + K - 1) / K;
-            if (hc->no_fit) { cl32.ctas = cl64.ctas = 0; continue; }   // uneven rows: the general path
+            if (hc->no_fit) {   // uneven rows: a wider cluster, at last the general path
+                if (cur_phase == 0) cl32 = plan_cluster<float>(a32, at32, nnz, 2 * plan.ctas);
+                else cl64 = plan_cluster<double>(a64, at64, nnz, 2 * plan.ctas);
+                continue;
+            }
             if (hs->total <= launched) return VAJRA_ERR_INTERNAL;   // a launch runs at least one chunk
             launched = hs->total;
         } else {

@@ -439,11 +439,13 @@ struct EpiStoreUnlessDone {
     __device__ void operator()(int row, double s) const { out[row] = s; }
 };
 
-// Sequential: the reference sums u_j^2 in index order.
-__global__ void k_power_step_exact(int n, const double* __restrict__ u, double tol, SetupState* sst) {
+// The reference sums u_j^2 in index order.  One CTA.
+__global__ void __launch_bounds__(1024)
+k_power_step_exact(int n, const double* __restrict__ u, double tol, SetupState* sst) {
     if (sst->power_done) return;
-    double norm_sq = 0.0;
-    for (int j = 0; j < n; ++j) norm_sq = __dadd_rn(norm_sq, __dmul_rn(u[j], u[j]));
+    __shared__ double tile[2 * kSerialTile];
+    const double norm_sq = serial_sum(n, 0.0, tile, [&](int64_t j) { return __dmul_rn(u[j], u[j]); });
+    if (threadIdx.x != 0) return;
     const double norm = __dsqrt_rn(norm_sq);
     const int it = sst->power_iter;
     if (norm < 1e-15 || isnan(norm) || isinf(norm)) {
@@ -495,7 +497,7 @@ vajra_status spectral_norm_exact(const Prepared& p, int m, int n, int max_iter, 
     for (int it = 0; it < max_iter; ++it) {
         launch_spmv_exact<double, true>(p.a, p.csr_val.get(), v.get(), EpiStoreUnlessDone{w.get(), done}, st);
         launch_spmv_exact<double, false>(p.at, p.csc_val.get(), w.get(), EpiStoreUnlessDone{u.get(), done}, st);
-        k_power_step_exact<<<1, 1, 0, st>>>(n, u.get(), tol, sst);
+        k_power_step_exact<<<1, 1024, 0, st>>>(n, u.get(), tol, sst);
         k_power_scale<<<grid_for(n), kThreads, 0, st>>>(n, u.get(), v.get(), sst);
         VJ_LAUNCH_CHECK();
         note_launch(2);

@@ -130,3 +130,17 @@ def test_unrolled_on_clusters_matches_the_packed_map(cuda, prec, every):
                            ("grad_row_upper", m, 2.0 ** -53 if prec == "fp64" else 2.0 ** -24)):
         u, v = a[key], b[key][:size]
         np.testing.assert_allclose(u, v, rtol=0, atol=2 * 30 * 64 * eps * (1.0 + np.abs(v).max()), err_msg=key)
+
+
+@pytest.mark.parametrize("kind", CASES + [(3300, 7400, 3)], ids=str)
+def test_reference_algorithm_on_clusters_equals_the_oracle(cuda, kind):
+    """The in-order row sums of the reference algorithm, bit for bit, at the edges of the slices and
+    of the sums' tiles (1,024 terms)."""
+    from oracle import bindings as B
+    lp = lp_of(kind)
+    kw = dict(iteration_limit=130, check_frequency=50, tolerance=1e-9, gap_tolerance=1e-9)
+    g = V.solve(lp, algorithm=V.ALGO_REFERENCE, **kw)
+    o = B.port_solve(lp, **kw)
+    for k in ("x", "y", "d", "row_value"):
+        np.testing.assert_array_equal(g[k], o[k], err_msg=k)
+    assert g["status"] == o["status"] and g["iterations"] == o["iterations"] and g["objective_value"] == o["objective_value"]

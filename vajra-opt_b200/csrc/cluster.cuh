@@ -327,8 +327,15 @@ __device__ __noinline__ ClTask cl_deal(const ClMat<V>& mat, ClSlice& s, uint32_t
 // `turn` pairs long; finished sums wait in s0, s1, s2 for their partners like the digits of a
 // binary counter.  One form for every number of chains: a form for each, inlined twice, drove the
 // iteration's registers into local memory.
-template <typename T>
+// EXACT: products rounded before they are added (the reference's arithmetic); DROP: an entry whose
+// vector entry is zero adds nothing, whatever its value.
+template <typename T, bool EXACT = false, bool DROP = false>
 __device__ __forceinline__ T cl_chains(const ClTask& t) {
+    auto add = [](T a, T v, T x) -> T {
+        if constexpr (!EXACT) return fma(v, x, a);
+        else if constexpr (DROP) return x == T(0) ? a : rn_add(a, rn_mul(v, x));
+        else return rn_add(a, rn_mul(v, x));
+    };
     constexpr int P = 4;   // pairs taken together: their loads overlap
     const ClArray<ClPair<T>> ep{t.pair};
     T acc = T(0), s0 = T(0), s1 = T(0), s2 = T(0), total = T(0);
@@ -349,8 +356,8 @@ __device__ __forceinline__ T cl_chains(const ClTask& t) {
 #pragma unroll
         for (int p = 0; p < P; ++p)
             if (p == 0 || u + p < t.pairs) {
-                acc = fma(e[p].val0, xx[2 * p], acc);
-                acc = fma(e[p].val1, xx[2 * p + 1], acc);
+                acc = add(acc, e[p].val0, xx[2 * p]);
+                acc = add(acc, e[p].val1, xx[2 * p + 1]);
                 if (--left == 0) {   // a chain is done (the same for all of a warp)
                     left = t.turn;
                     total = acc;
@@ -508,6 +515,10 @@ struct ClCore {
         if (s.n_long) t = cl_long_sum<T, V>(mat, s, task.row, vec, t);
         return t;
     }
+    // In the reference's arithmetic (group 1: a thread a row, no long rows); a padding entry of the
+    // transpose adds the product of zero and a zero.
+    __device__ __forceinline__ T col_sum_exact() { return cl_chains<T, true, false>(tc); }
+    __device__ __forceinline__ T row_sum_exact() { return cl_chains<T, true, true>(tr); }
     __device__ __forceinline__ T col_sum(const ClMat<V>& at, const ClInfo& I) { return sum(tc, tpr_c, at, I.cols, yf); }
     __device__ __forceinline__ T row_sum(const ClMat<V>& a, const ClInfo& I) { return sum(tr, tpr_r, a, I.rows, xb()); }
 };

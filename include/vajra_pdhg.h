@@ -130,7 +130,9 @@ typedef struct vajra_opts {
                                    -2 row-block kernel with two load groups per thread,
                                    -3 sliced ELL (degree-ordered LPs; else the row-block
                                    kernel), -4 sliced ELL with the first vector entries in
-                                   shared memory, 1..32 lanes per row (1, 2, 4, 8, 16, 32)   */
+                                   shared memory, 1..32 lanes per row (1, 2, 4, 8, 16, 32).
+                                   The batched solver: 0 as above, -3 sliced ELL over windows
+                                   of 256 rows, other values keep it off the clusters         */
     int32_t spmv_shape_at;      /* the same for the A^T y SpMV                           */
     double mixed_reflection;    /* MIXED: reflection coefficient of the FP32 phase once its
                                    relative KKT is within 10x of mixed_switch_tolerance (0.8);
@@ -207,7 +209,8 @@ typedef struct vajra_result {
     int32_t spmv_group_a;       /* SpMV shape chosen for A x: 1..32 lanes per row, 0 the
                                    shared-memory row-block kernel, 64 the same with two load
                                    groups per thread, 128 sliced ELL, 129 sliced ELL with the
-                                   hot vector prefix in shared memory, -1 the exact in-order
+                                   hot vector prefix in shared memory, 130 sliced ELL over
+                                   windows of 256 rows (batches), -1 the exact in-order
                                    kernel of VAJRA_ALGO_REFERENCE                            */
     int32_t spmv_group_at;      /* same for A^T y                                           */
     /* Live kernel timing (HALPERN): CUDA-event durations of the fused iteration kernels,

@@ -184,6 +184,13 @@ struct EpiStorePlain {
     __device__ void operator()(int r, double s) const { out[r] = s; }
 };
 
+// One SpMV in the view's shape; sliced ELL over windows reads its own copy of the values.
+template <typename VV, typename VX, typename Acc, class Epi>
+void launch_packed(const CsrView& v, const VV* csr_val, const VV* win_val, const VX* x, Epi epi, cudaStream_t st) {
+    if (v.group == kSellWin) launch_sellw<VV, VX, Acc>(v, csr_val, win_val, x, epi, st);
+    else launch_spmv_t<VV, VX, Acc>(v, csr_val, x, epi, st);
+}
+
 // Blocks of one launch shape that hold at least one row of an unfinished instance (order
 // irrelevant: every row's result is independent of which CTA computes it).
 __global__ void k_active_blocks(int nblocks, int rows, int rows_per_block, const int32_t* __restrict__ block_rows,
@@ -219,7 +226,7 @@ struct BlockList {
             block_rows = v.block_rows;
             cap = sms * 4;
         } else {
-            int g = v.group;
+            int g = v.group == kSellWin ? 1 : v.group;   // windows of kThreads rows
             if (g != 1 && g != 2 && g != 4 && g != 8 && g != 16) g = g == 0 ? 8 : 32;   // launch_spmv_t's dispatch
             rows_per_block = kThreads / g;
             nblocks = vec_block_count(v.rows, g);
@@ -880,8 +887,21 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     S.hist_n = di.get() + 4 * count;
     VJ_CUDA(cudaMemsetAsync(di.get(), 0, sizeof(int) * 5 * count, st));   // done = 0 for the power iteration
 
+    // A batch that the packed iteration streams (2^20 entries or more): copies over windows, one
+    // more launch shape for the autotuner and the power iteration's SpMVs.
+    const bool mixed = o.precision == VAJRA_PREC_MIXED;
+    if (mixed) VJ_TRY(make_f32_values(p, NNZ, st));
+    WindowData win_a, win_at;
+    const bool fixed_windows = o.spmv_shape_a == -3 || o.spmv_shape_at == -3;   // the caller's choice, for both
+    if (fixed_windows || (o.autotune && NNZ >= (int64_t(1) << 20))) {
+        VJ_TRY(build_windows(p.a, p.csr_val.get(), mixed ? p.csr_val32.get() : nullptr, win_a, st));
+        VJ_TRY(build_windows(p.at, p.csc_val.get(), mixed ? p.csc_val32.get() : nullptr, win_at, st));
+    }
     // batched power iteration (fixed 60 rounds)
     {
+        CsrView pa = p.a, pat = p.at;
+        if (pa.win_off) pa.group = kSellWin;
+        if (pat.win_off) pat.group = kSellWin;
         DeviceBuffer<double> v, w, u;
         VJ_TRY(v.alloc(n));
         VJ_TRY(w.alloc(m));
@@ -889,8 +909,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         k_bpower_init<<<grid_for(n), kThreads, 0, st>>>(n, col_inst.get(), d_coff.get(), v.get());
         note_launch(1);
         for (int it = 0; it < 60; ++it) {
-            launch_spmv_t<double, double, double>(p.a, p.csr_val.get(), v.get(), EpiStorePlain{w.get()}, st);
-            launch_spmv_t<double, double, double>(p.at, p.csc_val.get(), w.get(), EpiStorePlain{u.get()}, st);
+            launch_packed<double, double, double>(pa, p.csr_val.get(), win_a.val64.get(), v.get(), EpiStorePlain{w.get()}, st);
+            launch_packed<double, double, double>(pat, p.csc_val.get(), win_at.val64.get(), w.get(), EpiStorePlain{u.get()}, st);
             k_bpower<<<count, kThreads, 0, st>>>(d_coff.get(), u.get(), v.get(), S);
             note_launch(1);
         }
@@ -916,10 +936,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     VJ_LAUNCH_CHECK();
     // Mixed precision: an FP32 pass (FP32 values, iterates and sums, FP64 checks) runs first;
     // each instance finishes there or hands over to the FP64 pass.
-    const bool mixed = o.precision == VAJRA_PREC_MIXED;
     DeviceBuffer<float> x32, x0_32, xb32, xc32, y32, y0_32, yc32, c32, cl32, cu32, rl32, ru32;
     if (mixed) {
-        VJ_TRY(make_f32_values(p, NNZ, st));
         for (auto* b : {&x32, &x0_32, &xb32, &xc32, &c32, &cl32, &cu32}) VJ_TRY(b->alloc(n));
         for (auto* b : {&y32, &y0_32, &yc32, &rl32, &ru32}) VJ_TRY(b->alloc(m));
         const unsigned gn = grid_for(n, kThreads, 148 * 32), gm = grid_for(m, kThreads, 148 * 32);
@@ -965,7 +983,9 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
 
     // autotune the packed SpMVs (store epilogue, no skipping)
     CsrView a = p.a, at = p.at;
-    if (o.autotune && !all_fit) {
+    if (fixed_windows) {
+        a.group = at.group = kSellWin;
+    } else if (o.autotune && !all_fit) {
         cudaEvent_t e0, e1;
         VJ_CUDA(cudaEventCreate(&e0));
         VJ_CUDA(cudaEventCreate(&e1));
@@ -975,12 +995,14 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
             const double* val = (v == &a) ? p.csr_val.get() : p.csc_val.get();
             float best = 1e30f;
             int best_g = v->group;
-            for (int g : {0, kRowblock2, 1, 2, 4, 8, 16, 32}) {
+            const double* win = (v == &a) ? win_a.val64.get() : win_at.val64.get();
+            for (int g : {0, kRowblock2, 1, 2, 4, 8, 16, 32, kSellWin}) {
+                if (g == kSellWin && !v->win_off) continue;
                 CsrView t = *v;
                 t.group = g;
-                launch_spmv_t<double, double, double>(t, val, xin, EpiStorePlain{out}, st);
+                launch_packed<double, double, double>(t, val, win, xin, EpiStorePlain{out}, st);
                 VJ_CUDA(cudaEventRecord(e0, st));
-                for (int r = 0; r < 3; ++r) launch_spmv_t<double, double, double>(t, val, xin, EpiStorePlain{out}, st);
+                for (int r = 0; r < 3; ++r) launch_packed<double, double, double>(t, val, win, xin, EpiStorePlain{out}, st);
                 VJ_CUDA(cudaEventRecord(e1, st));
                 VJ_CUDA(cudaEventSynchronize(e1));
                 float ms = 0.f;
@@ -1052,6 +1074,9 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         const PassBuffers& b = sizeof(T) == 4 ? pb32 : pb64;
         const T* csr = static_cast<const T*>(b.csr);
         const T* csc = static_cast<const T*>(b.csc);
+        const T* wcsr; const T* wcsc;   // the copies over windows
+        if constexpr (sizeof(T) == 4) { wcsr = win_a.val32.get(); wcsc = win_at.val32.get(); }
+        else { wcsr = win_a.val64.get(); wcsc = win_at.val64.get(); }
         T* xv = static_cast<T*>(b.x); T* x0v = static_cast<T*>(b.x0); T* xbv = static_cast<T*>(b.xb);
         T* xcv = static_cast<T*>(b.xc); T* yv = static_cast<T*>(b.y); T* y0v = static_cast<T*>(b.y0);
         T* ycv = static_cast<T*>(b.yc);
@@ -1059,16 +1084,16 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
         list_at.rebuild(S.done, st);
         for (int kk = 0; kk < len; ++kk) {
             const int wc = kk == len - 1 ? 1 : 0;
-            launch_spmv_t<T, T, T>(at_it, csc, yv,
+            launch_packed<T, T, T>(at_it, csc, wcsc, yv,
                                    EpiBPrimal<T>{static_cast<const T*>(b.c), static_cast<const T*>(b.cl),
                                                  static_cast<const T*>(b.cu), x0v, xv, xbv, xcv, col_inst.get(), S,
                                                  kk, wc}, st);
-            launch_spmv_t<T, T, T>(a_it, csr, xbv,
+            launch_packed<T, T, T>(a_it, csr, wcsr, xbv,
                                    EpiBDual<T>{static_cast<const T*>(b.rl), static_cast<const T*>(b.ru), y0v, yv, ycv,
                                                row_inst.get(), S, kk, wc}, st);
         }
-        launch_spmv_t<double, T, double>(a_it, p.csr_val.get(), xcv, EpiBStore{ax.get(), row_inst.get(), S.done}, st);
-        launch_spmv_t<double, T, double>(at_it, p.csc_val.get(), ycv, EpiBStore{aty.get(), col_inst.get(), S.done}, st);
+        launch_packed<double, T, double>(a_it, p.csr_val.get(), win_a.val64.get(), xcv, EpiBStore{ax.get(), row_inst.get(), S.done}, st);
+        launch_packed<double, T, double>(at_it, p.csc_val.get(), win_at.val64.get(), ycv, EpiBStore{aty.get(), col_inst.get(), S.done}, st);
         k_bkkt<T><<<count, kThreads, 0, st>>>(d_roff.get(), d_coff.get(), ax.get(), aty.get(), xcv, ycv, kv, x_last.get(),
                                               y_last.get(), part.get(), S);
         BControl c2 = bc;
@@ -1238,8 +1263,11 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     k_bpost<<<grid_for(mx), kThreads, 0, st>>>(m, n, col_inst.get(), d_sense.get(), xc.get(), yc.get(),
                                                p.col_scale.get(), p.row_scale.get(), p.scaled ? 1 : 0, x_out.get(),
                                                y_out.get());
-    launch_spmv_t<double, double, double>(a, p.csr_val_orig.get(), x_out.get(), EpiStorePlain{row_value.get()}, st);
-    launch_spmv_t<double, double, double>(at, lp.values.get(), y_out.get(), EpiStorePlain{col_dual.get()}, st);
+    // the original values have no copy over windows
+    launch_spmv_t<double, double, double>(a.group == kSellWin ? p.a : a, p.csr_val_orig.get(), x_out.get(),
+                                          EpiStorePlain{row_value.get()}, st);
+    launch_spmv_t<double, double, double>(at.group == kSellWin ? p.at : at, lp.values.get(), y_out.get(),
+                                          EpiStorePlain{col_dual.get()}, st);
     k_breduced<<<grid_for(n), kThreads, 0, st>>>(n, col_inst.get(), d_sense.get(), lp.c.get(), col_dual.get());
     k_bobjective<<<count, kThreads, 0, st>>>(d_coff.get(), lp.c.get(), x_out.get(), d_offsets.get(), objs.get());
     note_launch(3);

@@ -38,6 +38,16 @@ struct SellData {
     DeviceBuffer<uint8_t> len;                     // row lengths, kSellLong for listed rows
 };
 
+// Sliced-ELL copy over windows of 256 rows (spmv.cuh, kSellWin).
+struct WindowData {
+    DeviceBuffer<int64_t> off;
+    DeviceBuffer<int32_t> idx;
+    DeviceBuffer<double> val64;
+    DeviceBuffer<float> val32;
+    DeviceBuffer<uint8_t> perm, len;               // by place in the window: the row, its length
+    DeviceBuffer<int32_t> long_rows, vlong_rows;   // rows kept in CSR (row order)
+};
+
 struct Prepared {
     // structure
     DeviceBuffer<int64_t> csr_ptr;
@@ -137,6 +147,9 @@ vajra_status order_by_degree(const DeviceLp& src, DeviceLp& dst, LpOrder& ord, c
 // Sliced-ELL copy (SellData) of `v`: builds `out` from v's CSR-order values (val32 may be
 // null) and sets v's sell_* fields.
 vajra_status build_sell(CsrView& v, const double* val64, const float* val32, SellData& out, cudaStream_t st);
+
+// The copy over windows: builds `out` and sets v's win_* and long-row fields (val32 may be null).
+vajra_status build_windows(CsrView& v, const double* val64, const float* val32, WindowData& out, cudaStream_t st);
 
 // dst[order[k]] = src[k] for k < count: a result vector back in the caller's numbering.
 vajra_status unorder(int count, const int32_t* order, const double* src, double* dst, cudaStream_t st);

@@ -978,6 +978,106 @@ vajra_status build_sell(CsrView& v, const double* val64, const float* val32, Sel
     return VAJRA_OK;
 }
 
+// One CTA per window: the rows' places by descending length (equal lengths in row order), their
+// lengths (kSellLong for listed rows, which come last), and the eight slices' sizes.
+__global__ void __launch_bounds__(kSellWindow)
+k_window_order(int rows, int windows, const int64_t* __restrict__ ptr, uint8_t* __restrict__ perm, uint8_t* __restrict__ len8,
+               int64_t* __restrict__ sizes) {
+    __shared__ int lens[kSellWindow], sorted[kSellWindow];
+    const int tid = threadIdx.x, row = blockIdx.x * kSellWindow + tid;
+    int len = -2;                              // past the end
+    if (row < rows) {
+        const int64_t l = ptr[row + 1] - ptr[row];
+        len = l > kSellWidth ? -1 : static_cast<int>(l);
+    }
+    lens[tid] = len;
+    __syncthreads();
+    int before = 0;
+    for (int q = 0; q < kSellWindow; ++q) before += (lens[q] > len || (lens[q] == len && q < tid)) ? 1 : 0;
+    sorted[before] = len;
+    const int64_t place = static_cast<int64_t>(blockIdx.x) * kSellWindow + before;
+    perm[place] = static_cast<uint8_t>(tid);
+    len8[place] = len == -1 ? kSellLong : (len < 0 ? 0 : static_cast<uint8_t>(len));
+    __syncthreads();
+    if (tid < kSellWindow / 32) {
+        const int most = sorted[32 * tid] > 0 ? sorted[32 * tid] : 0;   // a slice's first row is its longest
+        sizes[blockIdx.x * (kSellWindow / 32) + tid] = 32 * ((most + 1) / 2 * 2);
+    }
+    if (blockIdx.x == static_cast<unsigned>(windows) - 1 && tid == 0) sizes[static_cast<int64_t>(windows) * (kSellWindow / 32)] = 0;
+}
+
+// One thread per place: its row's entries to their slots; the slots behind them are zeros that are
+// never read.
+__global__ void k_window_fill(int rows, int places, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                              const double* __restrict__ v64, const float* __restrict__ v32, const uint8_t* __restrict__ perm,
+                              const uint8_t* __restrict__ len8, const int64_t* __restrict__ off, int32_t* __restrict__ sidx,
+                              double* __restrict__ s64, float* __restrict__ s32) {
+    const int place = blockIdx.x * blockDim.x + threadIdx.x;
+    if (place >= places) return;
+    const int row = place / kSellWindow * kSellWindow + perm[place];
+    const int len = row < rows && len8[place] != kSellLong ? len8[place] : 0;
+    const int64_t b = len > 0 ? ptr[row] : 0, o = off[place >> 5] + 2 * (place & 31);
+    for (int k = 0; k < len; ++k) {
+        const int64_t q = o + 64 * (k >> 1) + (k & 1);
+        sidx[q] = idx[b + k];
+        s64[q] = v64[b + k];
+        if (v32) s32[q] = v32[b + k];
+    }
+    if (len & 1) {   // the second half of an odd row's last pair is loaded, not used
+        const int64_t q = o + 64 * (len >> 1) + 1;
+        sidx[q] = 0;
+        s64[q] = 0.0;
+        if (v32) s32[q] = 0.f;
+    }
+}
+
+vajra_status build_windows(CsrView& v, const double* val64, const float* val32, WindowData& out, cudaStream_t st) {
+    v.win_off = nullptr;
+    if (v.rows <= 0) return VAJRA_OK;
+    const int windows = sell_windows(v.rows), slices = windows * (kSellWindow / 32);
+    {
+        DeviceBuffer<uint8_t> is_long, is_vlong, len;
+        VJ_TRY(is_long.alloc(static_cast<size_t>(v.rows)));
+        VJ_TRY(is_vlong.alloc(static_cast<size_t>(v.rows)));
+        VJ_TRY(len.alloc(static_cast<size_t>(v.rows)));
+        k_sell_classify<<<grid_for(v.rows), kThreads, 0, st>>>(v.rows, v.ptr, is_long.get(), is_vlong.get(), len.get());
+        VJ_LAUNCH_CHECK();
+        note_launch(1);
+        VJ_TRY(select_rows(v.rows, is_long.get(), out.long_rows, &v.sell_n_long, st));
+        VJ_TRY(select_rows(v.rows, is_vlong.get(), out.vlong_rows, &v.sell_n_vlong, st));
+    }
+    VJ_TRY(out.perm.alloc(static_cast<size_t>(windows) * kSellWindow));
+    VJ_TRY(out.len.alloc(static_cast<size_t>(windows) * kSellWindow));
+    VJ_TRY(out.off.alloc(static_cast<size_t>(slices) + 1));
+    DeviceBuffer<int64_t> sizes;
+    VJ_TRY(sizes.alloc(static_cast<size_t>(slices) + 1));
+    k_window_order<<<windows, kSellWindow, 0, st>>>(v.rows, windows, v.ptr, out.perm.get(), out.len.get(), sizes.get());
+    VJ_LAUNCH_CHECK();
+    size_t temp_bytes = 0;
+    VJ_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, sizes.get(), out.off.get(), slices + 1, st));
+    DeviceBuffer<unsigned char> temp;
+    VJ_TRY(temp.alloc(temp_bytes));
+    VJ_CUDA(cub::DeviceScan::ExclusiveSum(temp.get(), temp_bytes, sizes.get(), out.off.get(), slices + 1, st));
+    int64_t total = 0;
+    VJ_CUDA(cudaMemcpyAsync(&total, out.off.get() + slices, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    VJ_CUDA(cudaStreamSynchronize(st));
+    VJ_TRY(out.idx.alloc(static_cast<size_t>(total)));
+    VJ_TRY(out.val64.alloc(static_cast<size_t>(total)));
+    if (val32) VJ_TRY(out.val32.alloc(static_cast<size_t>(total)));
+    k_window_fill<<<windows, kSellWindow, 0, st>>>(v.rows, windows * kSellWindow, v.ptr, v.idx, val64, val32, out.perm.get(),
+                                                   out.len.get(), out.off.get(), out.idx.get(), out.val64.get(),
+                                                   val32 ? out.val32.get() : nullptr);
+    VJ_LAUNCH_CHECK();
+    note_launch(4);
+    v.win_off = out.off.get();
+    v.win_idx = out.idx.get();
+    v.win_perm = out.perm.get();
+    v.win_len = out.len.get();
+    v.sell_long_rows = out.long_rows.get();
+    v.sell_vlong_rows = out.vlong_rows.get();
+    return VAJRA_OK;
+}
+
 vajra_status unorder(int count, const int32_t* order, const double* src, double* dst, cudaStream_t st) {
     if (count <= 0) return VAJRA_OK;
     k_put<double><<<grid_for(count), kThreads, 0, st>>>(count, order, src, dst);

@@ -554,6 +554,87 @@ k_spmv_sell_hot(int rows, int slices, const int64_t* __restrict__ ptr, const int
     }
 }
 
+// ----- sliced ELL over windows ----------------------------------------------------------
+// For matrices whose rows are not numbered by length (the packed LPs of a batch): the rows are cut
+// into windows of 256, a CTA each; inside a window they are sorted by length and dealt to the
+// threads in that order, so that the window's eight slices are nearly full.  A thread forms its
+// row's sum in storage order from coalesced pairs of entries, as in k_spmv_sell, and leaves it in
+// shared memory; the epilogue then runs in row order, so its vector accesses coalesce and its early
+// loads are in flight beside the row's.  Long rows as in k_spmv_sell; list mode as in k_spmv_vec.
+// 256 LPs of 100 to 20,000 rows, 18.9M entries, FP64, an iteration (both SpMVs): 343 us with
+// the best lane groups (4 and 2 lanes a row: short strided runs of loads, a butterfly and one active
+// lane for the epilogue), 218 us here; 100 us of it is HBM traffic at the measured peak, and the gathers
+// alone take an SM's L1 about 135 us at one a cycle.
+constexpr int kSellWindow = kThreads;
+
+template <typename VV, typename VX, typename Acc, class Epi, int MB>
+__global__ void __launch_bounds__(kThreads, MB)
+k_spmv_sellw(int rows, int windows, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+             const VV* __restrict__ val, const int32_t* __restrict__ vlong_rows, int n_vlong,
+             const int32_t* __restrict__ long_rows, int n_long, const uint8_t* __restrict__ perm,
+             const uint8_t* __restrict__ sell_len, const int64_t* __restrict__ sell_off, const int32_t* __restrict__ sell_idx,
+             const VV* __restrict__ sell_val, const VX* __restrict__ x, const int32_t* __restrict__ blk_list,
+             const int* __restrict__ blk_count, Epi epi) {
+    __shared__ Acc sums[kSellWindow];
+    __shared__ uint8_t listed[kSellWindow];
+    pdl_enter();
+    if (!epi.active()) return;
+    int b = static_cast<int>(blockIdx.x);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (b < n_vlong) {
+        __shared__ Acc red[32];
+        const int row = vlong_rows[b];
+        if (skip_rows_impl(epi, row, row + 1, 0)) return;
+        const int64_t s = ptr[row], e = ptr[row + 1];
+        Acc acc = Acc(0);
+        for (int64_t k = s + tid; k < e; k += blockDim.x)
+            acc = fma(static_cast<Acc>(ld_stream(val + k)), static_cast<Acc>(ld_cached(x + ld_stream(idx + k))), acc);
+        Acc v[1] = {acc};
+        block_reduce<OpSum, Acc, 1>(v, red);
+        if (tid == 0) epi(row, v[0]);
+        return;
+    }
+    b -= n_vlong;
+    constexpr int kWarps = kThreads / 32;
+    const int long_ctas = (n_long + kWarps - 1) / kWarps;
+    if (b < long_ctas) {
+        const int w = b * kWarps + warp;
+        if (w < n_long) {
+            const int row = long_rows[w];
+            if (!skip_rows_impl(epi, row, row + 1, 0))
+                sell_warp_row<VV, VX, Acc>(row, ptr, idx, val, GatherGlobal<VX>{x}, epi);
+        }
+        return;
+    }
+    b -= long_ctas;
+    using VV2 = typename Pack2<VV>::type;
+    const int count = blk_list ? *blk_count : windows;
+    const int step = static_cast<int>(gridDim.x) - n_vlong - long_ctas;
+    for (int t = b; t < count; t += step) {
+        const int w = blk_list ? blk_list[t] : t;
+        const int row = w * kSellWindow + tid;
+        PreOf<Epi> pre{};
+        if (row < rows) pre = epi_pre(epi, row, 0);
+        const int len8 = __ldg(sell_len + row), p = __ldg(perm + row);   // padded to whole windows
+        const int64_t base = __ldg(sell_off + w * kWarps + warp) + 2 * lane;
+        const int len = len8 == kSellLong ? 0 : len8, pairs = (len + 1) >> 1;
+        Acc acc = Acc(0);
+#pragma unroll 4
+        for (int j = 0; j < pairs; ++j) {
+            const int64_t q = base + 64 * static_cast<int64_t>(j);
+            const int2 ii = __ldcs(reinterpret_cast<const int2*>(sell_idx + q));
+            const VV2 vv = __ldcs(reinterpret_cast<const VV2*>(sell_val + q));
+            acc = fma(static_cast<Acc>(vv.x), static_cast<Acc>(ld_cached(x + ii.x)), acc);
+            if (2 * j + 1 < len) acc = fma(static_cast<Acc>(vv.y), static_cast<Acc>(ld_cached(x + ii.y)), acc);
+        }
+        sums[p] = acc;
+        listed[p] = len8 == kSellLong;
+        __syncthreads();
+        if (row < rows && !listed[tid]) epi_fin(epi, row, sums[tid], pre, 0);
+        __syncthreads();   // the window's sums are taken
+    }
+}
+
 // Host-side description of one SpMV operand (a CSR, possibly the stored transpose) and the
 // launch shape the autotuner chose for it.
 struct CsrView {
@@ -588,6 +669,11 @@ struct CsrView {
     int sell_n_long = 0;
     const int32_t* sell_vlong_rows = nullptr;
     int sell_n_vlong = 0;
+    // Sliced ELL over windows (null where none was built); the long-row lists above are its too.
+    const int64_t* win_off = nullptr;
+    const int32_t* win_idx = nullptr;
+    const uint8_t* win_perm = nullptr;
+    const uint8_t* win_len = nullptr;
 };
 
 // Launch-shape code of the sliced-ELL kernel.
@@ -605,6 +691,23 @@ inline void launch_sell(const CsrView& a, const VV* csr_val, const VV* sell_val,
     launch_chained(k_spmv_sell<VV, VX, Acc, Epi, MB>, blocks, kThreads, 0, st,
                    a.rows, a.sell_slices, a.ptr, a.idx, csr_val, a.sell_vlong_rows, a.sell_n_vlong, a.sell_long_rows,
                    a.sell_n_long, a.sell_len, a.sell_off, a.sell_idx, sell_val, x, epi);
+    note_launch();
+}
+
+// Launch-shape code of sliced ELL over windows.
+constexpr int kSellWin = 130;
+inline int sell_windows(int rows) { return (rows + kSellWindow - 1) / kSellWindow; }
+
+template <typename VV, typename VX, typename Acc, class Epi>
+inline void launch_sellw(const CsrView& a, const VV* csr_val, const VV* win_val, const VX* x, Epi epi, cudaStream_t st) {
+    constexpr int MB = sizeof(VV) == 4 ? 6 : 4;
+    constexpr int kWarps = kThreads / 32;
+    const int windows = sell_windows(a.rows);
+    const int blocks = a.sell_n_vlong + (a.sell_n_long + kWarps - 1) / kWarps + (a.blk_list ? a.blk_grid : windows);
+    if (a.rows <= 0) return;
+    launch_chained(k_spmv_sellw<VV, VX, Acc, Epi, MB>, blocks, kThreads, 0, st, a.rows, windows, a.ptr, a.idx, csr_val,
+                   a.sell_vlong_rows, a.sell_n_vlong, a.sell_long_rows, a.sell_n_long, a.win_perm, a.win_len, a.win_off, a.win_idx,
+                   win_val, x, a.blk_list, a.blk_count, epi);
     note_launch();
 }
 

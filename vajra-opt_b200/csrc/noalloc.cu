@@ -31,7 +31,7 @@ static __device__ __align__(256) double g_noalloc_scratch[2 * 32768 * 4];
 namespace vajra {
 namespace {
 
-constexpr int kNaRowsPerBlock = 256;                 // 8 warps x 32 rows
+constexpr int kNaRowsPerBlock = 256;                 // at most
 constexpr int kNaMaxBlocks = 32768;                  // per pass
 constexpr int kNaQ = 4;                              // partial sums per block
 constexpr size_t kNoAllocScratchDoubles = 2ull * kNaMaxBlocks * kNaQ;
@@ -42,21 +42,37 @@ constexpr int kMaxDevices = 64;
 double* g_scratch_addr[kMaxDevices] = {};
 std::mutex g_scratch_mutex;
 
-// Row pass: one warp per row; primal residual A x - proj(A x), ||b||^2 (finite bounds, an
+// Row sums by lane groups: kNaLanes lanes a row, so that the lanes of rows of 8 to 20 entries have
+// work (a warp a row: two thirds of them idle, 32 rows one after another in every warp).  The whole
+// call: 100,003 x 250,007 (2M entries) 100 -> 49 us, 1000 x 2500 73 -> 19 us.
+constexpr int kNaLanes = 8;
+__device__ __forceinline__ double na_row_sum(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                                             const double* __restrict__ val, const double* __restrict__ x, int r, bool on) {
+    const int lane = threadIdx.x & (kNaLanes - 1);
+    double s = 0.0;
+    if (on) {
+        const int64_t e = ptr[r + 1];
+#pragma unroll 4
+        for (int64_t k = ptr[r] + lane; k < e; k += kNaLanes) s += __ldcs(val + k) * __ldg(x + __ldcs(idx + k));
+    }
+#pragma unroll
+    for (int o = kNaLanes / 2; o > 0; o /= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Row pass: primal residual A x - proj(A x), ||b||^2 (finite bounds, an
 // equality row once) and the row part of the dual objective.
 __global__ void __launch_bounds__(kThreads)
 k_na_rows(int m, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
           const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ rl,
-          const double* __restrict__ ru, double* __restrict__ part) {
+          const double* __restrict__ ru, int per_block, double* __restrict__ part) {
     __shared__ double red[kNaQ * 32];
     double v[kNaQ] = {0, 0, 0, 0};
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r0 = blockIdx.x * kNaRowsPerBlock;
-    for (int r = r0 + warp; r < r0 + kNaRowsPerBlock && r < m; r += kThreads / 32) {
-        double s = 0.0;
-        for (int64_t k = ptr[r] + lane; k < ptr[r + 1]; k += 32) s += val[k] * x[idx[k]];
-        s = warp_reduce<OpSum>(s);
-        if (lane == 0) {
+    const int r0 = blockIdx.x * per_block;
+    for (int q = threadIdx.x / kNaLanes; q < per_block; q += kThreads / kNaLanes) {   // whole warps
+        const int r = r0 + q;
+        const double s = na_row_sum(ptr, idx, val, x, r, r < m);
+        if (r < m && (threadIdx.x & (kNaLanes - 1)) == 0) {
             const double l = rl[r], u = ru[r];
             const bool lf = l > -1e20, uf = u < 1e20;
             const double p = s - fmin(fmax(s, l), u);
@@ -72,22 +88,20 @@ k_na_rows(int m, const int64_t* __restrict__ ptr, const int32_t* __restrict__ id
         for (int q = 0; q < kNaQ; ++q) part[blockIdx.x * kNaQ + q] = v[q];
 }
 
-// Column pass: one warp per column of the CSC; reduced cost r = c - A^T y (minimisation
+// Column pass over the CSC; reduced cost r = c - A^T y (minimisation
 // form), its bound-multiplier part, primal objective, ||c||^2, column part of the dual
 // objective.
 __global__ void __launch_bounds__(kThreads)
 k_na_cols(int n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
           const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ c,
-          const double* __restrict__ cl, const double* __restrict__ cu, int sense, double* __restrict__ part) {
+          const double* __restrict__ cl, const double* __restrict__ cu, int sense, int per_block, double* __restrict__ part) {
     __shared__ double red[kNaQ * 32];
     double v[kNaQ] = {0, 0, 0, 0};
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j0 = blockIdx.x * kNaRowsPerBlock;
-    for (int j = j0 + warp; j < j0 + kNaRowsPerBlock && j < n; j += kThreads / 32) {
-        double s = 0.0;
-        for (int64_t k = ptr[j] + lane; k < ptr[j + 1]; k += 32) s += val[k] * y[idx[k]];
-        s = warp_reduce<OpSum>(s);
-        if (lane == 0) {
+    const int j0 = blockIdx.x * per_block;
+    for (int q = threadIdx.x / kNaLanes; q < per_block; q += kThreads / kNaLanes) {   // whole warps
+        const int j = j0 + q;
+        const double s = na_row_sum(ptr, idx, val, y, j, j < n);
+        if (j < n && (threadIdx.x & (kNaLanes - 1)) == 0) {
             const double cm = sense ? -c[j] : c[j];
             const double r = cm - s;
             const bool lf = cl[j] > -1e20, uf = cu[j] < 1e20;
@@ -183,14 +197,21 @@ extern "C" vajra_status vajra_relative_kkt_noalloc_f64(
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double* scratch = nullptr;
     VJ_TRY(scratch_address(st, &scratch));
-    const int nb_r = (rows + kNaRowsPerBlock - 1) / kNaRowsPerBlock;
-    const int nb_c = (cols + kNaRowsPerBlock - 1) / kNaRowsPerBlock;
+    // 32 rows a block -- a round of its lane groups -- up to 1,024 blocks, then more, at most 256
+    const auto per_block = [](int count) {
+        int p = kThreads / kNaLanes;
+        while (p < kNaRowsPerBlock && (count + p - 1) / p > 1024) p *= 2;
+        return p;
+    };
+    const int per_r = per_block(rows), per_c = per_block(cols);
+    const int nb_r = (rows + per_r - 1) / per_r;
+    const int nb_c = (cols + per_c - 1) / per_c;
     double* part_r = scratch;
     double* part_c = scratch + static_cast<size_t>(kNaMaxBlocks) * kNaQ;
     if (has_rows)
-        k_na_rows<<<nb_r, kThreads, 0, st>>>(rows, row_ptr, col_idx, csr_values, x, y, row_lower, row_upper, part_r);
+        k_na_rows<<<nb_r, kThreads, 0, st>>>(rows, row_ptr, col_idx, csr_values, x, y, row_lower, row_upper, per_r, part_r);
     k_na_cols<<<nb_c, kThreads, 0, st>>>(cols, col_ptr, row_idx, csc_values, x, y, c, col_lower, col_upper, sense,
-                                         part_c);
+                                         per_c, part_c);
     k_na_final<<<1, 1024, 0, st>>>(nb_r, nb_c, part_r, part_c, sense ? -objective_offset : objective_offset, out);
     note_launch(has_rows ? 3 : 2);
     VJ_LAUNCH_CHECK();

@@ -891,7 +891,7 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
         std::fprintf(stderr, "[vajra] set-up %-14s %8.1f ms\n", what, 1e3 * seconds_since(t_start));
     };
     if (ordered && !h->ordered) {
-        VJ_TRY(order_by_degree(h->lp, h->lp_ordered, h->order, st));
+        VJ_TRY(order_by_degree(h->lp, h->lp_ordered, h->order, !mixed, st));
         h->ordered = true;
     }
     const DeviceLp& lp = ordered ? h->lp_ordered : h->lp;

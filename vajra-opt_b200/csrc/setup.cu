@@ -689,14 +689,23 @@ vajra_status plan_spmv(const DeviceLp& lp, Prepared& p, cudaStream_t st) {
 // ---------------------------------------------------------------------------------------
 // degree ordering
 // ---------------------------------------------------------------------------------------
-// Sort keys: descending entry count as an ascending unsigned key (the stable radix sort keeps
-// equal counts in index order).
-__global__ void k_col_count_keys(int n, const int64_t* __restrict__ col_ptr, uint32_t* __restrict__ keys,
-                                 int32_t* __restrict__ idx) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    keys[j] = 0xffffffffu - static_cast<uint32_t>(col_ptr[j + 1] - col_ptr[j]);
-    idx[j] = j;
+// Sort keys of the columns, eight lanes a column: descending entry count, then (row_bits > 0) the
+// smallest of its rows' new numbers.  Equal keys keep index order.
+__global__ void k_col_keys(int n, int m, int row_bits, const int64_t* __restrict__ col_ptr, const int32_t* __restrict__ row_idx,
+                           const int32_t* __restrict__ row_inv, uint64_t* __restrict__ keys, int32_t* __restrict__ idx) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int lane = static_cast<int>(t & 7);
+    const int64_t j = t >> 3;
+    int64_t s = 0, e = 0;
+    if (j < n) { s = col_ptr[j]; e = col_ptr[j + 1]; }
+    int first = row_bits > 0 && e > s ? m : 0;
+    if (row_bits > 0)
+        for (int64_t k = s + lane; k < e; k += 8) first = min(first, row_inv[row_idx[k]]);
+    for (int w = 4; w > 0; w >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, w));
+    if (lane != 0 || j >= n) return;
+    const int64_t len = e - s;
+    keys[j] = static_cast<uint64_t>(m - (len < m ? len : m)) << row_bits | static_cast<uint32_t>(first);
+    idx[j] = static_cast<int32_t>(j);
 }
 
 __global__ void k_row_counts(int64_t nnz, const int32_t* __restrict__ row_idx, uint32_t* __restrict__ counts) {
@@ -752,23 +761,24 @@ __global__ void k_put(int count, const int32_t* __restrict__ order, const T* __r
     if (k < count) dst[order[k]] = src[k];
 }
 
-static vajra_status sort_order(int count, const uint32_t* keys, DeviceBuffer<int32_t>& idx,
-                               DeviceBuffer<int32_t>& order, cudaStream_t st) {
-    DeviceBuffer<uint32_t> keys_out;
+template <typename Key>
+static vajra_status sort_order(int count, const Key* keys, int bits, DeviceBuffer<int32_t>& idx, DeviceBuffer<int32_t>& order,
+                               cudaStream_t st) {
+    DeviceBuffer<Key> keys_out;
     VJ_TRY(keys_out.alloc(static_cast<size_t>(count)));
     size_t temp_bytes = 0;
     VJ_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_out.get(), idx.get(), order.get(), count,
-                                            0, 32, st));
+                                            0, bits, st));
     DeviceBuffer<unsigned char> temp;
     VJ_TRY(temp.alloc(temp_bytes));
     VJ_CUDA(cub::DeviceRadixSort::SortPairs(temp.get(), temp_bytes, keys, keys_out.get(), idx.get(), order.get(),
-                                            count, 0, 32, st));
-    note_launch(4);
+                                            count, 0, bits, st));
+    note_launch((bits + 7) / 8);
     VJ_CUDA(cudaStreamSynchronize(st));   // temporaries die here
     return VAJRA_OK;
 }
 
-vajra_status order_by_degree(const DeviceLp& src, DeviceLp& dst, LpOrder& ord, cudaStream_t st) {
+vajra_status order_by_degree(const DeviceLp& src, DeviceLp& dst, LpOrder& ord, bool by_first_row, cudaStream_t st) {
     const int m = src.m, n = src.n;
     const int64_t nnz = src.nnz;
     dst.m = m;
@@ -780,15 +790,6 @@ vajra_status order_by_degree(const DeviceLp& src, DeviceLp& dst, LpOrder& ord, c
     VJ_TRY(ord.row_order.alloc(static_cast<size_t>(m)));
     DeviceBuffer<uint32_t> keys;
     DeviceBuffer<int32_t> idx, row_inv;
-    // columns
-    VJ_TRY(keys.alloc(static_cast<size_t>(n)));
-    VJ_TRY(idx.alloc(static_cast<size_t>(n)));
-    if (n > 0) {
-        k_col_count_keys<<<grid_for(n), kThreads, 0, st>>>(n, src.col_ptr.get(), keys.get(), idx.get());
-        VJ_LAUNCH_CHECK();
-        note_launch(1);
-        VJ_TRY(sort_order(n, keys.get(), idx, ord.col_order, st));
-    }
     // rows
     VJ_TRY(keys.alloc(static_cast<size_t>(m)));
     VJ_TRY(idx.alloc(static_cast<size_t>(m)));
@@ -799,10 +800,24 @@ vajra_status order_by_degree(const DeviceLp& src, DeviceLp& dst, LpOrder& ord, c
         k_row_count_keys<<<grid_for(m), kThreads, 0, st>>>(m, keys.get(), idx.get());
         VJ_LAUNCH_CHECK();
         note_launch(nnz > 0 ? 2 : 1);
-        VJ_TRY(sort_order(m, keys.get(), idx, ord.row_order, st));
+        VJ_TRY(sort_order(m, keys.get(), 32, idx, ord.row_order, st));
         k_invert<<<grid_for(m), kThreads, 0, st>>>(m, ord.row_order.get(), row_inv.get());
         VJ_LAUNCH_CHECK();
         note_launch(1);
+    }
+    // columns
+    if (n > 0) {
+        DeviceBuffer<uint64_t> col_keys;
+        VJ_TRY(col_keys.alloc(static_cast<size_t>(n)));
+        VJ_TRY(idx.alloc(static_cast<size_t>(n)));
+        int bits = 1;   // of a row number, and of a count (0..m)
+        while ((1LL << bits) <= m) ++bits;
+        const int row_bits = by_first_row ? bits : 0;
+        k_col_keys<<<grid_for(8 * static_cast<int64_t>(n)), kThreads, 0, st>>>(n, m, row_bits, src.col_ptr.get(), src.row_idx.get(),
+                                                                              row_inv.get(), col_keys.get(), idx.get());
+        VJ_LAUNCH_CHECK();
+        note_launch(1);
+        VJ_TRY(sort_order(n, col_keys.get(), row_bits + bits, idx, ord.col_order, st));
     }
     // matrix: new column pointers, then the columns' entries with renumbered rows
     VJ_TRY(dst.col_ptr.alloc(static_cast<size_t>(n) + 1));

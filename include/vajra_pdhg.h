@@ -102,7 +102,9 @@ typedef struct vajra_opts {
     double tolerance;           /* REFERENCE: max-abs primal and dual residual
                                    ("tolerance"); HALPERN: relative KKT target           */
     double gap_tolerance;       /* REFERENCE: relative gap ("gap_tolerance")             */
-    double time_limit;          /* seconds (Options::time_limit)                         */
+    double time_limit;          /* seconds (Options::time_limit); HALPERN checks it between
+                                   launches: after every check, or for LPs that run on a
+                                   thread-block cluster after up to 16 checks, then what fits */
     int64_t iteration_limit;    /* Options::iteration_limit                              */
     int32_t check_frequency;    /* REFERENCE: "check_frequency" (100); HALPERN: KKT /
                                    restart evaluation interval (64)                      */
@@ -126,7 +128,9 @@ typedef struct vajra_opts {
     int32_t restart_metric;     /* 0: primal-weighted KKT of T(z); 1: fixed-point residual
                                    sqrt(omega ||x+ - x||^2 + ||y+ - y||^2 / omega)          */
     int32_t spmv_shape_a;       /* HALPERN launch shape of the A x SpMV: 0 autotune (>= 2^20
-                                   entries) or the set-up heuristic, -1 row-block kernel,
+                                   entries) or the set-up heuristic (where the LP fits, its
+                                   iterations run on a thread-block cluster; any other value
+                                   keeps them off it), -1 row-block kernel,
                                    -2 row-block kernel with two load groups per thread,
                                    -3 sliced ELL (degree-ordered LPs; else the row-block
                                    kernel), -4 sliced ELL with the first vector entries in
@@ -141,8 +145,9 @@ typedef struct vajra_opts {
                                    rounding noise from building up within a restart epoch  */
     int32_t degree_order;       /* HALPERN: renumber rows and columns by descending entry
                                    count on the device, so that the vector entries the SpMVs
-                                   gather most often share cache lines; results come back in
-                                   the caller's numbering.  0 auto (on from 2^20 entries),
+                                   gather most often share cache lines (FP64 solves number
+                                   columns of equal counts by their first row); results come
+                                   back in the caller's numbering.  0 auto (on from 2^20 entries),
                                    1 on, -1 off                                            */
     int32_t pow2_scaling;       /* HALPERN: 1 = round the final row / column scale factors to
                                    the nearest power of two, so that scaling is exact: a
@@ -215,7 +220,8 @@ typedef struct vajra_result {
     int32_t spmv_group_at;      /* same for A^T y                                           */
     /* Live kernel timing (HALPERN): CUDA-event durations of the fused iteration kernels,
      * sampled on the solve's stream once per check interval, for the precision that ran
-     * most iterations, with the algorithmic bytes one launch must move. */
+     * most iterations, with the algorithmic bytes one launch must move.  Where a thread-block
+     * cluster runs the iterations: the two halves of one by the device's timer, exchange included. */
     double primal_kernel_us;    /* v = A^T y + primal prox / Halpern (stored transpose)   */
     double dual_kernel_us;      /* w = A x_bar + dual prox / Halpern (CSR)                 */
     double primal_kernel_bytes;
@@ -283,8 +289,10 @@ vajra_status vajra_pdhg_create(const vajra_lp* lp, const vajra_opts* opts, vajra
  * iterates and sums, FP64 checks), in which each instance either reaches the tolerance or -- at
  * mixed_switch_tolerance or on a stall -- hands over to an FP64 pass that restarts it from its
  * FP32 candidate; VAJRA_PREC_FP64 runs the FP64 pass alone.  Each pass runs on the device in
- * graph launches of many chunks; time_limit is checked after each (the first launch of a pass
- * runs 2048 iterations, later ones what fits in the time left at the measured rate).  Replaces a host loop of solve_pdhg_gpu calls (gpu.hpp:59), as
+ * launches of many chunks; time_limit is checked after each (the first launch of a pass runs 2048
+ * iterations, later ones what fits in the time left at the measured rate; without a limit to
+ * speak of, each twice what ran before).  Instances that fit a thread-block cluster run on one
+ * each, beside the packed rest.  Replaces a host loop of solve_pdhg_gpu calls (gpu.hpp:59), as
  * the reference's benchmark Suite 2 issues them (apps/benchmark_runner.cpp:936-944).
  * results[i] receives instance i; every result's device_time_sec is the whole batch's. */
 vajra_status vajra_pdhg_solve_batch(int32_t count, const vajra_lp* lps, const vajra_opts* opts,

@@ -63,8 +63,9 @@ void* pinned_scratch(size_t bytes);
 // serialization: the next kernel's CTAs may be scheduled while the previous kernel in the
 // stream is still draining, which hides most of the launch gap between the two SpMVs of an
 // iteration when the SpMVs themselves take a few microseconds.  Every kernel launched that way
-// runs pdl_enter() before anything else: griddepcontrol.wait returns once the previous kernel
-// has completed and its writes are visible, so nothing is read or written early, and a kernel
+// runs pdl_enter() before anything that a kernel of the solve writes is read (k_spmv_sell reads the row
+// lengths and slice offsets before it: the set-up wrote them and drained the stream):
+// griddepcontrol.wait returns once the previous kernel has completed and its writes are visible, and a kernel
 // that then returns at once has still waited (the kernel after it sees everything before it).
 // launch_dependents then lets the next kernel be scheduled.  In a kernel launched without the
 // attribute both instructions return at once.  VAJRA_PDL=0 in the environment launches the

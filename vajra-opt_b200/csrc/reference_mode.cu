@@ -108,7 +108,7 @@ k_cluster_reference(const __grid_constant__ ClMats<double> M, EpiRefDual D, EpiR
     const double tau = st->tau, sigma = st->sigma;
     const long long base = st->iter_base;
     double x = 0.0, xb = 0.0, c = 0.0, cl = 0.0, cu = 0.0, y = 0.0, rl = 0.0, ru = 0.0;
-    if (j >= 0) { x = Q.x[j]; c = Q.c[j]; cl = Q.cl[j]; cu = Q.cu[j]; }
+    if (j >= 0) { x = Q.x[j]; xb = Q.xb[j]; c = Q.c[j]; cl = Q.cl[j]; cu = Q.cu[j]; }   // (len may be 0: x_bar stays)
     if (i >= 0) { y = D.y[i]; rl = D.rl[i]; ru = D.ru[i]; }
     int bad = len + 1;   // my first iteration with a NaN or an infinity
 #pragma unroll 1

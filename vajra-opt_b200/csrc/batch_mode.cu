@@ -499,11 +499,18 @@ k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ 
                   smem_bytes);
 }
 
-// done = 1 for the instances that a path does not run: `on` (null: none) marks those on clusters,
-// `want` is the path's mark; an instance that has finished (status set) is run by neither.
-__global__ void k_bassign(int count, const int* __restrict__ on, int want, const int* __restrict__ status, int* __restrict__ done) {
+// Before a launch: done = 1 in each path's array for the instances that it does not run.  `on`
+// (null: none) marks those on clusters; an instance that has finished (status set) is run by
+// neither.  An instance may come from the other path: the restart that its last packed check asked
+// for has been carried out, so its flag is cleared -- the packed path would repeat the restart after
+// each of its chunks, into the vectors that a cluster iterates on beside it.
+__global__ void k_bassign(int count, const int* __restrict__ on, BatchArrays S, int* __restrict__ done_cl) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) done[i] = (on && on[i] != 0) == (want != 0) && status[i] == 0 ? 0 : 1;
+    if (i >= count) return;
+    const bool open = S.status[i] == 0, cluster = on && on[i] != 0;
+    S.done[i] = open && !cluster ? 0 : 1;
+    done_cl[i] = open && cluster ? 0 : 1;
+    S.restart_flag[i] = 0;
 }
 
 // Counts the unfinished instances.  Inside the WHILE body of a pass graph (`loop` = 1) it also
@@ -553,8 +560,10 @@ __global__ void k_brestart(int m, int n, const int* __restrict__ row_inst, const
                            T* __restrict__ x0, T* __restrict__ y, T* __restrict__ y0,
                            double* __restrict__ x_last, double* __restrict__ y_last, BatchArrays S) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n && S.restart_flag[col_inst[t]]) { const T v = xc[t]; x[t] = v; x0[t] = v; x_last[t] = v; }
-    if (t < m && S.restart_flag[row_inst[t]]) { const T v = yc[t]; y[t] = v; y0[t] = v; y_last[t] = v; }
+    // (an instance that is done here may be running on a cluster)
+    auto restarts = [&](int i) { return S.restart_flag[i] && !S.done[i]; };
+    if (t < n && restarts(col_inst[t])) { const T v = xc[t]; x[t] = v; x0[t] = v; x_last[t] = v; }
+    if (t < m && restarts(row_inst[t])) { const T v = yc[t]; y[t] = v; y0[t] = v; y_last[t] = v; }
 }
 
 // End of the FP32 pass, vectors: every instance's FP32 candidate becomes its FP64 candidate
@@ -1165,9 +1174,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
             bool general = false;
             for (int i = 0, q = 0; i < count; ++i) q += open[i], general = general || q > static_cast<int>(cl.insts.size());
             const unsigned cg = (count + 127) / 128;
-            k_bassign<<<cg, 128, 0, st>>>(count, cl.d_on.get(), 0, S.status, S.done);
-            k_bassign<<<cg, 128, 0, st>>>(count, cl.d_on.get(), 1, S.status, done_cl.get());
-            note_launch(2);
+            k_bassign<<<cg, 128, 0, st>>>(count, cl.d_on.get(), S, done_cl.get());
+            note_launch(1);
             if (!cl.insts.empty()) VJ_CUDA(cudaMemsetAsync(cl_shared.get(), 0, sizeof(ClControl) * cl.insts.size(), st));
             int64_t budget = 1;   // chunks of this launch
             if (remaining >= K) {
@@ -1245,11 +1253,10 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                                                        x.get(), x0.get(), xc.get(), x_last.get(), y.get(), y0.get(),
                                                        yc.get(), y_last.get(), S.status);
         k_bhandover_state<<<(count + 127) / 128, 128, 0, st>>>(count, o.reflection, S);
-        k_bassign<<<(count + 127) / 128, 128, 0, st>>>(count, nullptr, 0, S.status, S.done);
-        k_bassign<<<(count + 127) / 128, 128, 0, st>>>(count, nullptr, 1, S.status, done_cl.get());
+        k_bassign<<<(count + 127) / 128, 128, 0, st>>>(count, nullptr, S, done_cl.get());
         k_btotals<<<1, 1024, 0, st>>>(count, S.done, done_cl.get(), S.total, cl_shared.get(), 0, counters.get());
         VJ_LAUNCH_CHECK();
-        note_launch(5);
+        note_launch(4);
         VJ_CUDA(cudaMemcpyAsync(hc, counters.get(), sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
     }

@@ -49,3 +49,36 @@ def test_packed_instances_that_move_to_clusters_repeat_bit_for_bit(cuda, prec):
         assert u["iterations"] == v["iterations"] == FIRST + 1024 and u["restart_count"] == v["restart_count"]
         for k in KEYS:
             np.testing.assert_allclose(u[k], v[k], rtol=0, atol=bound * (1.0 + np.abs(v[k]).max()), err_msg=k)
+
+
+def singletons_first(seed):
+    """1,000 x 2,400: 300 columns of one entry, then 2,100 of 15.  Equal shares of the entries give a
+    CTA of 8 (512 threads) up to 420 columns, one of 16 (256 threads) 260: the wider cluster does not
+    hold it."""
+    lp = W.random_planted(1000, 2400, 15, seed=seed)
+    a = lp.to_scipy_csc().tolil()
+    for j in range(300):
+        a[:, j] = 0.0
+        a[(7 * j) % 1000, j] = 1.0 + 0.01 * j
+    a = a.tocsc()
+    a.eliminate_zeros()
+    a.sort_indices()
+    x, y, z = lp.x_planted, lp.y_planted, lp.c - lp.to_scipy_csc().T @ lp.y_planted
+    lp.col_ptr, lp.row_idx, lp.values = a.indptr.astype(np.int64), a.indices.astype(np.int32), a.data
+    lp.row_lower = lp.row_upper = a @ x
+    lp.c = a.T @ y + z
+    return lp
+
+
+@pytest.mark.parametrize("limit", [FIRST + 64, FIRST + 576])
+@pytest.mark.parametrize("prec", [V.PREC_FP64, V.PREC_MIXED])
+def test_an_instance_left_alone_goes_on_as_the_packed_iteration(cuda, prec, limit):
+    """Nine of ten finish at the first check; for the second launch the tenth could have a cluster
+    twice as wide, which does not hold it.  Bound as above, 2,624 iterations and 2,400 columns."""
+    lps = [solved_at_once(singletons_first(q)) for q in range(9)] + [singletons_first(9)]
+    kw = options(prec, limit)
+    u, v = V.solve_batch(lps, **kw)[9], V.solve_batch(lps, spmv_shape_a=1, **kw)[9]
+    assert u["iterations"] == v["iterations"] == limit and u["restart_count"] == v["restart_count"] > 0
+    bound = 2624 * (4 * 2400 * 2.0 ** -53 if prec == V.PREC_FP64 else 2.0 ** -24)
+    for k in KEYS:
+        np.testing.assert_allclose(u[k], v[k], rtol=0, atol=bound * (1.0 + np.abs(v[k]).max()), err_msg=k)

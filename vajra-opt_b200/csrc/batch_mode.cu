@@ -503,7 +503,8 @@ k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ 
 // (null: none) marks those on clusters; an instance that has finished (status set) is run by
 // neither.  An instance may come from the other path: the restart that its last packed check asked
 // for has been carried out, so its flag is cleared -- the packed path would repeat the restart after
-// each of its chunks, into the vectors that a cluster iterates on beside it.
+// each of its chunks, into the vectors that a cluster iterates on beside it.  And the packed path
+// reads an instance's Halpern weights from S.hw, which clusters do not keep up.
 __global__ void k_bassign(int count, const int* __restrict__ on, BatchArrays S, int* __restrict__ done_cl) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
@@ -511,6 +512,7 @@ __global__ void k_bassign(int count, const int* __restrict__ on, BatchArrays S, 
     S.done[i] = open && !cluster ? 0 : 1;
     done_cl[i] = open && cluster ? 0 : 1;
     S.restart_flag[i] = 0;
+    if (open && !cluster) instance_weights(S, i);
 }
 
 // Counts the unfinished instances.  Inside the WHILE body of a pass graph (`loop` = 1) it also

@@ -1176,6 +1176,7 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
     int timed_out = 0;
     int64_t cl_chunks = 0;   // chunks the clusters of this solve have run, and their host time
     double cl_seconds = 0.0;
+    bool weights_kept = true;   // cb.hw holds the next chunk's Halpern weights (clusters do not keep it up)
     while (launched < max_iter) {
         const ClusterPlan& plan = cur_phase == 0 ? cl32 : cl64;
         if (plan.ctas) {
@@ -1197,6 +1198,7 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
             }
             if (hs->total <= launched) return VAJRA_ERR_INTERNAL;   // a launch runs at least one chunk
             launched = hs->total;
+            weights_kept = false;
         } else {
             const int64_t remaining = max_iter - launched;
             const int len = static_cast<int>(remaining < K ? remaining : K);
@@ -1225,6 +1227,12 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
                 }
                 return VAJRA_OK;
             };
+            if (!weights_kept) {   // the phase before ran on a cluster
+                k_halpern_weights<<<1, kThreads, 0, st>>>(S, cb.hw_len, cb.hw.get());
+                VJ_LAUNCH_CHECK();
+                note_launch(1);
+                weights_kept = true;
+            }
             if (cur_phase == 0) { VJ_TRY(run_chunk(p32)); } else { VJ_TRY(run_chunk(p64)); }
             launched += len;
             VJ_CUDA(cudaMemcpyAsync(hs, S, sizeof(HState), cudaMemcpyDeviceToHost, st));

@@ -82,3 +82,13 @@ def test_an_instance_left_alone_goes_on_as_the_packed_iteration(cuda, prec, limi
     bound = 2624 * (4 * 2400 * 2.0 ** -53 if prec == V.PREC_FP64 else 2.0 ** -24)
     for k in KEYS:
         np.testing.assert_allclose(u[k], v[k], rtol=0, atol=bound * (1.0 + np.abs(v[k]).max()), err_msg=k)
+
+
+@pytest.mark.parametrize("prec", [V.PREC_FP64, V.PREC_MIXED])
+def test_a_cluster_that_holds_an_instance_is_kept(cuda, prec):
+    """The same batch: the wider cluster's refusal costs the tenth LP nothing.  Sixteen more checks are
+    sixteen packed chunks of 2 x 64 launches and more, or one launch of its cluster."""
+    lps = [solved_at_once(singletons_first(q)) for q in range(9)] + [singletons_first(9)]
+    a, b = (V.solve_batch(lps, **options(prec, FIRST + n)) for n in (64, 64 + 1024))
+    assert a[9]["iterations"] == FIRST + 64 and b[9]["iterations"] == FIRST + 1088
+    assert b[9]["kernel_launches"] - a[9]["kernel_launches"] < 128

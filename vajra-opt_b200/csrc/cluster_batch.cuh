@@ -47,6 +47,7 @@ struct ClusterClass {
 };
 struct ClusterBatch {
     std::vector<int> least;              // per instance: CTAs of its smallest cluster, 0: it has none
+    std::vector<int> most;               // per instance: CTAs of the widest that may hold it (set by the first plan)
     std::vector<int> insts;              // the instances of the present plan, by class, largest first
     std::vector<ClusterClass> classes;   // widest clusters first
     DeviceBuffer<int> d_insts, d_on;     // the same list; per instance: runs on a cluster
@@ -118,6 +119,7 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
     VJ_TRY(out.d_insts.alloc(count));
     VJ_TRY(out.d_on.alloc(count));
     std::vector<int> ctas(count), threads(count), on(count), h(count);
+    out.most.resize(count, kClMaxCtas);
     auto fits = [&](int i, int c, int t) {
         return cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, M.group_a, M.group_at, c, t);
     };
@@ -132,7 +134,7 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
         while (sms_used > 0 && 2 * sms_used <= sm_count()) {
             int64_t used = 0;
             for (int i = 0; i < count; ++i) {
-                if (ctas[i] > 0 && ctas[i] < kClMaxCtas && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
+                if (ctas[i] > 0 && ctas[i] < out.most[i] && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
                     ctas[i] *= 2;
                 used += ctas[i];
             }
@@ -163,7 +165,14 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
                 out.classes.push_back(k);
             }
         if (out.insts.empty()) break;
-        // Instances whose uneven rows do not fit after all get a wider cluster, at last none.
+        // Uneven rows may not fit after all, or the device may lack such a cluster.  An instance on more
+        // CTAs than it needs then goes back to half of them for good; one on its smallest cluster gets a
+        // wider one where its rows are uneven, at last none.
+        auto refuse = [&](int i, bool uneven) {
+            if (ctas[i] > out.least[i]) out.most[i] = ctas[i] / 2;
+            else out.least[i] = uneven ? least_cluster<T>(lps[i], M.group_a, M.group_at, 2 * ctas[i]) : 0;
+            again = true;
+        };
         VJ_CUDA(cudaMemcpyAsync(out.d_insts.get(), out.insts.data(), sizeof(int) * out.insts.size(), cudaMemcpyHostToDevice, st));
         VJ_CUDA(cudaMemsetAsync(nofit.get(), 0, sizeof(int) * count, st));
         for (const ClusterClass& k : out.classes) {
@@ -171,8 +180,7 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
             if (e == cudaSuccess) e = prepare_clusters(fit_kernel<T>(k.threads), k.ctas, k.threads, k.smem);
             if (e != cudaSuccess) {   // no such cluster on this device
                 cudaGetLastError();
-                for (int q = k.first; q < k.first + k.clusters; ++q) out.least[out.insts[q]] = 0;
-                again = true;
+                for (int q = k.first; q < k.first + k.clusters; ++q) refuse(out.insts[q], false);
                 continue;
             }
             VJ_CUDA(launch_clusters(fit_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, st, M, out.d_insts.get() + k.first,
@@ -181,7 +189,7 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
         VJ_CUDA(cudaMemcpyAsync(h.data(), nofit.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
         for (int q : out.insts)
-            if (h[q]) { out.least[q] = least_cluster<T>(lps[q], M.group_a, M.group_at, 2 * ctas[q]); again = true; }
+            if (h[q]) refuse(q, true);
     }
     for (int q : out.insts) on[q] = 1;
     VJ_CUDA(cudaMemcpyAsync(out.d_on.get(), on.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));

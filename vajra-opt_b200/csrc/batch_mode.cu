@@ -768,8 +768,10 @@ constexpr int64_t kClBatchEntries = int64_t(4) << 20;
 
 }  // namespace
 
-vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajra_result* results,
-                       cudaStream_t st, double* device_time) {
+// One attempt.  `windows`: may hold optional copies of the matrices over windows; false on return
+// where it held none.
+static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_opts& o, vajra_result* results,
+                                   cudaStream_t st, double* device_time, bool& windows) {
     const auto t_start = Clock::now();
     // ---- packing (block-diagonal CSC), straight into the device buffers ----------------------
     // Each instance's arrays are copied to their slots of the packed arrays as they are; two
@@ -907,7 +909,8 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
     // (Mixed batches take windows only by that choice: an FP32 row summed by one thread in storage order rounds
     // differently from one summed by lane groups, and instances then stop at other points.  512 LPs of
     // 100 to 20,000 rows, mixed: worst objective error 3.0e-5 against 8.8e-6, for 2.35 against 2.53 s.)
-    if (fixed_windows || (o.autotune && !mixed && NNZ >= (int64_t(1) << 20))) {
+    windows = windows && !fixed_windows && o.autotune && !mixed && NNZ >= (int64_t(1) << 20);
+    if (fixed_windows || windows) {
         VJ_TRY(build_windows(p.a, p.csr_val.get(), mixed ? p.csr_val32.get() : nullptr, win_a, st));
         VJ_TRY(build_windows(p.at, p.csc_val.get(), mixed ? p.csc_val32.get() : nullptr, win_at, st));
     }
@@ -1333,6 +1336,20 @@ vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajr
                       : "limit reached before this instance converged (batched)");
     }
     return VAJRA_OK;
+}
+
+vajra_status run_batch(int count, const vajra_lp* lps, const vajra_opts& o, vajra_result* results,
+                       cudaStream_t st, double* device_time) {
+    bool windows = true;
+    const vajra_status s = run_batch_once(count, lps, o, results, st, device_time, windows);
+    if (s != VAJRA_ERR_OUT_OF_MEMORY || !windows) return s;
+    // The copies over windows are for speed alone (24 bytes an entry): a batch that they do not leave
+    // enough memory for runs without them.  The first attempt's blocks are given back first.
+    cudaGetLastError();
+    VJ_CUDA(cudaStreamSynchronize(st));
+    release_cached_blocks(o.device);
+    windows = false;
+    return run_batch_once(count, lps, o, results, st, device_time, windows);
 }
 
 }  // namespace vajra

@@ -614,12 +614,18 @@ __global__ void k_bshift_cols(int n, const int* __restrict__ col_inst, const int
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j < n) col_ptr[j] += zoff[col_inst[j]];
 }
+// An index outside its instance's rows sets *bad: a cluster gathers from shared memory by it.
 __global__ void k_bshift_rows(int n, const int* __restrict__ col_inst, const int64_t* __restrict__ roff,
-                              const int64_t* __restrict__ col_ptr, int32_t* __restrict__ row_idx) {
+                              const int64_t* __restrict__ col_ptr, int32_t* __restrict__ row_idx, int* __restrict__ bad) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int32_t r0 = static_cast<int32_t>(roff[col_inst[j]]);
-    for (int64_t k = col_ptr[j]; k < col_ptr[j + 1]; ++k) row_idx[k] += r0;
+    const uint32_t rows = static_cast<uint32_t>(roff[col_inst[j] + 1] - r0);
+    for (int64_t k = col_ptr[j]; k < col_ptr[j + 1]; ++k) {
+        const int32_t r = row_idx[k];
+        if (static_cast<uint32_t>(r) >= rows) { *bad = 1; return; }
+        row_idx[k] = r0 + r;
+    }
 }
 __global__ void k_bmin_c(int n, const int* __restrict__ col_inst, const int* __restrict__ sense,
                          const double* __restrict__ c, double* __restrict__ cmin) {
@@ -840,12 +846,19 @@ static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_o
     k_fill_inst<<<count, kThreads, 0, st>>>(M, d_roff.get(), count, row_inst.get());
     k_fill_inst<<<count, kThreads, 0, st>>>(N, d_coff.get(), count, col_inst.get());
     k_bshift_cols<<<grid_for(n), kThreads, 0, st>>>(n, col_inst.get(), d_zoff.get(), lp.col_ptr.get());
+    DeviceBuffer<int> d_bad;
+    VJ_TRY(d_bad.alloc(1));
+    VJ_CUDA(cudaMemsetAsync(d_bad.get(), 0, sizeof(int), st));
     k_bshift_rows<<<grid_for(n), kThreads, 0, st>>>(n, col_inst.get(), d_roff.get(), lp.col_ptr.get(),
-                                                    lp.row_idx.get());
+                                                    lp.row_idx.get(), d_bad.get());
     // the packed problem is a minimisation: maximisation instances' objectives are negated
     k_bmin_c<<<grid_for(n), kThreads, 0, st>>>(n, col_inst.get(), d_sense.get(), lp.c.get(), d_cmin.get());
     VJ_LAUNCH_CHECK();
     note_launch(5);
+    int bad = 0;
+    VJ_CUDA(cudaMemcpyAsync(&bad, d_bad.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+    VJ_CUDA(cudaStreamSynchronize(st));
+    if (bad) { set_error("row index out of range in a batch instance"); return VAJRA_ERR_INVALID_ARGUMENT; }
     mark("packed on the device");
 
     // ---- set-up on the packed problem --------------------------------------------------

@@ -147,7 +147,7 @@ struct BwdVectors {
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 k_cluster_forward(const __grid_constant__ FwdVectors<T> F, const __grid_constant__ BMats<T> M, const int* __restrict__ insts,
-                  const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, uint32_t smem_bytes) {
+                  const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, ClLaunch L) {
     __shared__ ClInfo I;
     __shared__ ClMats<T> mats;
     const int inst = insts[blockIdx.x / cl_size()];
@@ -155,7 +155,7 @@ k_cluster_forward(const __grid_constant__ FwdVectors<T> F, const __grid_constant
     if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
     __syncthreads();
     ClCore<T, T> core;
-    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
+    if (!core.begin(mats.a, mats.at, L, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
     for (int i = threadIdx.x; i < I.m; i += NT) core.yf[i] = F.y[r0 + i];
     cl_barrier();
     if (*static_cast<volatile int*>(failed + inst)) return;   // uniform over the cluster
@@ -200,7 +200,7 @@ k_cluster_forward(const __grid_constant__ FwdVectors<T> F, const __grid_constant
     if (j >= 0) F.x[j] = x;
     if (i >= 0) F.y[i] = y;
     if (core.dead) failed[inst] = 2;
-    cl_barrier();   // no CTA ends while a peer may still send to it
+    core.leave(I);
 }
 
 // Cluster q: the reverse of `steps` steps for instance insts[q].  The full y holds w^ = sigma q^,
@@ -208,7 +208,7 @@ k_cluster_forward(const __grid_constant__ FwdVectors<T> F, const __grid_constant
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 k_cluster_backward(const __grid_constant__ BwdVectors<T> B, const __grid_constant__ BMats<T> M, const int* __restrict__ insts,
-                   const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, uint32_t smem_bytes) {
+                   const int64_t* __restrict__ roff, const int64_t* __restrict__ coff, int steps, int* failed, ClLaunch L) {
     __shared__ ClInfo I;
     __shared__ ClMats<T> mats;
     const int inst = insts[blockIdx.x / cl_size()];
@@ -216,7 +216,7 @@ k_cluster_backward(const __grid_constant__ BwdVectors<T> B, const __grid_constan
     if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
     __syncthreads();
     ClCore<T, T> core;
-    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
+    if (!core.begin(mats.a, mats.at, L, I) && threadIdx.x == 0) failed[inst] = 1;   // (planned to fit)
     cl_barrier();
     if (*static_cast<volatile int*>(failed + inst)) return;   // uniform over the cluster
     const int jl = core.my_col(I), il = core.my_row(I);
@@ -255,7 +255,7 @@ k_cluster_backward(const __grid_constant__ BwdVectors<T> B, const __grid_constan
     if (j >= 0) { B.xh[j] = xh; B.g_c[j] = g_c; }
     if (i >= 0) { B.yh[i] = yh; B.g_rl[i] = g_rl; B.g_ru[i] = g_ru; }
     if (core.dead) failed[inst] = 2;
-    cl_barrier();
+    core.leave(I);
 }
 
 // (x, y) of the instances insts[0, gridDim.y) from a checkpoint.
@@ -467,7 +467,7 @@ vajra_status run_unrolled_t(const vajra_lp* lps, const int64_t* d_roff, const Pa
     auto forward_cluster = [&](const ClusterClass& q, int steps, TF* ckpt, uint8_t* pm, uint8_t* dm, cudaStream_t s) -> vajra_status {
         const FwdVectors<TF> F{U.c.get(), U.cl.get(), U.cu.get(), U.rl.get(), U.ru.get(), U.x.get(), U.y.get(), step, n, m, ckpt, C, pm, dm};
         VJ_CUDA(launch_clusters(forward_kernel<TF>(q.threads), q.clusters, q.ctas, q.threads, q.smem, s, F, mats(TF{}),
-                                cl.d_insts.get() + q.first, d_roff, d_coff, steps, failed.get(), static_cast<uint32_t>(q.smem)));
+                                cl.d_insts.get() + q.first, d_roff, d_coff, steps, failed.get(), cl_launch(q.smem)));
         return VAJRA_OK;
     };
     // forward, with checkpoints
@@ -514,7 +514,7 @@ vajra_status run_unrolled_t(const vajra_lp* lps, const int64_t* d_roff, const Pa
                 VJ_TRY(forward_cluster(k, len, nullptr, U.pmask.get(), U.dmask.get(), ss));
                 const BwdVectors<TB> B{U.xh.get(), U.yh.get(), g_c.get(), g_rl.get(), g_ru.get(), step, n, m, U.pmask.get(), U.dmask.get()};
                 VJ_CUDA(launch_clusters(backward_kernel<TB>(k.threads), k.clusters, k.ctas, k.threads, k.smem, ss, B, mats(TB{}),
-                                        cl.d_insts.get() + k.first, d_roff, d_coff, len, failed.get(), static_cast<uint32_t>(k.smem)));
+                                        cl.d_insts.get() + k.first, d_roff, d_coff, len, failed.get(), cl_launch(k.smem)));
             }
         }
         if (clusters) VJ_TRY(side.join(st));

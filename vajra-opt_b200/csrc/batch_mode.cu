@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ BKktVectors V, const __grid_constant__ BMats<T> M,
                 const int* __restrict__ insts, const int64_t* __restrict__ roff, const int64_t* __restrict__ coff,
                 const __grid_constant__ BatchArrays S, const __grid_constant__ BControl cp0, double* part, ClControl* shared,
-                int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+                int K, long long budget, int max_chunks, ClLaunch L) {
     __shared__ double red[kBQ * kClWarps];
     __shared__ BInstance b;
     __shared__ BControl cp;
@@ -496,7 +496,7 @@ k_cluster_batch(const __grid_constant__ ClVectors<T> P, const __grid_constant__ 
     __syncthreads();
     BatchClusterControl<T> pol{P, V, S, inst, b, cp, red, part + static_cast<size_t>(cluster) * kClMaxCtas * kBQ};
     cl_run<T, NT>(P, mats, static_cast<int>(roff[inst]), static_cast<int>(coff[inst]), pol, shared + cluster, K, budget, max_chunks,
-                  smem_bytes);
+                  L);
 }
 
 // Before a launch: done = 1 in each path's array for the instances that it does not run.  `on`
@@ -1157,7 +1157,7 @@ static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_o
             VJ_CUDA(launch_clusters(batch_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, side.streams[q], P, kv,
                                     mats(tag), cl.d_insts.get() + k.first, d_roff.get(), d_coff.get(), Scl, c2,
                                     cl_part.get() + static_cast<size_t>(k.first) * kClMaxCtas * kBQ, cl_shared.get() + k.first, K,
-                                    static_cast<long long>(iters), static_cast<int>((iters + K - 1) / K), static_cast<uint32_t>(k.smem)));
+                                    static_cast<long long>(iters), static_cast<int>((iters + K - 1) / K), cl_launch(k.smem)));
         }
         return VAJRA_OK;
     };

@@ -12,6 +12,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cluster.cuh"
 #include "solver.cuh"
 
 namespace vajra {
@@ -304,6 +305,19 @@ bool pdl_enabled() {
         return !(e && std::strcmp(e, "0") == 0);
     }();
     return on;
+}
+
+int cluster_wait_tries() {
+    static const int tries = [] {
+        const char* v = std::getenv("VAJRA_CLUSTER_WAIT_TRIES");
+        if (v && *v) {
+            char* end = nullptr;
+            const long n = std::strtol(v, &end, 10);
+            if (end && *end == '\0' && n >= 0 && n <= kClWaitTries) return static_cast<int>(n);
+        }
+        return kClWaitTries;
+    }();
+    return tries;
 }
 
 void copy_out_vector(double* dst, const double* dev, int count, cudaStream_t st) {

@@ -22,6 +22,12 @@
 // its last read of x_bar; the same with the names exchanged.
 // Why each vector has its own mbarrier: a CTA that runs ahead sends at most one exchange ahead,
 // and that one goes to the other mbarrier, so bytes are never counted in the wrong phase.
+// Where a wait runs out, that thread waits, sends and arms no more (a second arrival could fall into a
+// phase that is not complete).  A CTA that no longer arms its mbarriers runs out in its other threads,
+// one that no longer sends makes its peers run out; each of them is at most one exchange ahead, so no
+// mbarrier sees a phase's arrivals twice.  Everybody goes through the remaining steps on garbage, but in
+// bounds and with the same decisions, and the kernel reports it.  At the end (ClCore::leave) the cluster then
+// stays for the copies still on their way, so that none outlives a CTA.
 // Row sums are formed exactly as the grouped-lane kernel forms them (G lanes a row, strided,
 // butterfly; rows longer than long_len by 256 threads), so results have the same bits.
 #pragma once
@@ -38,7 +44,18 @@ constexpr int kClMaxLong = 16;                 // rows summed by 256 threads tha
 constexpr int kClMaxCtas = 16;
 constexpr int kClRowWeight = 16;               // a row's share of the work beside its entries
 constexpr size_t kClSmemCap = 216 * 1024;      // dynamic shared memory a CTA may ask for
-constexpr int kClWaitTries = 1 << 20;          // bound of every mbarrier wait
+constexpr int kClWaitTries = 1 << 20;          // bound of every mbarrier wait, unless the environment sets it
+constexpr int kClDrainNaps = 2000;             // half microseconds that a failed cluster stays at its end
+
+// Tries of an mbarrier wait: kClWaitTries, or VAJRA_CLUSTER_WAIT_TRIES (read once).
+int cluster_wait_tries();
+
+// What a launch tells the kernel of its set-up.
+struct ClLaunch {
+    uint32_t smem_bytes;
+    int wait_tries;
+};
+inline ClLaunch cl_launch(size_t smem) { return {static_cast<uint32_t>(smem), cluster_wait_tries()}; }
 
 // One matrix of the LP: rows `rows`, indices minus idx_base are local.
 template <typename V>
@@ -152,6 +169,7 @@ struct ClInfo {                 // uniform over the CTA, in shared memory
     uint32_t expect_x, expect_y;         // what the peers send
     uint32_t top, end;                   // free dynamic shared memory
     int count;
+    int ran_out;                         // a wait ran out somewhere in the cluster (set by `leave`)
 };
 // Two entries of a task: the vector entries' places in shared memory (bytes) and the values.
 template <typename T> struct ClPair;
@@ -204,6 +222,7 @@ __device__ __noinline__ void cl_begin(const ClMat<V>& a, const ClMat<V>& at, uin
         I.expect_y = cl_bytes<T>(a.rows) - I.bytes_y;
         I.top = cl_y_offset<T>(at.rows) + cl_y_offset<T>(a.rows);
         I.end = bytes;
+        I.ran_out = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&I.bar_x)), "r"(ax) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&I.bar_y)), "r"(ay) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -430,14 +449,16 @@ struct ClCore {
     uint32_t size, rank;
     uint32_t peer_x, peer_y, peer_bar_x, peer_bar_y;   // thread t: my slices' places and the mbarriers in CTA t
     uint32_t par_x = 0, par_y = 0;
-    bool dead = false;          // a wait ran out: no further waiting
+    int tries;                  // bound of a wait (a kernel parameter: no register)
+    bool dead = false;          // a wait ran out: no further waiting, sending or arming
 
     __device__ __forceinline__ ClArray<T> xb() const { return ClArray<T>{0}; }
 
     // False when a slice does not fit into this CTA (uniform over the CTA).  A cluster barrier has
     // to follow before the first exchange.
-    __device__ __forceinline__ bool begin(const ClMat<V>& a, const ClMat<V>& at, uint32_t bytes, ClInfo& I) {
-        cl_begin<T, V>(a, at, bytes, I);
+    __device__ __forceinline__ bool begin(const ClMat<V>& a, const ClMat<V>& at, const ClLaunch& L, ClInfo& I) {
+        tries = L.wait_tries;
+        cl_begin<T, V>(a, at, L.smem_bytes, I);
         size = I.size;
         rank = I.rank;
         yf = ClArray<T>{cl_y_offset<T>(I.n)};
@@ -458,10 +479,11 @@ struct ClCore {
     __device__ __forceinline__ int my_col(const ClInfo& I) const { return tc.row >= 0 && (threadIdx.x & (tpr_c - 1)) == 0 ? I.cols.b0 + tc.row : -1; }
     __device__ __forceinline__ int my_row(const ClInfo& I) const { return tr.row >= 0 && (threadIdx.x & (tpr_r - 1)) == 0 ? I.rows.b0 + tr.row : -1; }
 
+    // Waits for the mbarrier's phase of that parity.
     __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
         if (dead) return;
 #pragma unroll 1
-        for (int t = 0; t < kClWaitTries; ++t) {
+        for (int t = 0; t < tries; ++t) {
             uint32_t ok;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
@@ -486,7 +508,7 @@ struct ClCore {
         const uint32_t bar = smem_addr(Y ? &I.bar_y : &I.bar_x);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (threadIdx.x < size) {
+        if (threadIdx.x < size && !dead) {
             if (threadIdx.x == rank) {
                 const uint32_t expect = (X ? I.expect_x : 0u) + (Y ? I.expect_y : 0u);
                 asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(expect) : "memory");
@@ -506,6 +528,22 @@ struct ClCore {
     __device__ __forceinline__ void exchange_y(ClInfo& I) { exchange<false, true>(I); }
     // Both at once, on y's mbarrier: only between two cluster barriers.
     __device__ __forceinline__ void exchange_both(ClInfo& I) { exchange<true, true>(I); }
+
+    // The end of a kernel, by all threads of the cluster, after the last exchange: no CTA may end
+    // while a peer still sends to it or a copy still reads its memory.  Where every wait was met,
+    // everything sent has arrived.
+    __device__ __forceinline__ void leave(ClInfo& I) {
+        if (dead)
+            for (uint32_t q = 0; q < size; ++q)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_map(smem_addr(&I.ran_out), q)), "r"(1) : "memory");
+        cl_barrier();
+        if (!*static_cast<volatile int*>(&I.ran_out)) return;
+        // Nobody sends any more, and nobody knows what is on its way (those phases were not armed): all stay
+        // for a millisecond, a thousand times as long as a copy takes.
+#pragma unroll 1
+        for (int t = 0; t < kClDrainNaps; ++t) __nanosleep(500);
+        cl_barrier();
+    }
 
     // The sum of my row against `vec`, valid in the row's owner.  All threads.
     __device__ __forceinline__ static T sum(const ClTask& task, int tpr, const ClMat<V>& mat, const ClSlice& s, ClArray<T> vec) {
@@ -599,13 +637,13 @@ __device__ __forceinline__ void cl_combine(const double* part, int ctas, double*
 // in global memory.  Returns false when a slice does not fit.
 template <typename T, int NT, class Pol>
 __device__ __forceinline__ bool cl_run(const ClVectors<T>& P, const ClMats<T>& M, int row0, int col0, Pol& pol,
-                                       ClControl* shared, int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+                                       ClControl* shared, int K, long long budget, int max_chunks, const ClLaunch& L) {
     __shared__ ClInfo I;
     __shared__ T hw[2 * kClWeights];
     __shared__ ClControl now;
     const int tid = threadIdx.x;
     ClCore<T, T> core;
-    const bool fits = core.begin(M.a, M.at, smem_bytes, I);
+    const bool fits = core.begin(M.a, M.at, L, I);
     for (int i = tid; i < I.m; i += NT) core.yf[i] = P.y[row0 + i];
     if (core.rank == 0) {
         if (tid == 0) now.wait_error = now.no_fit = now.restart = 0;
@@ -717,7 +755,7 @@ __device__ __forceinline__ bool cl_run(const ClVectors<T>& P, const ClMats<T>& M
     if (j >= 0) { P.x[j] = x; P.x0[j] = x0; }
     if (i >= 0) { P.y[i] = y; P.y0[i] = y0; }
     if (core.rank == 0) pol.finish();
-    cl_barrier();   // no CTA ends while a peer may still send to it
+    core.leave(I);
     return true;
 }
 

@@ -30,14 +30,14 @@ __device__ __forceinline__ void bmats_of(const BMats<T>& M, const int64_t* roff,
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 k_cluster_fit(const __grid_constant__ BMats<T> M, const int* __restrict__ insts, const int64_t* __restrict__ roff,
-              const int64_t* __restrict__ coff, int* __restrict__ nofit, uint32_t smem_bytes) {
+              const int64_t* __restrict__ coff, int* __restrict__ nofit, ClLaunch L) {
     __shared__ ClInfo I;
     __shared__ ClMats<T> mats;
     const int inst = insts[blockIdx.x / cl_size()];
     if (threadIdx.x == 0) bmats_of(M, roff, coff, inst, mats);
     __syncthreads();
     ClCore<T, T> core;
-    if (!core.begin(mats.a, mats.at, smem_bytes, I) && threadIdx.x == 0) nofit[inst] = 1;
+    if (!core.begin(mats.a, mats.at, L, I) && threadIdx.x == 0) nofit[inst] = 1;
 }
 
 // The instances that run on clusters, by cluster size and threads.
@@ -184,7 +184,7 @@ vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int
                 continue;
             }
             VJ_CUDA(launch_clusters(fit_kernel<T>(k.threads), k.clusters, k.ctas, k.threads, k.smem, st, M, out.d_insts.get() + k.first,
-                                    roff, coff, nofit.get(), static_cast<uint32_t>(k.smem)));
+                                    roff, coff, nofit.get(), cl_launch(k.smem)));
         }
         VJ_CUDA(cudaMemcpyAsync(h.data(), nofit.get(), sizeof(int) * count, cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));

@@ -614,35 +614,37 @@ template <typename T, int NT>
 __global__ void __launch_bounds__(NT, 1)
 k_cluster_halpern(const __grid_constant__ ClVectors<T> P, const __grid_constant__ KktVectors V,
                   const __grid_constant__ ClMats<T> M, const __grid_constant__ ControlParams cp0, HState* st, double* part,
-                  ClControl* shared, int K, long long budget, int max_chunks, uint32_t smem_bytes) {
+                  ClControl* shared, int K, long long budget, int max_chunks, ClLaunch L) {
     __shared__ double red[2 * kQ * kClWarps];
     __shared__ HState hs;
     __shared__ ControlParams cp;
     if (st->stop || st->phase != cp0.phase) return;   // uniform over the cluster
     if (threadIdx.x == 0) cp = cp0;
     HalpernControl<T> pol{P, V, st, hs, cp, red, part};
-    cl_run<T, NT>(P, M, 0, 0, pol, shared, K, budget, max_chunks, smem_bytes);
+    cl_run<T, NT>(P, M, 0, 0, pol, shared, K, budget, max_chunks, L);
 }
 
 // The power iteration of spectral_norm_fast (setup.cu) on one cluster: sst->spectral_norm after at
 // most max_iter rounds.  The set-up's loop launches five kernels a round, 1.9 ms of a small LP's
-// 2.6 ms of set-up; here a round is two row sums, two exchanges and a reduction.  `part`: 16 values.
+// 2.6 ms of set-up; here a round is two row sums, two exchanges and a reduction.  `part`: 2 x 16
+// values, used in turn, so that every CTA reads the same sums and ends in the same round even where
+// a wait ran out and nobody waits any more.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1)
 k_cluster_norm(const __grid_constant__ ClMats<double> M, int max_iter, double tol, SetupState* sst, double* part, ClControl* shared,
-               uint32_t smem_bytes) {
+               ClLaunch L) {
     __shared__ ClInfo I;
     __shared__ double red[kClWarps];
     __shared__ double sum;
     const int tid = threadIdx.x;
     ClCore<double, double> core;
-    if (!core.begin(M.a, M.at, smem_bytes, I) && tid == 0) shared->no_fit = 1;
+    if (!core.begin(M.a, M.at, L, I) && tid == 0) shared->no_fit = 1;
     for (int j = tid; j < I.n; j += NT) core.xb()[j] = 1.0 / sqrt(static_cast<double>(I.n));
     cl_barrier();
     if (*static_cast<volatile int*>(&shared->no_fit)) return;   // the host takes the set-up's loop
     const int jl = core.my_col(I), il = core.my_row(I);
     double lambda = 1.0, prev = 0.0, norm = 0.0;
-    bool done = false;   // uniform over the cluster: every CTA adds the same partials in the same order
+    bool done = false, odd = false;   // uniform over the cluster: every CTA adds the same partials in the same order
 #pragma unroll 1
     for (int it = 0; it < max_iter && !done; ++it) {
         const double w = core.row_sum(M.a, I);
@@ -650,21 +652,18 @@ k_cluster_norm(const __grid_constant__ ClMats<double> M, int max_iter, double to
         core.exchange_y(I);
         const double u = core.col_sum(M.at, I);
         double v[1] = {jl >= 0 ? u * u : 0.0};
-        cl_reduce<1, 0u>(v, red, part + core.rank);
+        double* here = part + (it & 1) * kClMaxCtas;
+        cl_reduce<1, 0u>(v, red, here + core.rank);
         cl_barrier();
         if (tid == 0) {
             double t = 0.0;
-            for (uint32_t r = 0; r < core.size; ++r) t += __ldcg(part + r);
+            for (uint32_t r = 0; r < core.size; ++r) t += __ldcg(here + r);
             sum = t;
         }
         __syncthreads();
         norm = sqrt(sum);
-        if (norm < 1e-15 || isnan(norm) || isinf(norm)) {
-            norm = lambda > 1e-6 ? sqrt(lambda) : 1e-3;
-            if (core.rank == 0 && tid == 0) sst->spectral_norm = norm;
-            cl_barrier();
-            return;
-        }
+        odd = norm < 1e-15 || isnan(norm) || isinf(norm);
+        if (odd) break;
         lambda = norm;
         done = it > 0 && fabs(norm - prev) <= tol * norm;
         prev = norm;
@@ -674,9 +673,9 @@ k_cluster_norm(const __grid_constant__ ClMats<double> M, int max_iter, double to
     if (core.dead) shared->wait_error = 1;
     if (core.rank == 0 && tid == 0) {
         const double s = sqrt(lambda);
-        sst->spectral_norm = s > 1e-12 ? s : 1e-6;
+        sst->spectral_norm = odd ? (lambda > 1e-6 ? s : 1e-3) : s > 1e-12 ? s : 1e-6;
     }
-    cl_barrier();   // no CTA ends while a peer may still send to it
+    core.leave(I);
 }
 
 // How an LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
@@ -952,7 +951,7 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
         ClControl hc{};
         VJ_CUDA(cudaMemsetAsync(cl_shared.get(), 0, sizeof(ClControl), st));
         VJ_CUDA(launch_clusters(cl64.threads == 256 ? &k_cluster_norm<256> : &k_cluster_norm<512>, 1, cl64.ctas, cl64.threads, cl64.smem,
-                                st, M, 100, 1e-5, sst.get(), cl_part.get(), cl_shared.get(), static_cast<uint32_t>(cl64.smem)));
+                                st, M, 100, 1e-5, sst.get(), cl_part.get(), cl_shared.get(), cl_launch(cl64.smem)));
         VJ_CUDA(cudaMemcpyAsync(&hss, sst.get(), sizeof(hss), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaMemcpyAsync(&hc, cl_shared.get(), sizeof(hc), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
@@ -1167,7 +1166,7 @@ vajra_status run_halpern(vajra_pdhg* h, vajra_result* r) {
         c2.phase = ph.phase;
         VJ_CUDA(launch_clusters(cluster_kernel<T>(plan.threads), 1, plan.ctas, plan.threads, plan.smem, st, P, kv, M, c2, S,
                                 cl_part.get(), cl_shared.get(), K, static_cast<long long>(budget), chunks,
-                                static_cast<uint32_t>(plan.smem)));
+                                cl_launch(plan.smem)));
         return VAJRA_OK;
     };
     const auto t_iter = Clock::now();

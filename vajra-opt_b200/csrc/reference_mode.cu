@@ -93,13 +93,13 @@ struct EpiRefPrimal {
 // whose loads from global memory do not coalesce.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1)
-k_cluster_reference(const __grid_constant__ ClMats<double> M, EpiRefDual D, EpiRefPrimal Q, int len, int* no_fit, uint32_t smem_bytes) {
+k_cluster_reference(const __grid_constant__ ClMats<double> M, EpiRefDual D, EpiRefPrimal Q, int len, int* no_fit, ClLaunch L) {
     RefState* st = D.st;
     if (st->stop) return;   // uniform over the cluster
     __shared__ ClInfo I;
     const int tid = threadIdx.x;
     ClCore<double, double> core;
-    if (!core.begin(M.a, M.at, smem_bytes, I) && tid == 0) *no_fit = 1;
+    if (!core.begin(M.a, M.at, L, I) && tid == 0) *no_fit = 1;
     auto dropped = [](double v) { return fabs(v) <= kZeroDrop ? 0.0 : v; };
     for (int j = tid; j < I.n; j += NT) core.xb()[j] = dropped(Q.xb[j]);
     cl_barrier();
@@ -137,8 +137,8 @@ k_cluster_reference(const __grid_constant__ ClMats<double> M, EpiRefDual D, EpiR
         atomicMin(&st->stop_iter, base + bad);
         flag_nan_state(st);
     }
-    if (core.dead) *no_fit = 2;
-    cl_barrier();   // no CTA ends while a peer may still send to it
+    if (core.dead) { *no_fit = 2; st->stop = 1; }
+    core.leave(I);
 }
 
 struct EpiStoreRef {
@@ -388,7 +388,7 @@ vajra_status run_reference(vajra_pdhg* h, vajra_result* r) {
         return launch_clusters(cluster_kernel(cl_threads), 1, cl_ctas, cl_threads, kClSmemCap, st, mats,
                                EpiRefDual{p.row_lower.get(), p.row_upper.get(), y.get(), S, 0},
                                EpiRefPrimal{p.c.get(), p.col_lower.get(), p.col_upper.get(), x.get(), xb.get(), S, 0}, len,
-                               no_fit.get(), static_cast<uint32_t>(kClSmemCap));
+                               no_fit.get(), cl_launch(kClSmemCap));
     };
     plan(1);
     while (cl_ctas) {   // no iterations: only whether the slices fit; a wider cluster where they do not

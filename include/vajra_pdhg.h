@@ -104,7 +104,8 @@ typedef struct vajra_opts {
     double gap_tolerance;       /* REFERENCE: relative gap ("gap_tolerance")             */
     double time_limit;          /* seconds (Options::time_limit); HALPERN checks it between
                                    launches: after every check, or for LPs that run on a
-                                   thread-block cluster after up to 16 checks, then what fits */
+                                   thread-block cluster after the first check and then after
+                                   as many as fit in the time left at the rate so far     */
     int64_t iteration_limit;    /* Options::iteration_limit                              */
     int32_t check_frequency;    /* REFERENCE: "check_frequency" (100); HALPERN: KKT /
                                    restart evaluation interval (64)                      */

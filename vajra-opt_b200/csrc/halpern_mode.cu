@@ -856,12 +856,12 @@ std::map<TuneKey, TuneEntry> g_tune_cache;
 
 }  // namespace
 
-// Chunks of the next launch of several: a first short launch, then what fits in the time left at
-// the rate measured so far, all that a launch may run where there is no limit to speak of.
+// Chunks of the next launch of a cluster: one, then what fits in the time left at the rate measured so
+// far; all that a launch may run where there is no limit to speak of.
 static int64_t launch_chunks(int64_t ran, double seconds, double left) {
-    constexpr int64_t kFirst = 16, kMost = 4096;
+    constexpr int64_t kMost = 4096;
     if (left > 1e9) return kMost;
-    if (ran == 0 || seconds <= 0.0) return kFirst;
+    if (ran == 0 || seconds <= 0.0) return 1;
     const double fit = left * static_cast<double>(ran) / seconds;
     return fit >= static_cast<double>(kMost) ? kMost : (fit < 1.0 ? 1 : static_cast<int64_t>(fit));
 }

@@ -38,7 +38,8 @@ enum {
     VAJRA_ERR_NO_DEVICE = 2,
     VAJRA_ERR_CUDA = 3,
     VAJRA_ERR_OUT_OF_MEMORY = 4,
-    VAJRA_ERR_WAIT_TIMEOUT = 5,  /* reserved: no entry point waits on the device today      */
+    VAJRA_ERR_WAIT_TIMEOUT = 5,  /* a bounded wait between the blocks of a thread-block cluster
+                                    ran out (LPs small enough for one); the context stays usable */
     VAJRA_ERR_INTERNAL = 6
 };
 
@@ -136,8 +137,9 @@ typedef struct vajra_opts {
                                    -3 sliced ELL (degree-ordered LPs; else the row-block
                                    kernel), -4 sliced ELL with the first vector entries in
                                    shared memory, 1..32 lanes per row (1, 2, 4, 8, 16, 32).
-                                   The batched solver: 0 as above, -3 sliced ELL over windows
-                                   of 256 rows, other values keep it off the clusters         */
+                                   The batched solver: 0 for both matrices as above; -3 for
+                                   either, sliced ELL over windows of 256 rows for both;
+                                   another value only keeps its instances off the clusters    */
     int32_t spmv_shape_at;      /* the same for the A^T y SpMV                           */
     double mixed_reflection;    /* MIXED: reflection coefficient of the FP32 phase once its
                                    relative KKT is within 10x of mixed_switch_tolerance (0.8);

@@ -14,8 +14,9 @@
 // (same rules as the single-LP solver), and one thread counts the active instances.  A pass
 // is one CUDA graph whose WHILE node repeats the chunk (iterations plus check) on the device
 // while an instance is active, up to a chunk budget per launch; the host reads the
-// counters once per launch.  No kernel waits on another kernel, so nothing in this path can
-// spin, and the loop's chunk budget ends every launch.
+// counters once per launch.  Instances that fit a thread-block cluster run on one each instead, where
+// that is the faster (cluster.cuh), on streams beside the packed rest.  No kernel waits on another
+// kernel, the waits between the CTAs of a cluster are bounded, and the chunk budget ends every launch.
 //
 // Scaling is per instance: Ruiz and Pock-Chambolle factors are local to a row or column, and
 // each instance ends its Ruiz passes on its own stopping test, so every instance is scaled

@@ -453,7 +453,7 @@ const char* vajra_status_string(vajra_status s) {
         case VAJRA_ERR_NO_DEVICE: return "no CUDA device";
         case VAJRA_ERR_CUDA: return "CUDA error";
         case VAJRA_ERR_OUT_OF_MEMORY: return "out of device memory";
-        case VAJRA_ERR_WAIT_TIMEOUT: return "device wait timed out (reserved)";
+        case VAJRA_ERR_WAIT_TIMEOUT: return "device wait timed out";
         case VAJRA_ERR_INTERNAL: return "internal error";
         default: return "unknown status";
     }

@@ -52,12 +52,13 @@ inline vajra_status pack_lps(int count, const vajra_lp* lps, PackedHost& P) {
         const vajra_lp& L = lps[i];
         const int64_t c0 = P.coff[i], r0 = P.roff[i], z0 = P.zoff[i];
         for (int j = 0; j < L.num_cols; ++j) P.col_ptr[c0 + j] = z0 + L.col_ptr[j];
-        bool in_range = true;   // a cluster gathers from shared memory by these
+        uint32_t outside = 0;   // a cluster gathers from shared memory by these (no branch: the loop is vectorised)
         for (int64_t k = 0; k < L.nnz; ++k) {
-            in_range = in_range && static_cast<uint32_t>(L.row_idx[k]) < static_cast<uint32_t>(L.num_rows);
-            P.row_idx[z0 + k] = static_cast<int32_t>(r0 + L.row_idx[k]);
+            const uint32_t r = static_cast<uint32_t>(L.row_idx[k]);
+            outside |= r >= static_cast<uint32_t>(L.num_rows) ? 1u : 0u;
+            P.row_idx[z0 + k] = static_cast<int32_t>(static_cast<uint32_t>(r0) + r);
         }
-        if (!in_range) { set_error("row index out of range in instance %d", i); return VAJRA_ERR_INVALID_ARGUMENT; }
+        if (outside) { set_error("row index out of range in instance %d", i); return VAJRA_ERR_INVALID_ARGUMENT; }
         if (L.nnz) std::memcpy(&P.values[z0], L.values, sizeof(double) * L.nnz);
         if (L.num_cols) {
             std::memcpy(&P.c[c0], L.c, sizeof(double) * L.num_cols);

@@ -116,13 +116,23 @@ struct EpiStore {
 // each row's thread adds the row's part of the tile in storage order, so a row's sum is the chain of
 // additions of one thread whatever its length.  (A thread a row that also loaded the row's entries:
 // loads 4 to 20 entries apart across a warp, 3 to 5 times the traffic.  100,003 x 250,007, 2M
-// entries, FP64: 56 us for A x and A^T y with their proxes, 30 us now.)
-constexpr int kSeqTile = 2048;
-template <typename V, bool ZERO_DROP, class Epi>
+// entries, FP64: 56 us for A x and A^T y with their proxes, 30 us so.)
+// Chains of rows in one CTA that are longer than a tile follow one another, so few rows get a CTA each
+// (launch_spmv_exact): 300 rows of 5,000 entries 1,183 us with a thread a row, 1,344 with 32 rows
+// a CTA, 52 with one.  CTAs of kThreads rows are the many-row case: the tile is half as large, which leaves
+// the L1 more for the gathers (1M rows of 16 entries 120 -> 116 us, of 8 51 -> 47), and up to four
+// entries a row a thread loads its row itself (1M rows of 4: 24.6 us staged, 21.2 so; 19.5 in a
+// kernel without the tile).  That path in the other kernel cost a PDHG step 4 % of its time.
+constexpr int kSeqTile = 2048;        // products a CTA stages,
+constexpr int kSeqTileFull = 1024;    // and one of kThreads rows
+constexpr int kSeqDirect = 4;         // entries a row up to which a thread of those loads them itself
+// FULL: CTAs of kThreads rows.
+template <typename V, bool ZERO_DROP, class Epi, bool FULL>
 __global__ void __launch_bounds__(kThreads)
 k_spmv_seq(int rows, int R, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
            const V* __restrict__ val, const V* __restrict__ x, Epi epi) {
-    __shared__ V prod[kSeqTile];
+    constexpr int TILE = FULL ? kSeqTileFull : kSeqTile;
+    __shared__ V prod[TILE];
     pdl_enter();
     if (!epi.active()) return;
     const int tid = threadIdx.x, r0 = blockIdx.x * R, r1 = r0 + R < rows ? r0 + R : rows;
@@ -137,8 +147,19 @@ k_spmv_seq(int rows, int R, const int64_t* __restrict__ ptr, const int32_t* __re
         e = ptr[row + 1];
     }
     V sum = V(0);
-    for (int64_t t0 = e0; t0 < e1; t0 += kSeqTile) {
-        const int n = static_cast<int>(e1 - t0 < kSeqTile ? e1 - t0 : kSeqTile);
+    if constexpr (FULL) {
+        if (e1 - e0 <= kSeqDirect * kThreads) {
+            for (int64_t k = s; k < e; ++k) {
+                const V xv = x[idx[k]];
+                if (ZERO_DROP && fabs(xv) <= V(kZeroDrop)) continue;
+                sum = rn_add(sum, rn_mul(val[k], xv));
+            }
+            if (mine) epi_fin(epi, row, sum, pre, 0);
+            return;
+        }
+    }
+    for (int64_t t0 = e0; t0 < e1; t0 += TILE) {
+        const int n = static_cast<int>(e1 - t0 < TILE ? e1 - t0 : TILE);
 #pragma unroll 4
         for (int k = tid; k < n; k += kThreads) {
             const V xv = x[ld_stream(idx + t0 + k)];
@@ -860,8 +881,10 @@ inline void launch_spmv_exact(const CsrView& a, const V* val, const V* x, Epi ep
     if (a.rows <= 0) return;
     // fewer rows a CTA where 256 would leave an SM fewer than eight CTAs to overlap
     int R = kThreads;
-    while (R > 32 && (a.rows + R - 1) / R < 8 * sm_count()) R /= 2;
-    launch_chained(k_spmv_seq<V, ZERO_DROP, Epi>, (a.rows + R - 1) / R, kThreads, 0, st, a.rows, R, a.ptr, a.idx, val, x, epi);
+    while (R > 1 && (a.rows + R - 1) / R < 8 * sm_count()) R /= 2;
+    const int blocks = (a.rows + R - 1) / R;
+    auto* kernel = R == kThreads ? &k_spmv_seq<V, ZERO_DROP, Epi, true> : &k_spmv_seq<V, ZERO_DROP, Epi, false>;
+    launch_chained(kernel, blocks, kThreads, 0, st, a.rows, R, a.ptr, a.idx, val, x, epi);
     note_launch();
 }
 

@@ -28,9 +28,9 @@ calls = {
     "reference": lambda: V.solve(several, algorithm=V.ALGO_REFERENCE, iteration_limit=500),
     "batch64": lambda: V.solve_batch(batch, precision=V.PREC_FP64),
     "batch32": lambda: V.solve_batch(batch),
-    "unrolled64": lambda: unrolled(batch, ones, iterations=30, precision=PREC_FP64),
-    "unrolled_mixed": lambda: unrolled(batch, ones, iterations=30, precision=PREC_MIXED),
-    "unrolled32": lambda: unrolled(batch, ones, iterations=30, precision=PREC_FP32),
+    "unrolled64": lambda: unrolled(batch, ones, iterations=1000, precision=PREC_FP64),
+    "unrolled_mixed": lambda: unrolled(batch, ones, iterations=1000, precision=PREC_MIXED),
+    "unrolled32": lambda: unrolled(batch, ones, iterations=1000, precision=PREC_FP32),
 }
 for _ in range(2):
     for name, call in calls.items():

@@ -383,6 +383,12 @@ void values_of(Prepared& p, const T** csr, const T** csc) {
     }
 }
 
+// Clusters of a launch where there are more of them than the GPU holds at once.  They come in rounds, and in one
+// stream each launch waits for the last round of the one before, nearly empty; launches of several
+// streams fill each other's.  32 LPs of 1000 x 3000, three rounds: 39.0 ms in one launch, 32.5 in launches of
+// 8, 32.8 of 4.  A stream costs about 0.1 ms of host time, so there are at most 8 for clusters of a size.
+constexpr int kAtOnce = 8;
+
 template <typename TF, typename TB>
 vajra_status run_unrolled_t(const vajra_lp* lps, const int64_t* d_roff, const PackedHost& P, const vajra_unrolled_opts& o, Prepared& p, const DeviceLp& lp,
                             const int* row_inst, const int* col_inst, const int64_t* d_coff, const double* step,
@@ -443,20 +449,27 @@ vajra_status run_unrolled_t(const vajra_lp* lps, const int64_t* d_roff, const Pa
     DeviceBuffer<int> failed;
     VJ_TRY(failed.alloc(count));
     VJ_CUDA(cudaMemsetAsync(failed.get(), 0, sizeof(int) * count, st));
+    bool rounds = false;   // more clusters than the GPU holds at once
     if (clusters) {
-        VJ_TRY(plan_clusters(lps, count, std::vector<int>(count, 1), 0, mats(TF{}), d_roff, d_coff, cl,
+        // A step takes 20 to 25 us packed, forward, recomputed and back, and 42 ps an entry (forward alone 5 us and
+        // 13 ps); on clusters three (one) of 0.8 to 0.9 of a solver's iteration, which has checks.
+        VJ_TRY(plan_clusters(lps, count, std::vector<int>(count, 1), mats(TF{}), d_roff, d_coff, cl,
+                             [&](const ClusterLoad& L) {
+                                 rounds = L.at_once > 1.0;
+                                 const double e = 1e-6 * static_cast<double>(L.entries);
+                                 const double packed = want_grad ? 17.0 + 42.0 * e : 5.0 + 13.0 * e;
+                                 const double here = (want_grad ? 3.0 : 1.0) * 0.9 * L.us;
+                                 const double start = 250.0 + 100.0 * (rounds ? std::min(16, count / kAtOnce + 1) : 1);
+                                 return L.outside == 0 && start + K * here <= K * packed;
+                             },
                              [](const ClusterClass& q) {
                                  cudaError_t e = prepare_clusters(forward_kernel<TF>(q.threads), q.ctas, q.threads, q.smem);
                                  return e != cudaSuccess ? e : prepare_clusters(backward_kernel<TB>(q.threads), q.ctas, q.threads, q.smem);
                              }, st));
         clusters = static_cast<int>(cl.insts.size()) == count;
-        // At most kAtOnce clusters a stream: the GPU holds 15 clusters of 8 CTAs, and 32 of them in one
-        // launch after another would take three rounds each, the last one nearly empty; launches
-        // of several streams fill each other's rounds.
-        constexpr int kAtOnce = 4;
         std::vector<ClusterClass> parts;
         for (const ClusterClass& q : cl.classes) {
-            const int cut = std::max(kAtOnce, (q.clusters + 15) / 16);
+            const int cut = rounds ? std::max(kAtOnce, (q.clusters + 7) / 8) : q.clusters;
             for (int f = 0; f < q.clusters; f += cut) {
                 parts.push_back(q);
                 parts.back().first = q.first + f;

@@ -770,8 +770,14 @@ auto batch_kernel(int threads) -> decltype(&k_cluster_batch<T, 256>) {
 // takes the small instances along at no worse a rate than clusters beside it do (256 LPs of 100 to
 // 20,000 rows: 477 ms packed, 526 ms with the small ones on clusters).  Below it an iteration costs
 // its launches (9 to 20 us) and the small instances finish sooner by themselves (96 LPs of 100 to
-// 2,000 rows: 43.8 -> 30.6 ms).
+// 2,000 rows: 43.8 -> 30.6 ms), as long as the clusters themselves are the faster (rates: cluster_us).
+// 200 LPs of 1,000 to 2,000 rows, FP64, 2,048 iterations: 256 ms on clusters, 195 packed.
 constexpr int64_t kClBatchEntries = int64_t(4) << 20;
+inline bool clusters_pay(const ClusterLoad& L, size_t t, bool windows) {
+    const double entries = 1e-6 * static_cast<double>(L.entries);
+    const double packed = t == 4 ? 8.0 + 6.5 * entries : windows ? 5.0 + 9.0 * entries : 6.5 + 9.5 * entries;
+    return L.outside <= kClBatchEntries && L.us <= packed;
+}
 
 }  // namespace
 
@@ -997,12 +1003,19 @@ static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_o
                         p.a.group, p.at.group, p.a.long_len, p.at.long_len};
     };
     ClusterBatch clus32, clus64;
-    bool all_fit = true;
+    bool no_packed = true;   // every instance starts on a cluster
     const bool may_cluster = o.spmv_shape_a == 0 && o.spmv_shape_at == 0;   // as for a single LP
     for (int i = 0; i < count; ++i) {
         clus32.least.push_back(may_cluster && mixed ? least_cluster<float>(lps[i], p.a.group, p.at.group, 1) : 0);
         clus64.least.push_back(may_cluster ? least_cluster<double>(lps[i], p.a.group, p.at.group, 1) : 0);
-        all_fit = all_fit && clus64.least[i] > 0;   // FP32 vectors are smaller
+        no_packed = no_packed && clus64.least[i] > 0;   // FP32 vectors are smaller
+    }
+    const bool has_windows = p.a.win_off != nullptr;
+    if (no_packed) {
+        const std::vector<int> all(count, 1);
+        const int ga = p.a.group, gat = p.at.group;
+        no_packed = clusters_pay(cluster_load(8, lps, all, size_clusters<double>(lps, count, all, ga, gat, clus64)), 8, has_windows) &&
+                    (!mixed || clusters_pay(cluster_load(4, lps, all, size_clusters<float>(lps, count, all, ga, gat, clus32)), 4, false));
     }
     DeviceBuffer<double> cl_part;
     DeviceBuffer<ClControl> cl_shared;
@@ -1016,7 +1029,7 @@ static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_o
     CsrView a = p.a, at = p.at;
     if (fixed_windows) {
         a.group = at.group = kSellWin;
-    } else if (o.autotune && !all_fit) {
+    } else if (o.autotune && !no_packed) {
         cudaEvent_t e0, e1;
         VJ_CUDA(cudaEventCreate(&e0));
         VJ_CUDA(cudaEventCreate(&e1));
@@ -1186,7 +1199,8 @@ static vajra_status run_batch_once(int count, const vajra_lp* lps, const vajra_o
             VJ_CUDA(cudaMemcpyAsync(status.data(), S.status, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
             VJ_CUDA(cudaStreamSynchronize(st));
             for (int i = 0; i < count; ++i) open[i] = status[i] == 0 ? 1 : 0;
-            VJ_TRY(plan_clusters(lps, count, open, kClBatchEntries, mats(tag), d_roff.get(), d_coff.get(), cl,
+            VJ_TRY(plan_clusters(lps, count, open, mats(tag), d_roff.get(), d_coff.get(), cl,
+                                 [&](const ClusterLoad& L) { return clusters_pay(L, sizeof(T), has_windows); },
                                  [](const ClusterClass& q) {
                                      return prepare_clusters(batch_kernel<T>(q.threads), q.ctas, q.threads, q.smem);
                                  }, st));

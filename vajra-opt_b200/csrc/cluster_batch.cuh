@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "cluster.cuh"
@@ -107,40 +108,88 @@ int least_cluster(const vajra_lp& L, int group_a, int group_at, int from) {
     return 0;
 }
 
-// Plans the instances with open[i] != 0 for a launch, unless those that no cluster holds have more
-// than `most_outside` entries.  A plan that leaves half of the SMs idle gets clusters of twice the
-// size, as far as their CTAs keep 512 entries.  `prepare`: what a class's launch needs (an error:
-// there is no such cluster on this device).
-template <typename T, class Prepare>
-vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, int64_t most_outside, const BMats<T>& M,
-                           const int64_t* roff, const int64_t* coff, ClusterBatch& out, Prepare prepare, cudaStream_t st) {
+// CTAs of the cluster of every instance with open[i] != 0, 0: none.  A plan that leaves half of the SMs
+// idle gets clusters of twice the size, as far as their CTAs keep 512 entries.
+template <typename T>
+std::vector<int> size_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, int group_a, int group_at, ClusterBatch& out) {
+    out.most.resize(count, kClMaxCtas);
+    std::vector<int> ctas(count);
+    int64_t sms_used = 0;
+    for (int i = 0; i < count; ++i) {
+        ctas[i] = open[i] ? out.least[i] : 0;
+        sms_used += ctas[i];
+    }
+    while (sms_used > 0 && 2 * sms_used <= sm_count()) {
+        int64_t used = 0;
+        for (int i = 0; i < count; ++i) {
+            if (ctas[i] > 0 && ctas[i] < out.most[i] && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) &&
+                cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, group_a, group_at, 2 * ctas[i], 512))
+                ctas[i] *= 2;
+            used += ctas[i];
+        }
+        if (used == sms_used) break;
+        sms_used = used;
+    }
+    return ctas;
+}
+
+// Whether clusters are the faster way for a plan is estimated from measured rates (B200; batches of 1 to 1,024
+// equal LPs of 60 to 3,000 rows, 20 entries a row; us an iteration, checks included).  A cluster on 1, 4, 8,
+// 16 CTAs of 4,000, 3,000, 2,500, 2,500 entries: 3.8, 4.5, 4.3, 5.3 in FP64, 2.3, 2.9, 2.7, 3.2 in
+// FP32; the device holds 148, about 34, 15 and 7 of them, and more of them come one after another.  An
+// entry costs a full device 7, 11.5, 15, 20 ps so (FP32: 4, 7.5, 10, 12), the packed iteration 9
+// over windows, 9.5 to 12 in lane groups (6.5) beside its 5 to 8 us of launches.
+inline double cluster_us(size_t t, int ctas, int64_t nnz) {
+    const double entries = static_cast<double>(nnz) / ctas;
+    const double step = ctas == 1 ? 0.1 : ctas <= 4 ? 1.65 : ctas == 8 ? 1.9 : 2.95;
+    return t == 8 ? step + 0.95e-3 * entries : (ctas == 1 ? 0.1 : 0.7 * step) + 0.54e-3 * entries;
+}
+struct ClusterLoad {
+    double us = 0.0;        // an iteration of all clusters
+    double at_once = 0.0;   // the share of the device that they take together, 1: all of it
+    int64_t entries = 0, outside = 0;   // of open instances on clusters, and of the others
+};
+inline ClusterLoad cluster_load(size_t t, const vajra_lp* lps, const std::vector<int>& open, const std::vector<int>& ctas) {
+    ClusterLoad L;
+    double sum = 0.0, longest = 0.0, widths[5] = {0, 0, 0, 0, 0}, counts[5] = {0, 0, 0, 0, 0}, sums[5] = {0, 0, 0, 0, 0};
+    for (size_t i = 0; i < ctas.size(); ++i) {
+        if (!open[i]) continue;
+        if (!ctas[i]) { L.outside += lps[i].nnz; continue; }
+        int k = 0;
+        while ((1 << k) < ctas[i]) ++k;
+        widths[k] = k == 0 ? sm_count() : std::max(1.0, std::floor(0.82 * sm_count() / ctas[i]));   // clusters the device holds
+        const double us = cluster_us(t, ctas[i], lps[i].nnz);
+        L.entries += lps[i].nnz;
+        L.at_once += 1.0 / widths[k];
+        sum += us / widths[k];
+        longest = std::max(longest, us);
+        counts[k] += 1.0;
+        sums[k] += us;
+    }
+    if (L.at_once <= 1.0) { L.us = longest; return L; }
+    L.us = sum + 0.5 * longest;
+    for (int k = 0; k < 5; ++k)   // equal clusters leave their last round half empty
+        if (counts[k] > 0.0) L.us = std::max(L.us, std::ceil(counts[k] / widths[k]) * sums[k] / counts[k]);
+    return L;
+}
+
+// Plans the instances with open[i] != 0 for a launch, if `pays` says so of the clusters' load.  `prepare`: what a
+// class's launch needs (an error: there is no such cluster on this device).
+template <typename T, class Pays, class Prepare>
+vajra_status plan_clusters(const vajra_lp* lps, int count, const std::vector<int>& open, const BMats<T>& M, const int64_t* roff,
+                           const int64_t* coff, ClusterBatch& out, Pays pays, Prepare prepare, cudaStream_t st) {
     DeviceBuffer<int> nofit;
     VJ_TRY(nofit.alloc(count));
     VJ_TRY(out.d_insts.alloc(count));
     VJ_TRY(out.d_on.alloc(count));
-    std::vector<int> ctas(count), threads(count), on(count), h(count);
-    out.most.resize(count, kClMaxCtas);
+    std::vector<int> threads(count), on(count), h(count);
     auto fits = [&](int i, int c, int t) {
         return cl_fits(sizeof(T), lps[i].num_rows, lps[i].num_cols, lps[i].nnz, M.group_a, M.group_at, c, t);
     };
     for (bool again = true; again;) {
         again = false;
-        int64_t outside = 0, sms_used = 0;
-        for (int i = 0; i < count; ++i) if (open[i] && !out.least[i]) outside += lps[i].nnz;
-        for (int i = 0; i < count; ++i) {
-            ctas[i] = open[i] && outside <= most_outside ? out.least[i] : 0;
-            sms_used += ctas[i];
-        }
-        while (sms_used > 0 && 2 * sms_used <= sm_count()) {
-            int64_t used = 0;
-            for (int i = 0; i < count; ++i) {
-                if (ctas[i] > 0 && ctas[i] < out.most[i] && lps[i].nnz > 1024 * static_cast<int64_t>(ctas[i]) && fits(i, 2 * ctas[i], 512))
-                    ctas[i] *= 2;
-                used += ctas[i];
-            }
-            if (used == sms_used) break;
-            sms_used = used;
-        }
+        std::vector<int> ctas = size_clusters<T>(lps, count, open, M.group_a, M.group_at, out);
+        if (!pays(cluster_load(sizeof(T), lps, open, ctas))) ctas.assign(count, 0);
         for (int i = 0; i < count; ++i)
             threads[i] = ctas[i] && fits(i, ctas[i], 256) && lps[i].nnz <= 2048 * static_cast<int64_t>(ctas[i]) ? 256 : 512;
         out.classes.clear();

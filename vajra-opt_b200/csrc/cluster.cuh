@@ -803,4 +803,28 @@ inline cudaError_t prepare_clusters(void (*kernel)(Params...), int ctas, int thr
     return e != cudaSuccess ? e : fit >= 1 ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
+// How a single LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
+struct ClusterPlan { int ctas = 0, threads = 0; size_t smem = 0; };
+
+// The smallest cluster whose CTAs have at most 256 rows and columns and about 1,000 entries of
+// each matrix, else 16 CTAs of up to 512.  Fewer CTAs exchange faster (0.6 us for 8, 0.8 us for
+// 16), more share the row sums; 256 threads pass a CTA's barriers faster than 512.  Microseconds
+// an iteration (FP32 / FP64; two launches an iteration: 5.5 to 6.8), checks included: 60 x 150 on
+// 1 CTA 1.2 / 1.3, on 4 1.7 / 1.7; 301 x 807 on 4 CTAs 1.9 / 2.1, on 8 1.9 / 2.1; 2000 x 5000 on
+// 16 CTAs of 512 threads 3.4 / 4.9; 5000 x 12000 (1,024 threads) 8.4 against 7.2, which is why the
+// line lies at 512.  Every thread forms at most kClMaxChains chains of a row.
+// `from`: CTAs it has at least.  `prepare(ctas, threads)`: what a launch needs (an error: there is
+// no such cluster on this device).
+template <class Prepare>
+inline ClusterPlan plan_one_cluster(size_t t, int64_t m, int64_t n, int64_t nnz, int group_a, int group_at, int from, Prepare prepare) {
+    for (int ctas = from; ctas <= kClMaxCtas; ctas *= 2) {
+        const int threads = cl_fits(t, m, n, nnz, group_a, group_at, ctas, 256) ? 256 : 512;
+        if (!cl_fits(t, m, n, nnz, group_a, group_at, ctas, threads)) continue;
+        if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
+        if (prepare(ctas, threads) != cudaSuccess) { cudaGetLastError(); continue; }
+        return ClusterPlan{ctas, threads, kClSmemCap};   // all of it: slices may be uneven
+    }
+    return {};
+}
+
 }  // namespace vajra

@@ -678,35 +678,18 @@ k_cluster_norm(const __grid_constant__ ClMats<double> M, int max_iter, double to
     core.leave(I);
 }
 
-// How an LP is laid over a cluster: CTAs (0: it does not go there), threads, shared memory.
-struct ClusterPlan { int ctas = 0, threads = 0; size_t smem = 0; };
-
 template <typename T>
 auto cluster_kernel(int threads) -> decltype(&k_cluster_halpern<T, 256>) {
     return threads == 256 ? &k_cluster_halpern<T, 256> : &k_cluster_halpern<T, 512>;
 }
 
-// The smallest cluster whose CTAs have at most 256 rows and columns and about 1,000 entries of
-// each matrix, else 16 CTAs of up to 512.  Fewer CTAs exchange faster (0.6 us for 8, 0.8 us for
-// 16), more share the row sums; 256 threads pass a CTA's barriers faster than 512.  Microseconds
-// an iteration (FP32 / FP64; two launches an iteration: 5.5 to 6.8), checks included: 60 x 150 on
-// 1 CTA 1.2 / 1.3, on 4 1.7 / 1.7; 301 x 807 on 4 CTAs 1.9 / 2.1, on 8 1.9 / 2.1; 2000 x 5000 on
-// 16 CTAs of 512 threads 3.4 / 4.9; 5000 x 12000 (1,024 threads) 8.4 against 7.2, which is why the
-// line lies at 512.  Every thread forms at most kClMaxChains chains of a row.
-// `from`: CTAs it has at least.
 template <typename T>
 ClusterPlan plan_cluster(const CsrView& a, const CsrView& at, int64_t nnz, int from) {
-    for (int ctas = from; ctas <= kClMaxCtas; ctas *= 2) {
-        const int threads = cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, 256) ? 256 : 512;
-        if (!cl_fits(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, ctas, threads)) continue;
-        if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
-        cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
-        if (sizeof(T) == 8 && e == cudaSuccess)
-            e = prepare_clusters(threads == 256 ? &k_cluster_norm<256> : &k_cluster_norm<512>, ctas, threads, kClSmemCap);
-        if (e != cudaSuccess) { cudaGetLastError(); continue; }   // no such cluster on this device
-        return ClusterPlan{ctas, threads, kClSmemCap};   // all of it: slices may be uneven
-    }
-    return {};
+    return plan_one_cluster(sizeof(T), a.rows, at.rows, nnz, a.group, at.group, from, [](int ctas, int threads) {
+        const cudaError_t e = prepare_clusters(cluster_kernel<T>(threads), ctas, threads, kClSmemCap);
+        if (sizeof(T) != 8 || e != cudaSuccess) return e;
+        return prepare_clusters(threads == 256 ? &k_cluster_norm<256> : &k_cluster_norm<512>, ctas, threads, kClSmemCap);
+    });
 }
 
 struct CheckBuffers {

@@ -364,9 +364,8 @@ vajra_status run_reference(vajra_pdhg* h, vajra_result* r) {
     const double tol = o.tolerance, gap_tol = o.gap_tolerance;
     const int mx = m > n ? m : n;
 
-    // Small LPs: the iterations of a chunk in one launch, on the smallest cluster that holds the LP
-    // (lines as in halpern_mode.cu).
-    int cl_ctas = 0, cl_threads = 0;
+    // Small LPs: the iterations of a chunk in one launch, on a cluster.
+    ClusterPlan cl;
     DeviceBuffer<int> no_fit;
     VJ_TRY(no_fit.alloc(1));
     VJ_CUDA(cudaMemsetAsync(no_fit.get(), 0, sizeof(int), st));
@@ -374,35 +373,29 @@ vajra_status run_reference(vajra_pdhg* h, vajra_result* r) {
                               ClMat<double>{n, lp.col_ptr.get(), lp.row_idx.get(), p.csc_val.get(), 0, 1, int64_t(1) << 30}};
     auto cluster_kernel = [](int threads) { return threads == 256 ? &k_cluster_reference<256> : &k_cluster_reference<512>; };
     auto plan = [&](int from) {
-        cl_ctas = 0;
-        for (int ctas = from; ctas <= kClMaxCtas && !cl_ctas; ctas *= 2) {
-            const int threads = cl_fits(8, m, n, nnz, 1, 1, ctas, 256) ? 256 : 512;
-            if (!cl_fits(8, m, n, nnz, 1, 1, ctas, threads)) continue;
-            if (ctas < kClMaxCtas && (threads > 256 || nnz > 1024 * static_cast<int64_t>(ctas))) continue;
-            if (prepare_clusters(cluster_kernel(threads), ctas, threads, kClSmemCap) != cudaSuccess) { cudaGetLastError(); continue; }
-            cl_ctas = ctas;
-            cl_threads = threads;
-        }
+        cl = plan_one_cluster(8, m, n, nnz, 1, 1, from, [&](int ctas, int threads) {
+            return prepare_clusters(cluster_kernel(threads), ctas, threads, kClSmemCap);
+        });
     };
     auto launch_cluster = [&](int len) {
-        return launch_clusters(cluster_kernel(cl_threads), 1, cl_ctas, cl_threads, kClSmemCap, st, mats,
+        return launch_clusters(cluster_kernel(cl.threads), 1, cl.ctas, cl.threads, cl.smem, st, mats,
                                EpiRefDual{p.row_lower.get(), p.row_upper.get(), y.get(), S, 0},
                                EpiRefPrimal{p.c.get(), p.col_lower.get(), p.col_upper.get(), x.get(), xb.get(), S, 0}, len,
-                               no_fit.get(), cl_launch(kClSmemCap));
+                               no_fit.get(), cl_launch(cl.smem));
     };
     plan(1);
-    while (cl_ctas) {   // no iterations: only whether the slices fit; a wider cluster where they do not
+    while (cl.ctas) {   // no iterations: only whether the slices fit; a wider cluster where they do not
         int h_fit = 0;
         VJ_CUDA(launch_cluster(0));
         VJ_CUDA(cudaMemcpyAsync(&h_fit, no_fit.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));
         if (!h_fit) break;
         VJ_CUDA(cudaMemsetAsync(no_fit.get(), 0, sizeof(int), st));
-        plan(2 * cl_ctas);
+        plan(2 * cl.ctas);
     }
     auto enqueue_chunk = [&](int len) {
-        if (cl_ctas) launch_cluster(len);   // an error shows at the end of the capture or at the launch check
-        for (int kk = 0; kk < len && !cl_ctas; ++kk) {
+        if (cl.ctas) launch_cluster(len);   // an error shows at the end of the capture or at the launch check
+        for (int kk = 0; kk < len && !cl.ctas; ++kk) {
             launch_spmv_exact<double, true>(a, p.csr_val.get(), xb.get(),
                                             EpiRefDual{p.row_lower.get(), p.row_upper.get(), y.get(), S, kk}, st);
             launch_spmv_exact<double, false>(at, p.csc_val.get(), y.get(),
@@ -466,7 +459,7 @@ vajra_status run_reference(vajra_pdhg* h, vajra_result* r) {
         if (hs->stop) break;
         if (seconds_since(t_start) > o.time_limit) { timed_out = 1; break; }
     }
-    if (cl_ctas) {
+    if (cl.ctas) {
         int h_fit = 0;
         VJ_CUDA(cudaMemcpyAsync(&h_fit, no_fit.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
         VJ_CUDA(cudaStreamSynchronize(st));

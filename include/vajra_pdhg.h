@@ -295,8 +295,10 @@ vajra_status vajra_pdhg_create(const vajra_lp* lp, const vajra_opts* opts, vajra
  * launches of many chunks; time_limit is checked after each (the first launch of a pass runs 2048
  * iterations, later ones what fits in the time left at the measured rate; without a limit to
  * speak of, each twice what ran before).  Instances that fit a thread-block cluster run on one
- * each, beside the packed rest.  Replaces a host loop of solve_pdhg_gpu calls (gpu.hpp:59), as
+ * each, beside the packed rest, where that is estimated to be the faster.  Replaces a host loop of solve_pdhg_gpu calls (gpu.hpp:59), as
  * the reference's benchmark Suite 2 issues them (apps/benchmark_runner.cpp:936-944).
+ * A row index outside its instance's rows returns VAJRA_ERR_INVALID_ARGUMENT (unsorted or repeated
+ * ones are added up as they come).
  * results[i] receives instance i; every result's device_time_sec is the whole batch's. */
 vajra_status vajra_pdhg_solve_batch(int32_t count, const vajra_lp* lps, const vajra_opts* opts,
                                     vajra_result* results);
@@ -349,7 +351,8 @@ void vajra_default_unrolled_opts(vajra_unrolled_opts* opts);
  * loss[count] and x_final[N] are outputs (x_final may be NULL); grad_c[N],
  * grad_row_lower[M], grad_row_upper[M] (any may be NULL; all NULL = forward only) receive
  * dL_i/d(c, row_lower, row_upper) of the unrolled map (an equality row's right-hand side
- * gradient is grad_row_lower + grad_row_upper). */
+ * gradient is grad_row_lower + grad_row_upper).  A row index outside its instance's rows returns
+ * VAJRA_ERR_INVALID_ARGUMENT. */
 vajra_status vajra_pdhg_unrolled(int32_t count, const vajra_lp* lps, const vajra_unrolled_opts* opts,
                                  const double* weights, double* loss, double* x_final, double* grad_c,
                                  double* grad_row_lower, double* grad_row_upper);
